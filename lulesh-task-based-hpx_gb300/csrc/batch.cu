@@ -162,7 +162,6 @@ int finish_admit(lulesh_batch* b, int slot, size_t off, size_t bytes, Mesh m, co
     m.result = b->d_results + slot;
     m.dtime = b->d_times + slot;
     m.partials = nullptr;
-    m.matGrid = 0;
     DevTime t{};
     t.time = ts.time;
     t.deltatime = ts.deltatime;
@@ -257,19 +256,28 @@ int effective_tile(const lulesh_batch* b) {
 bool rebuild_tiles(lulesh_batch* b) {
     const int T = effective_tile(b);
     for (auto& t : b->h_tiles) t.clear();
+    // lanes per element of the material tiles, from all running problems
+    std::map<int, int, std::greater<int>> count;
+    for (const Slot& sl : b->slots)
+        for (size_t c = 0; sl.in_use && !sl.finished && c < sl.repCount.size(); ++c)
+            count[sl.repValue[c]] += sl.repCount[c];
+    lulesh::RepClasses classes;
+    for (const auto& kv : count) classes.push_back(make_int2(kv.first, kv.second));
+    const int passes = classes.empty() ? 1 : lulesh::mat_passes_per_lane(classes, b->sms);
     for (int s = 0; s < int(b->slots.size()); ++s) {
         const Slot& sl = b->slots[s];
         if (!sl.in_use || sl.finished) continue;
         for (int e = 0; e < sl.numElem; e += T)
-            b->h_tiles[lulesh::TILES_ELEM].push_back({s, e, std::min(T, sl.numElem - e), std::min(T, sl.numElem - e)});
+            b->h_tiles[lulesh::TILES_ELEM].push_back({s, e, std::min(T, sl.numElem - e), std::min(T, sl.numElem - e), 1});
         for (int n = 0; n < sl.numNode; n += T)
-            b->h_tiles[lulesh::TILES_NODE].push_back({s, n, std::min(T, sl.numNode - n), std::min(T, sl.numNode - n)});
+            b->h_tiles[lulesh::TILES_NODE].push_back({s, n, std::min(T, sl.numNode - n), std::min(T, sl.numNode - n), 1});
         int pos = 0;
         for (size_t c = 0; c < sl.repCount.size(); ++c) {
             const int end = pos + sl.repCount[c];
             for (int t = pos; t < end; t += T) {
                 const int cnt = std::min(T, end - t);
-                b->h_tiles[lulesh::TILES_MAT].push_back({s, t, cnt, cnt * sl.repValue[c]});
+                b->h_tiles[lulesh::TILES_MAT].push_back(
+                    {s, t, cnt, cnt * sl.repValue[c], lulesh::lanes_for_rep(sl.repValue[c], passes)});
             }
             pos = end;
         }

@@ -70,8 +70,13 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 1) kb_phase(BatchCtl c, int gr
             if (!s_active) continue;
             if (PHASE == 3) {
                 double dtc = 1.0e+20, dth = 1.0e+20;
-                for (int k = threadIdx.x; k < tile.count; k += blockDim.x)
-                    material_elem(m, tile.first + k, dtc, dth);
+                const MatClass cls{tile.first, tile.count, tile.lanes, 0};
+                const int per_warp = 32 / cls.lanes;
+                for (int w = threadIdx.x >> 5; w * per_warp < cls.count; w += blockDim.x >> 5) {
+                    int pos, r;
+                    material_place(cls, w, pos, r);
+                    material_elem<true>(m, pos, r, cls.lanes, dtc, dth);
+                }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     dtc = fmin(dtc, __shfl_down_sync(0xffffffffu, dtc, o));

@@ -15,16 +15,17 @@
 namespace {
 
 using lulesh::DevTime;
+using lulesh::MatPlan;
 using lulesh::Mesh;
+using lulesh::RepClasses;
 using lulesh::StepResult;
 
 struct Launchers {
     int (*forces)(const Mesh&, cudaStream_t);
     int (*nodes)(const Mesh&, double, cudaStream_t);
     int (*kinematics)(const Mesh&, double, cudaStream_t);
-    int (*material)(const Mesh&, cudaStream_t);
+    int (*material)(const Mesh&, const MatPlan&, cudaStream_t);
     int (*forces_range)(const Mesh&, int, int, cudaStream_t);
-    int (*material_range)(const Mesh&, int, int, bool, cudaStream_t);
     // the resident loop's geometry form (fast double variant; else null):
     // kinematics store the element geometry the next forces read
     int (*forces_geo)(const Mesh&, cudaStream_t);
@@ -40,19 +41,17 @@ Launchers launchers_for(int precision) {
         case LULESH_FP64:
             return {lulesh::fp64::launch_forces, lulesh::fp64::launch_nodes,
                     lulesh::fp64::launch_kinematics, lulesh::fp64::launch_material,
-                    lulesh::fp64::launch_forces_range, lulesh::fp64::launch_material_range,
+                    lulesh::fp64::launch_forces_range,
                     lulesh::fp64::launch_forces_geo, lulesh::fp64::launch_kinematics_geo,
                     lulesh::fp64::launch_geometry, lulesh::fp64::launch_kinematics_range, lulesh::fp64::launch_kinematics_geo_range};
         case LULESH_FP64_EXACT:
             return {lulesh::fp64x::launch_forces, lulesh::fp64x::launch_nodes,
                     lulesh::fp64x::launch_kinematics, lulesh::fp64x::launch_material,
-                    lulesh::fp64x::launch_forces_range, lulesh::fp64x::launch_material_range,
-                    nullptr, nullptr, nullptr, lulesh::fp64x::launch_kinematics_range, nullptr};
+                    lulesh::fp64x::launch_forces_range, nullptr, nullptr, nullptr, lulesh::fp64x::launch_kinematics_range, nullptr};
         default:
             return {lulesh::mixed::launch_forces, lulesh::mixed::launch_nodes,
                     lulesh::mixed::launch_kinematics, lulesh::mixed::launch_material,
-                    lulesh::mixed::launch_forces_range, lulesh::mixed::launch_material_range,
-                    nullptr, nullptr, nullptr, lulesh::mixed::launch_kinematics_range, nullptr};
+                    lulesh::mixed::launch_forces_range, nullptr, nullptr, nullptr, lulesh::mixed::launch_kinematics_range, nullptr};
     }
 }
 
@@ -85,6 +84,9 @@ struct lulesh_dev {
     int64_t launches = 0;
     int32_t err_elem = -1;
     int32_t nx = 0;                  // edge of the cube (Domain::sizeX)
+    int32_t sms = 0;
+    MatPlan mat{};                   // the material launch over all elements
+    std::vector<MatPlan> mat_slab;   // lulesh_leapfrog's, one per slab (positions in matOrderSlab)
     double* d_verify = nullptr;      // [4] lulesh_dev_verify output (arena)
     double* h_verify = nullptr;      // [4] pinned
     // lulesh_leapfrog's upload and download streams and its hand-off events
@@ -226,16 +228,54 @@ void carve_mesh(Mesh& m, Arena& a, int precision, int ne, int nn) {
     }
 }
 
+// Most blocks of a material launch over n elements (material_plan).
+int mat_max_grid(int n, int sms) {
+    return lulesh::blocks_for(n, lulesh::kMatBlock) + lulesh::kMaxMatClasses + 8 * sms;
+}
+
+// The material launch over the classes, whose matOrder positions begin at
+// `first`, in at most max_grid blocks.
+MatPlan material_plan(const RepClasses& classes, int first, int sms, int max_grid) {
+    MatPlan p{};
+    const int passes = lulesh::mat_passes_per_lane(classes, sms);
+    for (const int2& c : classes) {
+        lulesh::MatClass& k = p.cls[p.n++];
+        k.first = first;
+        k.count = c.y;
+        k.lanes = lulesh::lanes_for_rep(c.x, passes);
+        k.warp0 = p.warps;
+        first += c.y;
+        p.count += c.y;
+        p.spread |= k.lanes > 1;
+        p.warps += lulesh::blocks_for(c.y, 32 / k.lanes);
+    }
+    p.grid = std::max(1, std::min(lulesh::blocks_for(p.warps, lulesh::kMatBlock / 32), max_grid));
+    return p;
+}
+
+// The handle's material launches: over all elements at most `per_sm` blocks
+// per multiprocessor, over a slab one warp per 32 / lanes elements.
+void plan_material(lulesh_dev* d, const RepClasses& classes, const std::vector<RepClasses>& slab_classes, int per_sm) {
+    d->mat = material_plan(classes, 0, d->sms, d->sms * per_sm);
+    d->mat_slab.clear();
+    int first = 0;
+    for (const RepClasses& c : slab_classes) {
+        int n = 0;
+        for (const int2& k : c) n += k.y;
+        d->mat_slab.push_back(material_plan(c, first, d->sms, mat_max_grid(n, d->sms)));
+        first += n;
+    }
+}
+
 // Every device array of a single-problem handle: the mesh, then the
 // reduction scratch and the graph form's time state.
-void layout(lulesh_dev* d, Arena& a, int ne, int nn, int matGrid) {
+void layout(lulesh_dev* d, Arena& a, int ne, int nn) {
     Mesh& m = d->m;
     carve_mesh(m, a, d->precision, ne, nn);
-    // one partial per block of the material launch: the full grid, or the
-    // slab launches of lulesh_leapfrog with one thread per element, each in
-    // its own part (at most one block more per slab than one launch over all)
-    m.partials = a.take<lulesh::DtPartial>(
-        std::max(matGrid, lulesh::blocks_for(ne, lulesh::kMatBlock) + kLeapfrogSlabs));
+    // one partial per block of the material launch: the launch over all
+    // elements, or lulesh_leapfrog's slab launches, each in its own part
+    m.partials = a.take<lulesh::DtPartial>(size_t(lulesh::blocks_for(ne, lulesh::kMatBlock)) +
+                                           kLeapfrogSlabs * mat_max_grid(1, d->sms));
     m.result = a.take<StepResult>(1);
     for (double*& p : d->stage) p = d->L.forces_geo ? a.take<double>(nn) : nullptr;
     d->upload_flag = a.take<int32_t>(kLeapfrogSlabs);
@@ -293,7 +333,7 @@ std::vector<Copy> groups(const Mesh& m, const lulesh_domain_view* v, uint32_t ma
 // float-pair mirrors, and waits for the copies (some read host vectors that
 // live only in this call).
 int upload_mesh(const Mesh& m, const lulesh_domain_view* v, int precision, cudaStream_t s, int slabs,
-                int32_t* slab_order) {
+                int32_t* slab_order, RepClasses* classes, std::vector<RepClasses>* slab_classes) {
     const int ne = v->numElem, nn = v->numNode;
     // per-node symmetry bits, per-element EOS repeat count and the
     // repeat-count grouping of the material phase
@@ -307,6 +347,15 @@ int upload_mesh(const Mesh& m, const lulesh_domain_view* v, int precision, cudaS
     for (int i = 0; i < ne; ++i) rep[i] = lulesh::region_rep(v->regNumList[i] - 1, v->numReg, v->cost);
     for (int i = 0; i < ne; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rep[a] > rep[b]; });
+    auto count_classes = [&](const int32_t* elems, size_t n, RepClasses& out) {
+        out.clear();
+        for (size_t k = 0; k < n; ++k) {
+            if (out.empty() || out.back().x != rep[elems[k]]) out.push_back(make_int2(rep[elems[k]], 0));
+            ++out.back().y;
+        }
+    };
+    if (classes) count_classes(order.data(), order.size(), *classes);
+    if (slab_classes) slab_classes->assign(1, classes ? *classes : RepClasses{});
     std::vector<int32_t> sorder;
     if (slab_order && slabs > 1) {
         // the same order split by slab of whole element planes (a stable
@@ -321,6 +370,14 @@ int upload_mesh(const Mesh& m, const lulesh_domain_view* v, int precision, cudaS
         sorder = order;
         std::stable_sort(sorder.begin(), sorder.end(),
                          [&](int a, int b) { return slab_of[a / s2] < slab_of[b / s2]; });
+        if (slab_classes) {
+            slab_classes->assign(slabs, RepClasses{});
+            for (int sl = 0; sl < slabs; ++sl) {
+                int p0, p1;
+                slab_planes(sx, slabs, sl, p0, p1);
+                count_classes(sorder.data() + size_t(p0) * s2, size_t(p1 - p0) * s2, (*slab_classes)[sl]);
+            }
+        }
         CK(cudaMemcpyAsync(slab_order, sorder.data(), sizeof(int32_t) * size_t(ne), cudaMemcpyHostToDevice, s));
     }
 
@@ -389,7 +446,7 @@ int queue_rest(lulesh_dev* d, double dt, int set) {
     d->launches += geo ? d->L.kinematics_geo(m, dt, d->stream) : d->L.kinematics(m, dt, d->stream);
     d->geo_valid = geo;
     if (prof) CK(cudaEventRecord(d->ev[set][3], d->stream));
-    d->launches += d->L.material(m, d->stream);
+    d->launches += d->L.material(m, d->mat, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][4], d->stream));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(d->h_result, m.result, sizeof(StepResult), cudaMemcpyDeviceToHost, d->stream));
@@ -433,7 +490,7 @@ int build_graph(lulesh_dev* d) {
     k += geo ? d->L.forces_geo(gm, d->stream) : d->L.forces(gm, d->stream);
     k += d->L.nodes(gm, 0.0, d->stream);
     k += geo ? d->L.kinematics_geo(gm, 0.0, d->stream) : d->L.kinematics(gm, 0.0, d->stream);
-    k += d->L.material(gm, d->stream);
+    k += d->L.material(gm, d->mat, d->stream);
     k += lulesh::launch_time_finish(d->d_time, gm.result, d->stream);
     cudaError_t ce = cudaStreamEndCapture(d->stream, &g);
     if (ce != cudaSuccess) return LULESH_ECUDA;
@@ -446,6 +503,12 @@ int build_graph(lulesh_dev* d) {
     d->graph_kernels = k;
     return LULESH_OK;
 }
+
+// Material blocks per SM of the grid-stride launch (elements in repeat-count
+// order; 6 blocks of 78 registers fit per SM): a sweep of 6, 8, 12 per SM and
+// one thread per element at s=150 gave the double kernel 1.38, 1.34, 1.37,
+// 1.51 ms and the mixed kernel 0.92, 0.98, 0.95, 1.08 ms
+int mat_blocks_per_sm(int precision) { return precision == LULESH_MIXED ? 6 : 8; }
 
 // A handle for ne elements and nn nodes: the arena carved, the stream and
 // the pinned result buffers created, the device result word cleared. The
@@ -462,15 +525,9 @@ int new_handle(int32_t precision, int ne, int nn, lulesh_dev** out) {
     if (!d) return LULESH_ENOMEM;
     d->precision = precision;
     d->L = launchers_for(precision);
-    // Material blocks per SM of the grid-stride launch (elements in
-    // repeat-count order; 6 blocks of 78 registers fit per SM): a sweep of
-    // 6, 8, 12 per SM and one thread per element at s=150 gave the double
-    // kernel 1.38, 1.34, 1.37, 1.51 ms and the mixed kernel 0.92, 0.98, 0.95,
-    // 1.08 ms
-    const int mat_per_sm = precision == LULESH_MIXED ? 6 : 8;
-    const int matGrid = std::max(1, std::min(lulesh::blocks_for(ne, lulesh::kMatBlock), sms * mat_per_sm));
+    d->sms = sms;
     Arena measure;
-    layout(d, measure, ne, nn, matGrid);
+    layout(d, measure, ne, nn);
     d->arena_bytes = measure.used;
     auto fail = [&](int code) {
         lulesh_dev_destroy(d);
@@ -479,11 +536,10 @@ int new_handle(int32_t precision, int ne, int nn, lulesh_dev** out) {
     if (cudaMalloc(&d->arena, d->arena_bytes) != cudaSuccess) return fail(LULESH_ENOMEM);
     Arena carve;
     carve.base = static_cast<char*>(d->arena);
-    layout(d, carve, ne, nn, matGrid);
+    layout(d, carve, ne, nn);
     Mesh& m = d->m;
     m.numElem = ne;
     m.numNode = nn;
-    m.matGrid = matGrid;
     m.dtime = nullptr;
     if (cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(LULESH_ECUDA);
@@ -511,11 +567,15 @@ int lulesh_dev_create(const lulesh_domain_view* v, int32_t precision, lulesh_dev
     if (st != LULESH_OK) return st;
     d->m.prm = v->params;
     d->nx = v->sizeX;
-    st = upload_mesh(d->m, v, precision, d->stream, slab_count(v->sizeX, v->numElem), d->matOrderSlab);
+    RepClasses classes;
+    std::vector<RepClasses> slab_classes;
+    st = upload_mesh(d->m, v, precision, d->stream, slab_count(v->sizeX, v->numElem), d->matOrderSlab, &classes,
+                     &slab_classes);
     if (st != LULESH_OK) {
         lulesh_dev_destroy(d);
         return st;
     }
+    plan_material(d, classes, slab_classes, mat_blocks_per_sm(precision));
     if (precision == LULESH_MIXED) ++d->launches;  // the float-pair mirror kernel
     *out = d;
     return LULESH_OK;
@@ -532,12 +592,15 @@ int lulesh_dev_create_problem(const lulesh_problem* p, int32_t precision, lulesh
     st = new_handle(precision, ne, nn, &d);
     if (st != LULESH_OK) return st;
     d->nx = p->s;
-    st = lulesh::mesh_fill_problem(d->m, p, precision, d->stream, ts, nullptr, slab_count(p->s, ne),
-                                   d->matOrderSlab);
+    RepClasses classes;
+    std::vector<RepClasses> slab_classes;
+    st = lulesh::mesh_fill_problem(d->m, p, precision, d->stream, ts, &classes, slab_count(p->s, ne),
+                                   d->matOrderSlab, &slab_classes);
     if (st != LULESH_OK) {
         lulesh_dev_destroy(d);
         return st;
     }
+    plan_material(d, classes, slab_classes, mat_blocks_per_sm(precision));
     // the build kernels, the material orders (and the mirror)
     d->launches += 5 + (slab_count(p->s, ne) > 1 ? 1 : 0) + (precision == LULESH_MIXED ? 1 : 0);
     *out = d;
@@ -860,14 +923,13 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     if (slabs > 1) ms.matOrder = d->matOrderSlab;
     int part = 0;  // first block partial of the slab
     for (int sl = 0; sl < slabs; ++sl) {
-        // one thread per element: blocks schedule dynamically, the slab's
-        // most expensive elements first (repeat-count order within a slab)
+        // no grid-stride: blocks schedule dynamically, the slab's most
+        // expensive elements first (repeat-count order within a slab)
         cudaStream_t cs = (sl & 1) ? d->stream2 : d->stream;
-        ms.matGrid = std::max(1, lulesh::blocks_for(int(e_hi[sl] - e_lo[sl]), lulesh::kMatBlock));
         ms.partials = m.partials + part;
         ms.result = d->slab_result + sl;
-        part += ms.matGrid;
-        d->launches += d->L.material_range(ms, int(e_lo[sl]), int(e_hi[sl]), false, cs);
+        part += d->mat_slab[sl].grid;
+        d->launches += d->L.material(ms, d->mat_slab[sl], cs);
         if (int st = elem_down(out_mat, e_lo[sl], e_hi[sl], d->ev_mat[sl], cs, LULESH_TL_MAT, sl)) return st;
     }
     CK(cudaGetLastError());
@@ -1006,7 +1068,7 @@ int lulesh_dev_phase(lulesh_dev* d, int32_t phase, double dt) {
         case LULESH_PHASE_FORCES: d->launches += d->L.forces(m, d->stream); break;
         case LULESH_PHASE_NODES: d->launches += d->L.nodes(m, dt, d->stream); break;
         case LULESH_PHASE_KINEMATICS: d->launches += d->L.kinematics(m, dt, d->stream); break;
-        case LULESH_PHASE_MATERIAL: d->launches += d->L.material(m, d->stream); break;
+        case LULESH_PHASE_MATERIAL: d->launches += d->L.material(m, d->mat, d->stream); break;
         default: return LULESH_EINVAL;
     }
     CK(cudaGetLastError());
@@ -1114,6 +1176,38 @@ namespace lulesh {
 
 int validate_view(const lulesh_domain_view* v) { return check_view(v); }
 
+// The time of a material phase whose lanes run at most k passes each, in
+// units of one warp's pass on a busy SM quarter (3.2 us measured at s=150):
+// the longest lane's chain (its passes and the rest of the phase as one more,
+// 1.4 units each: a lone warp's pass takes 4.3 us) and the warps' work over
+// the 4 quarters of each SM (a warp's passes and, for the Q terms and the
+// save, three more). Few elements leave the quarters idle, so more lanes per
+// element win (s=8: 87 -> 24 us, s=30: 94 -> 48 us); many keep them busy, and
+// spreading an element then only repeats its Q terms (s=91 with 4 lanes for
+// 20 passes 0.450 -> 0.483 ms, so one lane there).
+int mat_passes_per_lane(const RepClasses& classes, int sms) {
+    int top = 1;
+    for (const int2& c : classes) top = std::max(top, c.x);
+    int best = top;
+    double best_t = 0.0;  // a split has to save a tenth of the unsplit time
+    for (int k = top; k >= 1; k = std::min(k, 64) - 1) {
+        double load = 0.0;
+        int chain = 0;
+        for (const int2& c : classes) {
+            const int lanes = lanes_for_rep(c.x, k), passes = (c.x + lanes - 1) / lanes;
+            chain = std::max(chain, passes);
+            load += double(blocks_for(c.y, 32 / lanes)) * (passes + 3);
+        }
+        const double t = 1.4 * (chain + 1) + load / (4.0 * sms);
+        if (k == top) best_t = 0.9 * t;
+        else if (t < best_t) {
+            best_t = t;
+            best = k;
+        }
+    }
+    return best;
+}
+
 size_t mesh_bytes(int precision, int numElem, int numNode) {
     Mesh m{};
     Arena a;
@@ -1128,7 +1222,7 @@ int mesh_init(Mesh& m, char* base, const lulesh_domain_view* v, int precision, c
     m.numElem = v->numElem;
     m.numNode = v->numNode;
     m.prm = v->params;
-    return upload_mesh(m, v, precision, s, 1, nullptr);
+    return upload_mesh(m, v, precision, s, 1, nullptr, nullptr, nullptr);
 }
 
 int check_problem(const lulesh_problem* p) {
@@ -1163,7 +1257,7 @@ void order_ranges(const std::vector<RegionRun>& runs, const std::vector<int>& re
 }  // namespace
 
 int mesh_fill_problem(Mesh& m, const lulesh_problem* p, int precision, cudaStream_t s, lulesh_time_state* ts,
-                      std::vector<int2>* classes, int slabs, int32_t* slab_order) {
+                      RepClasses* classes, int slabs, int32_t* slab_order, std::vector<RepClasses>* slab_classes) {
     const int ne = m.numElem;
     default_params(m.prm);
     double einit = 0.0;
@@ -1187,6 +1281,7 @@ int mesh_fill_problem(Mesh& m, const lulesh_problem* p, int precision, cudaStrea
             if (classes->empty() || classes->back().x != r) classes->push_back(make_int2(r, 0));
             classes->back().y += runs[idx[k]].count;
         }
+        if (slab_classes) slab_classes->assign(1, *classes);
     }
     // the slab-major order: runs cut at the slab boundaries (whole element
     // planes), ordered by slab, then repeat count
@@ -1215,7 +1310,16 @@ int mesh_fill_problem(Mesh& m, const lulesh_problem* p, int precision, cudaStrea
                 ++sl;
             }
         }
-        order_ranges(cut, cut_rep, [&](int k) { return slab_of[k]; }, sorder, soff);
+        std::vector<int> sidx;
+        order_ranges(cut, cut_rep, [&](int k) { return slab_of[k]; }, sorder, soff, &sidx);
+        if (slab_classes) {
+            slab_classes->assign(slabs, RepClasses{});
+            for (int k : sidx) {
+                RepClasses& c = (*slab_classes)[slab_of[k]];
+                if (c.empty() || c.back().x != cut_rep[k]) c.push_back(make_int2(cut_rep[k], 0));
+                c.back().y += cut[k].count;
+            }
+        }
     }
     // the tables in one stream-ordered temporary allocation
     const int nruns = int(runs.size()), ncut = int(sorder.size());
@@ -1255,14 +1359,14 @@ int mesh_fill_problem(Mesh& m, const lulesh_problem* p, int precision, cudaStrea
 }
 
 int mesh_init_problem(Mesh& m, char* base, const lulesh_problem* p, int precision, cudaStream_t s,
-                      lulesh_time_state* ts, std::vector<int2>* classes) {
+                      lulesh_time_state* ts, RepClasses* classes) {
     Arena a;
     a.base = base;
     const int ne = p->s * p->s * p->s, nn = (p->s + 1) * (p->s + 1) * (p->s + 1);
     carve_mesh(m, a, precision, ne, nn);
     m.numElem = ne;
     m.numNode = nn;
-    return mesh_fill_problem(m, p, precision, s, ts, classes, 1, nullptr);
+    return mesh_fill_problem(m, p, precision, s, ts, classes, 1, nullptr, nullptr);
 }
 
 int copy_fields(const Mesh& m, const lulesh_domain_view* v, uint32_t mask, bool to_device, cudaStream_t s) {

@@ -376,21 +376,10 @@ __device__ __forceinline__ void kinematics_fast(const Mesh& m, int i, double dt)
 __device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt) { kinematics_fast<false>(m, i, dt); }
 #endif
 
-// Material phase of the element at position t of the repeat-count order
-// (matOrder): Q limiter and q terms, rep EOS passes, sound speed and save;
-// folds its Courant and hydro constraints into dtc, dth.
-__device__ __forceinline__ void material_elem(const Mesh& m, int t, double& dtc, double& dth) {
-    const int i = LD(m.matOrder + t);
-    const double vnew = LD(m.vnew + i), vdov = LD(m.vdov + i);
-    double ql, qq;
-    q_terms<double>(m, i, m.dvxi, m.dveta, m.dvzeta, m.dxxi, m.dxeta, m.dxzeta, vnew, vdov, ql, qq);
-    m.qq[i] = qq;
-    m.ql[i] = ql;
-    double vnewc = vnew;
-    if (!f_is_zero(m.prm.eosvmin) && f_lt(vnewc, m.prm.eosvmin)) vnewc = m.prm.eosvmin;
-    if (!f_is_zero(m.prm.eosvmax) && f_gt(vnewc, m.prm.eosvmax)) vnewc = m.prm.eosvmax;
-    const double ss = eos_element(m, i, vnewc, LD(m.elemRep + i));
-    dt_constraints(m.prm, ss, vdov, LD(m.arealg + i), dtc, dth);
+// Material phase of an element by several lanes (material_share).
+template <bool SPREAD>
+__device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int lanes, double& dtc, double& dth) {
+    material_share<SPREAD>(m, t, r, lanes, m.dvxi, m.dveta, m.dvzeta, m.dxxi, m.dxeta, m.dxzeta, dtc, dth);
 }
 
 // --- single-problem kernels -------------------------------------------------
@@ -494,12 +483,25 @@ __global__ void __launch_bounds__(kForceBlock) k_geometry(Mesh m) {
 // 8 blocks of 128 per SM (64 registers): the EOS passes are a chain of
 // dependent integer-pipe products and FP64 operations, latency-bound at 6
 // blocks per SM (1.34 -> 1.02 ms at s=150 with 8).
-__global__ void __launch_bounds__(kMatBlock, 8) k_material(Mesh m, int first, int end, int accumulate) {
+// SPREAD: some class has several lanes per element (MatPlan).
+template <bool SPREAD>
+__global__ void __launch_bounds__(kMatBlock, 8) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
     if (m.dtime && !m.dtime->active) return;
     double dtc = 1.0e+20, dth = 1.0e+20;  // lulesh.cc:2214-2215
-    for (int t = first + blockIdx.x * blockDim.x + threadIdx.x; t < end; t += gridDim.x * blockDim.x)
-        material_elem(m, t, dtc, dth);
-    finish_dt_reduction(m, dtc, dth, accumulate != 0);
+    if (SPREAD) {
+        const int nwarps = gridDim.x * (kMatBlock / 32);
+        for (int w = blockIdx.x * (kMatBlock / 32) + (threadIdx.x >> 5); w < plan.warps; w += nwarps) {
+            int k = 0;
+            while (k + 1 < plan.n && w >= plan.cls[k + 1].warp0) ++k;
+            int t, r;
+            material_place(plan.cls[k], w - plan.cls[k].warp0, t, r);
+            material_elem<true>(m, t, r, plan.cls[k].lanes, dtc, dth);
+        }
+    } else {
+        for (int t = blockIdx.x * kMatBlock + threadIdx.x; t < plan.count; t += gridDim.x * kMatBlock)
+            material_elem<false>(m, plan.cls[0].first + t, 0, 1, dtc, dth);
+    }
+    finish_dt_reduction(m, dtc, dth);
 }
 
 int launch_forces(const Mesh& m, cudaStream_t s) {
@@ -524,12 +526,9 @@ int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaSt
     k_kinematics<true><<<blocks_for(end - first, kKinBlock), kKinBlock, 0, s>>>(m, dt, first, end);
     return 1;
 }
-int launch_material(const Mesh& m, cudaStream_t s) {
-    k_material<<<m.matGrid, kMatBlock, 0, s>>>(m, 0, m.numElem, 0);
-    return 1;
-}
-int launch_material_range(const Mesh& m, int first, int end, bool accumulate, cudaStream_t s) {
-    k_material<<<m.matGrid, kMatBlock, 0, s>>>(m, first, end, accumulate ? 1 : 0);
+int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s) {
+    if (plan.spread) k_material<true><<<plan.grid, kMatBlock, 0, s>>>(m, plan);
+    else k_material<false><<<plan.grid, kMatBlock, 0, s>>>(m, plan);
     return 1;
 }
 #if !LULESH_EXACT

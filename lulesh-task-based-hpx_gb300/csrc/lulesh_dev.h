@@ -90,10 +90,9 @@ struct Mesh {
     float *fcx, *fcy, *fcz;
     float *gvxi, *gveta, *gvzeta, *gxxi, *gxeta, *gxzeta;
     // reduction scratch
-    DtPartial* partials;
+    DtPartial* partials;  // one per block of a material launch
     StepResult* result;
     DevTime* dtime;  // non-null only in the graph form: kernels take dt from here
-    int32_t matGrid; // blocks of the material kernel (= entries of partials)
     lulesh_params prm;
 };
 
@@ -109,6 +108,32 @@ constexpr int kMatBlock = 128;
 
 inline int blocks_for(int n, int b) { return (n + b - 1) / b; }
 
+// How a material launch spreads its elements over lanes. The passes of an
+// element's EOS repeat loop do not depend on one another (each one starts
+// from the saved state), so an element with rep passes may be given up to rep
+// lanes of one warp, each running its share. One class per repeat count, in
+// matOrder order; a warp holds 32 / lanes elements of one class.
+constexpr int kMaxMatClasses = 4;
+struct MatClass {
+    int32_t first, count;  // matOrder positions [first, first + count)
+    int32_t lanes;         // lanes per element, 1..32
+    int32_t warp0;         // first warp of the class
+};
+struct MatPlan {
+    int32_t n, warps, grid;  // classes, warps in all, blocks of the launch
+    int32_t count, spread;   // elements in all; does any class have more than one lane per element
+    MatClass cls[kMaxMatClasses];
+};
+// (repeat count, elements) pairs, largest repeat count first.
+using RepClasses = std::vector<int2>;
+// EOS passes a lane should run at most, for these classes on a GPU of `sms`
+// multiprocessors (lanes_for_rep gives the lanes).
+int mat_passes_per_lane(const RepClasses& classes, int sms);
+inline int lanes_for_rep(int rep, int passes) {
+    const int l = (rep + passes - 1) / passes;
+    return l < 1 ? 1 : l > 32 ? 32 : l;
+}
+
 // Launchers, one set per arithmetic variant. Each returns the number of
 // kernels it launched. `dt` is used unless m.dtime is set.
 namespace fp64 {
@@ -117,9 +142,7 @@ int launch_forces_range(const Mesh& m, int first, int end, cudaStream_t s);  // 
 int launch_nodes(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaStream_t s);  // elements
-int launch_material(const Mesh& m, cudaStream_t s);
-// matOrder positions [first, end); accumulate: fold the dt minima into m.result's
-int launch_material_range(const Mesh& m, int first, int end, bool accumulate, cudaStream_t s);
+int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s);  // the plan's matOrder positions
 // the resident loop's form: kinematics that also stores the element geometry
 // of the updated coordinates (m.geo), forces that read it, and the pass that
 // forms it from the current coordinates when it is stale
@@ -147,9 +170,7 @@ int launch_forces_range(const Mesh& m, int first, int end, cudaStream_t s);  // 
 int launch_nodes(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaStream_t s);  // elements
-int launch_material(const Mesh& m, cudaStream_t s);
-// matOrder positions [first, end); accumulate: fold the dt minima into m.result's
-int launch_material_range(const Mesh& m, int first, int end, bool accumulate, cudaStream_t s);
+int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s);  // the plan's matOrder positions
 }  // namespace fp64x
 namespace mixed {
 int launch_forces(const Mesh& m, cudaStream_t s);
@@ -157,9 +178,7 @@ int launch_forces_range(const Mesh& m, int first, int end, cudaStream_t s);  // 
 int launch_nodes(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaStream_t s);  // elements
-int launch_material(const Mesh& m, cudaStream_t s);
-// matOrder positions [first, end); accumulate: fold the dt minima into m.result's
-int launch_material_range(const Mesh& m, int first, int end, bool accumulate, cudaStream_t s);
+int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s);  // the plan's matOrder positions
 int launch_mirror(const Mesh& m, cudaStream_t s);
 int launch_mirror_range(const Mesh& m, int first, int end, cudaStream_t s);  // nodes [first, end)
 }  // namespace mixed
@@ -178,6 +197,7 @@ struct BatchTile {
     int32_t first;  // first element / node / matOrder position
     int32_t count;  // number of units
     int32_t cost;   // units x EOS passes (material tiles), for ordering
+    int32_t lanes;  // lanes per element (material tiles, as MatClass::lanes)
 };
 
 enum { TILES_ELEM = 0, TILES_NODE = 1, TILES_MAT = 2 };
@@ -271,14 +291,15 @@ int check_problem(const lulesh_problem* p);
 // given, *classes as mesh_init_problem does. With slab_order and slabs > 1
 // it also writes the material order split into that many slabs of whole
 // element planes (repeat-count order within a slab) to slab_order[N_e],
-// for a material phase run slab by slab.
+// for a material phase run slab by slab, and each slab's classes to
+// *slab_classes.
 int mesh_fill_problem(Mesh& m, const lulesh_problem* p, int precision, cudaStream_t s, lulesh_time_state* ts,
-                      std::vector<int2>* classes, int slabs, int32_t* slab_order);
+                      RepClasses* classes, int slabs, int32_t* slab_order, std::vector<RepClasses>* slab_classes);
 // The same for problem p built on the device (no host Domain): fills *ts
-// with the problem's initial time state and *classes with (repeat count,
-// elements) pairs, largest repeat count first; waits for the build.
+// with the problem's initial time state and *classes with its repeat
+// classes; waits for the build.
 int mesh_init_problem(Mesh& m, char* base, const lulesh_problem* p, int precision, cudaStream_t s,
-                      lulesh_time_state* ts, std::vector<int2>* classes);
+                      lulesh_time_state* ts, RepClasses* classes);
 // Copies the LULESH_F_* field groups of mask between m and v (either way)
 // on stream s and waits.
 int copy_fields(const Mesh& m, const lulesh_domain_view* v, uint32_t mask, bool to_device, cudaStream_t s);

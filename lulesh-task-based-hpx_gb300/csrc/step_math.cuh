@@ -1063,9 +1063,14 @@ __device__ __forceinline__ double q_sound(double ssc) {
 #endif
 }
 
-// rep evaluations of EvalEOSAllInOneTask (lulesh.cc:1692-1871) for element i,
-// each from the saved state, then the sound speed and the save of
-// CalcSoundSpeedForElemsAndSaveTask (lulesh.cc:1873-1904). Returns ss.
+// The state one EOS evaluation ends with, and its sound speed.
+struct EosState {
+    double e, p, q, ss;
+};
+
+// `passes` evaluations of EvalEOSAllInOneTask (lulesh.cc:1692-1871) for
+// element i, each from the saved state, then the sound speed of
+// CalcSoundSpeedForElemsAndSaveTask (lulesh.cc:1873-1904).
 // UNIT_RHO: refdens == 1, so the divisions by it are identities.
 #if LULESH_EXACT
 // The reference's "+ 0.5 * work" terms add 0.5 * 0 (work is zero,
@@ -1073,11 +1078,11 @@ __device__ __forceinline__ double q_sound(double ssc) {
 // leave them out.
 #define LULESH_PLUS_ZERO_WORK +0.5 * 0.0
 template <bool UNIT_RHO>
-__device__ __forceinline__ double eos_body(const Mesh& m, int i, double vnewc, int rep) {
+__device__ __forceinline__ EosState eos_body(const Mesh& m, int i, double vnewc, int passes) {
     const lulesh_params& P = m.prm;
     double e_new = 0., p_new = 0., q_new = 0., bvc = 0., pbvc = 0.;
     const bool vmin_on = !f_is_zero(P.eosvmin), vmax_on = !f_is_zero(P.eosvmax);
-    for (int r = 0; r < rep; ++r) {
+    for (int r = 0; r < passes; ++r) {
         // Each evaluation re-reads its inputs from memory as the reference's
         // EvalEOSInit does (lulesh.cc:1720-1727), and vnewc is made opaque,
         // so the compiler can hoist no part of the evaluation out of the
@@ -1135,11 +1140,7 @@ __device__ __forceinline__ double eos_body(const Mesh& m, int i, double vnewc, i
         }
     }
     const double sst = ss_guard(over_rho<UNIT_RHO>((pbvc * e_new + vnewc * vnewc * bvc * p_new), P));
-    m.ss[i] = sst;
-    m.p[i] = p_new;
-    m.e[i] = e_new;
-    m.q[i] = q_new;
-    return sst;
+    return {e_new, p_new, q_new, sst};
 }
 
 #else
@@ -1159,12 +1160,12 @@ __device__ __forceinline__ double pressure(double bvc, double e, double vnewc, c
 }
 
 template <bool UNIT_RHO>
-__device__ __forceinline__ double eos_body(const Mesh& m, int i, double vnewc, int rep) {
+__device__ __forceinline__ EosState eos_body(const Mesh& m, int i, double vnewc, int passes) {
     const lulesh_params& P = m.prm;
     const double cls = 2.0 / 3.0;
     double e_new = 0., p_new = 0., q_new = 0., vf = vnewc;
     const bool vmin_on = !f_is_zero(P.eosvmin), vmax_on = !f_is_zero(P.eosvmax);
-    for (int r = 0; r < rep; ++r) {
+    for (int r = 0; r < passes; ++r) {
         asm volatile("" ::: "memory");
         asm volatile("" : "+d"(vnewc));
         const double e_old = m.e[i], delvc = m.delv[i], q_old = m.q[i];
@@ -1211,16 +1212,12 @@ __device__ __forceinline__ double eos_body(const Mesh& m, int i, double vnewc, i
         }
     }
     const double sst = ss_guard(over_rho<UNIT_RHO>(pmul(cls, fma(vf, p_new, e_new)), P));
-    m.ss[i] = sst;
-    m.p[i] = p_new;
-    m.e[i] = e_new;
-    m.q[i] = q_new;
-    return sst;
+    return {e_new, p_new, q_new, sst};
 }
 #endif
 
-__device__ __forceinline__ double eos_element(const Mesh& m, int i, double vnewc, int rep) {
-    return m.prm.refdens == 1.0 ? eos_body<true>(m, i, vnewc, rep) : eos_body<false>(m, i, vnewc, rep);
+__device__ __forceinline__ EosState eos_element(const Mesh& m, int i, double vnewc, int passes) {
+    return m.prm.refdens == 1.0 ? eos_body<true>(m, i, vnewc, passes) : eos_body<false>(m, i, vnewc, passes);
 }
 
 // Courant and hydro candidates of one element (lulesh.cc:1938-1974); false
@@ -1251,6 +1248,63 @@ __device__ __forceinline__ void dt_constraints(const lulesh_params& P, double ss
     dth = nonneg_min(dth, hydro);
 }
 
+// Material phase of the element at position t of the repeat-count order
+// (matOrder) by `lanes` lanes of one warp, of which this is lane r: Q limiter
+// and q terms, this lane's share of the element's EOS passes, then (lane 0,
+// whose share is the largest) the save (lulesh.cc:1881-1904) and the
+// element's Courant and hydro constraints folded into dtc, dth. dv and dx are
+// the Q gradients, R their type. Every lane of the warp must call it; one
+// with r >= lanes runs no pass and saves nothing. Without SPREAD each lane
+// has an element of its own (r = 0, lanes = 1).
+template <bool SPREAD, class R>
+__device__ __forceinline__ void material_share(const Mesh& m, int t, int r, int lanes, const R* dvxi, const R* dveta,
+                                               const R* dvzeta, const R* dxxi, const R* dxeta, const R* dxzeta,
+                                               double& dtc, double& dth) {
+    const int i = LD(m.matOrder + t);
+    const double vnew = LD(m.vnew + i), vdov = LD(m.vdov + i);
+    double ql, qq;
+    q_terms<R>(m, i, dvxi, dveta, dvzeta, dxxi, dxeta, dxzeta, vnew, vdov, ql, qq);
+    if (!SPREAD || r == 0) {
+        m.qq[i] = qq;
+        m.ql[i] = ql;
+    }
+    if (SPREAD) __syncwarp();  // the passes of every lane read ql and qq back
+    double vnewc = vnew;
+    if (!f_is_zero(m.prm.eosvmin) && f_lt(vnewc, m.prm.eosvmin)) vnewc = m.prm.eosvmin;
+    if (!f_is_zero(m.prm.eosvmax) && f_gt(vnewc, m.prm.eosvmax)) vnewc = m.prm.eosvmax;
+    const int rep = LD(m.elemRep + i);
+    const int passes = !SPREAD || lanes == 1 ? (r == 0 ? rep : 0) : r < lanes ? (rep - r + lanes - 1) / lanes : 0;
+    const EosState s = eos_element(m, i, vnewc, passes);
+    if (SPREAD) {
+        __syncwarp();  // no lane reads e, p, q of this element any more
+        if (r != 0) return;
+    }
+    m.ss[i] = s.ss;
+    m.p[i] = s.p;
+    m.e[i] = s.e;
+    m.q[i] = s.q;
+    dt_constraints(m.prm, s.ss, vdov, LD(m.arealg + i), dtc, dth);
+}
+
+// The lane's element and share in warp w of a class: position t (the last
+// one again where the warp has lanes left over) and lane r of the element.
+__device__ __forceinline__ void material_place(const MatClass& c, int w, int& t, int& r) {
+    const int lane = threadIdx.x & 31;
+    if (c.lanes == 1) {
+        t = 32 * w + lane;
+        r = 0;
+    } else {
+        const int per_warp = 32 / c.lanes, g = lane / c.lanes;
+        t = per_warp * w + g;
+        r = g < per_warp ? lane - g * c.lanes : c.lanes;
+    }
+    if (t >= c.count) {
+        t = c.count - 1;
+        r = c.lanes;
+    }
+    t += c.first;
+}
+
 // Block-wide min of (a, b); the result is valid in thread 0.
 __device__ __forceinline__ void block_min2(double& a, double& b) {
     __shared__ double sa[32], sb[32];
@@ -1278,11 +1332,9 @@ __device__ __forceinline__ void block_min2(double& a, double& b) {
 }
 
 // Publishes this block's (dtc, dth) minima; the last block to arrive reduces
-// all partials into m.result (with accumulate, into the minima already
-// there: a launch over part of the elements) and re-arms the counter. One
-// pass, no second launch. Every thread of the block must call it.
-__device__ __forceinline__ void finish_dt_reduction(const Mesh& m, double dtc, double dth,
-                                                    bool accumulate = false) {
+// all partials into m.result and re-arms the counter. One pass, no second
+// launch. Every thread of the block must call it.
+__device__ __forceinline__ void finish_dt_reduction(const Mesh& m, double dtc, double dth) {
     block_min2(dtc, dth);
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -1303,8 +1355,8 @@ __device__ __forceinline__ void finish_dt_reduction(const Mesh& m, double dtc, d
     __syncthreads();  // block_min2's shared scratch is reused
     block_min2(a, b);
     if (threadIdx.x == 0) {
-        m.result->dtcourant = accumulate ? fmin(a, m.result->dtcourant) : a;
-        m.result->dthydro = accumulate ? fmin(b, m.result->dthydro) : b;
+        m.result->dtcourant = a;
+        m.result->dthydro = b;
         m.result->blocks_done = 0u;
     }
 }

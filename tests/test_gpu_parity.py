@@ -104,6 +104,27 @@ def test_tiny_meshes_to_stoptime(lulesh, oracle_mod, problem):
         assert abs(d2.e[0] - e0) <= tol * abs(e0), precision
 
 
+@pytest.mark.parametrize("s,r,c,its", [(1, 11, 9, 1), (2, 21, 1, 20), (7, 16, 2, 30), (19, 21, 4, 12), (31, 11, 0, 6),
+                                       (38, 16, 1, 5), (46, 11, 3, 4), (62, 21, 1, 3)])
+def test_material_lanes_vs_oracle(lulesh, oracle_mod, s, r, c, its):
+    """The material phase gives an element with several EOS passes 1 to 32
+    lanes of a warp, more of them the fewer elements there are. Over sizes on
+    both sides of each choice, 1 to 100 passes per element and warps with
+    lanes left over, the exact variant keeps the oracle's bits (host loop and
+    drop-in call, whose slabs choose for themselves)."""
+    o = oracle_mod.Oracle(s, r, 1, c, threads=8, portable_cbrt=True)
+    assert o.run(its) == 0
+    dom, dev, n = _run_device(lulesh, s, r, 1, c, "fp64_exact", its)
+    assert n == o.cycle  # s=1 and s=2 reach the stoptime first
+    _assert_fields_equal(dom, o)
+    dom2 = lulesh.HostDomain(s, r, 1, c)
+    dev2 = lulesh.Device(dom2, "fp64_exact")
+    for _ in range(n):
+        dom2.time_increment()
+        dev2.leapfrog()
+    _assert_fields_equal(dom2, o)
+
+
 @pytest.mark.parametrize("s", [8, 10, 16, 20, 30, 45])
 def test_fp64_full_run_vs_reference(lulesh, golden_results, s):
     g = _golden(golden_results, s)

@@ -158,11 +158,7 @@ typedef struct lulesh_verify_result {
 /* Allocates device mirrors of the Domain arrays the step touches and uploads
  * all of them (constant topology and the full mutable state). Replaces the
  * reference's per-cycle malloc/free of temporaries (lulesh.cc:2017-2022,
- * lulesh.h:203-214): scratch is allocated once here. A LULESH_FP64 handle
- * also keeps each element's geometry between the kinematics and the next
- * force phase (48 doubles per element) and copies of the node coordinates
- * for lulesh_leapfrog: lulesh_batch_footprint(LULESH_FP64, s) plus
- * 24 (s + 1)^3 bytes in all. */
+ * lulesh.h:203-214): scratch is allocated once here. */
 int lulesh_dev_create(const lulesh_domain_view* host, int32_t precision, lulesh_dev** out);
 void lulesh_dev_destroy(lulesh_dev* dev);
 
@@ -197,10 +193,7 @@ int lulesh_dev_step(lulesh_dev* dev, double deltatime, double* dtcourant, double
  * dtcourant/dthydro into view->time. The cycle runs in slabs of element
  * planes and the copies overlap it: each slab's inputs upload ahead of its
  * force kernel, node fields go back behind the node update of each pair of
- * slabs, element fields behind each kinematics and material slab. With
- * LULESH_FP64, slabs whose node coordinates all equal those the previous
- * call left on the device reuse the element geometry it stored; the others
- * form it from the uploaded coordinates (same results either way). The
+ * slabs, element fields behind each kinematics and material slab. The
  * host arrays must stay untouched until the call returns; pin them
  * (lulesh_domain_pin) for full link bandwidth. On LULESH_EVOLUME (where the
  * reference exits) the host fields hold the partly advanced state and
@@ -255,8 +248,7 @@ typedef struct lulesh_batch_tuning {
  * problems at once. */
 int lulesh_batch_create(int32_t precision, uint64_t pool_bytes, int32_t max_slots, lulesh_batch** out);
 void lulesh_batch_destroy(lulesh_batch* b);
-/* Device bytes one s^3 problem takes in a pool of this precision (for
- * LULESH_FP64 including its element geometry, 384 bytes per element). */
+/* Device bytes one s^3 problem takes in a pool of this precision. */
 int lulesh_batch_footprint(int32_t precision, int32_t s, uint64_t* bytes);
 /* Builds the problem on the device in its pool block (the state
  * Domain::Domain makes, bit for bit; the region runs of the reference's

@@ -26,14 +26,8 @@ struct Launchers {
     int (*kinematics)(const Mesh&, double, cudaStream_t);
     int (*material)(const Mesh&, const MatPlan&, cudaStream_t);
     int (*forces_range)(const Mesh&, int, int, cudaStream_t);
-    // the resident loop's geometry form (fast double variant; else null):
-    // kinematics store the element geometry the next forces read
-    int (*forces_geo)(const Mesh&, cudaStream_t);
-    int (*kinematics_geo)(const Mesh&, double, cudaStream_t);
-    int (*geometry)(const Mesh&, cudaStream_t);
     // lulesh_leapfrog's kinematics slabs: elements [first, end)
     int (*kinematics_range)(const Mesh&, double, int, int, cudaStream_t);
-    int (*kinematics_geo_range)(const Mesh&, double, int, int, cudaStream_t);
 };
 
 Launchers launchers_for(int precision) {
@@ -42,16 +36,15 @@ Launchers launchers_for(int precision) {
             return {lulesh::fp64::launch_forces, lulesh::fp64::launch_nodes,
                     lulesh::fp64::launch_kinematics, lulesh::fp64::launch_material,
                     lulesh::fp64::launch_forces_range,
-                    lulesh::fp64::launch_forces_geo, lulesh::fp64::launch_kinematics_geo,
-                    lulesh::fp64::launch_geometry, lulesh::fp64::launch_kinematics_range, lulesh::fp64::launch_kinematics_geo_range};
+                    lulesh::fp64::launch_kinematics_range};
         case LULESH_FP64_EXACT:
             return {lulesh::fp64x::launch_forces, lulesh::fp64x::launch_nodes,
                     lulesh::fp64x::launch_kinematics, lulesh::fp64x::launch_material,
-                    lulesh::fp64x::launch_forces_range, nullptr, nullptr, nullptr, lulesh::fp64x::launch_kinematics_range, nullptr};
+                    lulesh::fp64x::launch_forces_range, lulesh::fp64x::launch_kinematics_range};
         default:
             return {lulesh::mixed::launch_forces, lulesh::mixed::launch_nodes,
                     lulesh::mixed::launch_kinematics, lulesh::mixed::launch_material,
-                    lulesh::mixed::launch_forces_range, nullptr, nullptr, nullptr, lulesh::mixed::launch_kinematics_range, nullptr};
+                    lulesh::mixed::launch_forces_range, lulesh::mixed::launch_kinematics_range};
     }
 }
 
@@ -105,16 +98,9 @@ struct lulesh_dev {
     cudaEvent_t tl_ev[LULESH_TL_MAX + 1] = {};
     int tl_n = 0;
     lulesh_timeline tl_last{};
-    int32_t* upload_flag = nullptr;  // [kLeapfrogSlabs] per-slab "host changed a coordinate" (arena)
     StepResult* slab_result = nullptr;  // [kLeapfrogSlabs] per material slab: dt minima and block counter
     int32_t* matOrderSlab = nullptr;           // [N_e] slab-major material order (arena)
     Launchers L{};
-    // m.geo holds the geometry of the current coordinates (set by the
-    // geometry form's kinematics and the geometry pass; cleared by anything
-    // that writes coordinates or runs the phases another way)
-    bool geo_valid = false;
-    // lulesh_leapfrog's copies of the uploaded coordinates (with m.geo)
-    double* stage[3] = {nullptr, nullptr, nullptr};
     // device-side timing (lulesh_dev_profile_begin/end)
     bool profiling = false;
     cudaEvent_t ev[2][5] = {};  // per-phase boundaries; two sets, for a cycle and the next one's forces
@@ -192,7 +178,6 @@ int check_view(const lulesh_domain_view* v) {
 // only measures.
 void carve_mesh(Mesh& m, Arena& a, int precision, int ne, int nn) {
     const bool mixed = precision == LULESH_MIXED;
-    m.geo = nullptr;
     for (double** f : {&m.x, &m.y, &m.z, &m.xd, &m.yd, &m.zd, &m.xdd, &m.ydd, &m.zdd, &m.fx, &m.fy,
                        &m.fz})
         *f = a.take<double>(nn);
@@ -223,8 +208,6 @@ void carve_mesh(Mesh& m, Arena& a, int precision, int ne, int nn) {
             for (double** f : {&m.fhx, &m.fhy, &m.fhz}) *f = a.take<double>(8 * size_t(ne));
         for (double** f : {&m.dvxi, &m.dveta, &m.dvzeta, &m.dxxi, &m.dxeta, &m.dxzeta})
             *f = a.take<double>(ne);
-        // the fast double variant's element geometry (kinematics -> next forces)
-        if (precision == LULESH_FP64) m.geo = a.take<double>(size_t(lulesh::kGeoWords) * ne);
     }
 }
 
@@ -277,8 +260,6 @@ void layout(lulesh_dev* d, Arena& a, int ne, int nn) {
     m.partials = a.take<lulesh::DtPartial>(size_t(lulesh::blocks_for(ne, lulesh::kMatBlock)) +
                                            kLeapfrogSlabs * mat_max_grid(1, d->sms));
     m.result = a.take<StepResult>(1);
-    for (double*& p : d->stage) p = d->L.forces_geo ? a.take<double>(nn) : nullptr;
-    d->upload_flag = a.take<int32_t>(kLeapfrogSlabs);
     d->slab_result = a.take<StepResult>(kLeapfrogSlabs);
     d->d_time = a.take<DevTime>(1);
     d->d_verify = a.take<double>(4);
@@ -417,20 +398,13 @@ int upload_mesh(const Mesh& m, const lulesh_domain_view* v, int precision, cudaS
 // current cycle's dt minima (lulesh_dev_run). `set` picks the profiling
 // events of the cycle (two sets: a cycle's and the next one's forces).
 //
-// The force phase: the error word cleared, the element geometry formed where
-// it is stale, forces.
+// The force phase: the error word cleared, forces.
 int queue_forces(lulesh_dev* d, int set) {
     const Mesh& m = d->m;
     const bool prof = d->profiling;
     CK(cudaMemsetAsync(&m.result->err, 0, 3 * sizeof(int32_t), d->stream));
-    const bool geo = d->L.forces_geo != nullptr;
     if (prof) CK(cudaEventRecord(d->ev[set][0], d->stream));
-    if (geo) {
-        if (!d->geo_valid) d->launches += d->L.geometry(m, d->stream);
-        d->launches += d->L.forces_geo(m, d->stream);
-    } else {
-        d->launches += d->L.forces(m, d->stream);
-    }
+    d->launches += d->L.forces(m, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][1], d->stream));
     return LULESH_OK;
 }
@@ -439,12 +413,10 @@ int queue_forces(lulesh_dev* d, int set) {
 int queue_rest(lulesh_dev* d, double dt, int set) {
     const Mesh& m = d->m;
     const bool prof = d->profiling;
-    const bool geo = d->L.forces_geo != nullptr;
     if (!d->ev_done) CK(cudaEventCreateWithFlags(&d->ev_done, cudaEventDisableTiming));
     d->launches += d->L.nodes(m, dt, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][2], d->stream));
-    d->launches += geo ? d->L.kinematics_geo(m, dt, d->stream) : d->L.kinematics(m, dt, d->stream);
-    d->geo_valid = geo;
+    d->launches += d->L.kinematics(m, dt, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][3], d->stream));
     d->launches += d->L.material(m, d->mat, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][4], d->stream));
@@ -485,11 +457,10 @@ int build_graph(lulesh_dev* d) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
     int k = 0;
-    const bool geo = d->L.forces_geo != nullptr;
     k += lulesh::launch_time_increment(d->d_time, gm.result, d->stream);
-    k += geo ? d->L.forces_geo(gm, d->stream) : d->L.forces(gm, d->stream);
+    k += d->L.forces(gm, d->stream);
     k += d->L.nodes(gm, 0.0, d->stream);
-    k += geo ? d->L.kinematics_geo(gm, 0.0, d->stream) : d->L.kinematics(gm, 0.0, d->stream);
+    k += d->L.kinematics(gm, 0.0, d->stream);
     k += d->L.material(gm, d->mat, d->stream);
     k += lulesh::launch_time_finish(d->d_time, gm.result, d->stream);
     cudaError_t ce = cudaStreamEndCapture(d->stream, &g);
@@ -662,7 +633,6 @@ int lulesh_dev_verify(lulesh_dev* d, int32_t cycle, lulesh_verify_result* out) {
 int lulesh_dev_upload(lulesh_dev* d, const lulesh_domain_view* v, uint32_t mask) {
     if (!d || !v || v->numElem != d->m.numElem || v->numNode != d->m.numNode) return LULESH_EINVAL;
     if (mask & LULESH_F_MESH) return LULESH_EINVAL;  // the mesh is fixed at creation
-    if (mask & LULESH_F_POS) d->geo_valid = false;  // the element geometry follows the coordinates
     for (const Copy& c : groups(d->m, v, mask)) {
         if (!c.host) return LULESH_EINVAL;
         CK(cudaMemcpyAsync(c.dev, c.host, c.bytes, cudaMemcpyHostToDevice, d->stream));
@@ -698,12 +668,6 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     if (!d || !v || !v->time || v->numElem != d->m.numElem || v->numNode != d->m.numNode)
         return LULESH_EINVAL;
     if (!(v->time->deltatime > 0.0)) return LULESH_EINVAL;
-    // The coordinates come from the host buffers. With the geometry form they
-    // upload into copies, and slabs whose nodes the host left as the previous
-    // step made them reuse the geometry that step stored.
-    const bool geo = d->L.forces_geo != nullptr;
-    const bool have_geo = geo && d->geo_valid;
-    d->geo_valid = false;
     const auto in = groups(d->m, v, LULESH_F_STEP_IN);
     const auto out_nodes = groups(d->m, v, LULESH_F_POS | LULESH_F_VEL | LULESH_F_ACC | LULESH_F_FORCE);
     const auto out_kin = groups(d->m, v, LULESH_F_V | LULESH_F_KIN);
@@ -769,7 +733,6 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         n_hi[sl] = cube ? (p1 + 1) * plane_n : m.numNode;
     }
     CK(cudaMemsetAsync(&m.result->err, 0, 3 * sizeof(int32_t), d->stream));
-    if (have_geo) CK(cudaMemsetAsync(d->upload_flag, 0, sizeof(int32_t) * slabs, d->stream));
     CK(cudaMemsetAsync(d->slab_result, 0, sizeof(StepResult) * slabs, d->stream));
     const auto t_call = std::chrono::steady_clock::now();
     d->tl_n = 0;
@@ -808,8 +771,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     };
 
     // Node update of nodes [a, b) on the node stream after both compute
-    // streams' work so far, then those node fields go down. With the
-    // geometry form the positions advanced are the uploaded copies.
+    // streams' work so far, then those node fields go down.
     auto node_range = [&](int64_t a, int64_t b, cudaEvent_t ev, int r) -> int {
         CK(cudaEventRecord(d->ev_s1, d->stream));
         CK(cudaEventRecord(d->ev_s2, d->stream2));
@@ -826,9 +788,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         mn.nodeElemStart += a;
         if (mn.pxp)
             for (float2** f : {&mn.pxp, &mn.pyp, &mn.pzp, &mn.vxp, &mn.vyp, &mn.vzp}) *f += a;
-        d->launches += geo ? lulesh::fp64::launch_nodes_upload(mn, dt, d->stage[0] + a, d->stage[1] + a,
-                                                               d->stage[2] + a, d->nstream)
-                           : d->L.nodes(mn, dt, d->nstream);
+        d->launches += d->L.nodes(mn, dt, d->nstream);
         CK(cudaEventRecord(ev, d->nstream));
         if (int st = mark(LULESH_TL_NODES, r, d->nstream)) return st;
         CK(cudaStreamWaitEvent(d->mstream, ev, 0));
@@ -858,11 +818,6 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
             const bool node = c.bytes == sizeof(double) * size_t(m.numNode);
             const int64_t a = node ? node_done : e0, b = node ? n1 : e1;
             double* dst = static_cast<double*>(c.dev);
-            if (geo) {
-                if (dst == m.x) dst = d->stage[0];
-                else if (dst == m.y) dst = d->stage[1];
-                else if (dst == m.z) dst = d->stage[2];
-            }
             if (b > a)
                 CK(cudaMemcpyAsync(dst + a, static_cast<const double*>(c.host) + a, sizeof(double) * size_t(b - a),
                                    cudaMemcpyHostToDevice, d->cstream));
@@ -878,21 +833,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
             CK(cudaEventRecord(d->ev_mir[sl], cs));
             if (sl > 0) CK(cudaStreamWaitEvent(cs, d->ev_mir[sl - 1], 0));
         }
-        if (geo && have_geo) {
-            // the slab's nodes against the device's own: the stored geometry
-            // where none changed, else the geometry of the uploaded values
-            int32_t* flag = d->upload_flag + sl;
-            d->launches += lulesh::fp64::launch_upload_check(m, d->stage[0], d->stage[1], d->stage[2],
-                                                             int(n_lo[sl]), int(n1), flag, cs);
-            d->launches += lulesh::fp64::launch_forces_geo_unless(m, int(e0), int(e1), flag, cs);
-            d->launches += lulesh::fp64::launch_forces_upload(m, d->stage[0], d->stage[1], d->stage[2], int(e0),
-                                                              int(e1), flag, cs);
-        } else if (geo) {
-            d->launches += lulesh::fp64::launch_forces_upload(m, d->stage[0], d->stage[1], d->stage[2], int(e0),
-                                                              int(e1), nullptr, cs);
-        } else {
-            d->launches += d->L.forces_range(m, int(e0), int(e1), cs);
-        }
+        d->launches += d->L.forces_range(m, int(e0), int(e1), cs);
         if (int st = mark(LULESH_TL_FORCES, sl, cs)) return st;
         node_done = n1;
     }
@@ -907,8 +848,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     for (int k = 0; k < slabs; k += 2) {
         const int64_t e0 = e_lo[k], e1 = e_hi[std::min(k + 1, slabs - 1)];
         cudaStream_t cs = (k & 2) ? d->stream2 : d->stream;
-        d->launches += geo ? d->L.kinematics_geo_range(m, dt, int(e0), int(e1), cs)
-                           : d->L.kinematics_range(m, dt, int(e0), int(e1), cs);
+        d->launches += d->L.kinematics_range(m, dt, int(e0), int(e1), cs);
         if (int st = elem_down(out_kin, e0, e1, d->ev_kin[k], cs, LULESH_TL_KIN, k / 2)) return st;
     }
     // the material phase reads the kinematics of both compute streams (the
@@ -958,7 +898,6 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     }
     v->time->dtcourant = dtc;
     v->time->dthydro = dth;
-    d->geo_valid = geo;
     return LULESH_OK;
 }
 
@@ -1029,13 +968,6 @@ int lulesh_dev_run_graph(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycle
     const int32_t start = ts->cycle;
     CK(cudaMemsetAsync(d->m.result, 0, sizeof(StepResult), d->stream));
     CK(cudaMemcpyAsync(d->d_time, d->h_time, sizeof(DevTime), cudaMemcpyHostToDevice, d->stream));
-    if (d->L.forces_geo) {
-        if (!d->geo_valid) {
-            d->launches += d->L.geometry(d->m, d->stream);
-            CK(cudaGetLastError());
-        }
-        d->geo_valid = true;
-    }
     for (;;) {
         for (int k = 0; k < sync_every; ++k) {
             CK(cudaGraphLaunch(d->graph, d->stream));
@@ -1062,7 +994,6 @@ int lulesh_dev_run_graph(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycle
 int lulesh_dev_phase(lulesh_dev* d, int32_t phase, double dt) {
     if (!d) return LULESH_EINVAL;
     const Mesh& m = d->m;
-    d->geo_valid = false;  // the single phases use the forming kernels
     CK(cudaMemsetAsync(&m.result->err, 0, 3 * sizeof(int32_t), d->stream));
     switch (phase) {
         case LULESH_PHASE_FORCES: d->launches += d->L.forces(m, d->stream); break;

@@ -19,6 +19,7 @@
 //                    (lulesh.cc:1420-1974)
 #pragma once
 
+#include "block_fixed.cuh"
 #include "step_math.cuh"
 
 namespace lulesh {
@@ -86,90 +87,40 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
     }
 }
 #else
-// Element geometry (fast variant): everything the force phase derives from
-// the corner coordinates alone. J holds the body-diagonal sums (8 x the
-// centre Jacobian, columns along xi, eta, zeta) and h the hourglass mode sums
-// of each coordinate, both from one Walsh-Hadamard transform; c the cofactors
-// of J; fa the six faces' t x s, unscaled. The kinematics phase forms the
-// same geometry of the updated coordinates for its own needs (J and c for
-// the Q gradients and vdov, fa for the characteristic length) and, in the
-// resident loop, stores it for the next cycle's force phase, whose
-// coordinates those are. Every path forms it with the same operations, so
-// stored and recomputed geometry are the same bits.
-struct ElemGeo {
+// Corner forces of element i in double: the path of the elements that do not
+// fit the block fixed point of forces_elem (coordinates, velocities or
+// scalars that are infinite, NaN or of extreme magnitude, a centre Jacobian
+// determinant near zero). Stress plus hourglass, summed in registers and
+// stored once (corner-major fsx, fsy, fsz). The zero test on the centre
+// Jacobian's determinant (lulesh.cc:817-821) is taken in another summation
+// order: zero for the same collapsed elements, though a near-singular element
+// may round differently. The hourglass vectors come from the volume gradient
+// (192 x dV/dx_k) and the mode sums scaled by volinv / 192. The stress force
+// (p + q) n enters through the face vectors scaled by (p + q) / 8 and starts
+// each corner's hourglass multiply-add chain. Elements that fail a test store
+// nothing: the step reports the error and its state is not used.
+__device__ __noinline__ void forces_double(const Mesh& m, int i) {
+    const size_t N = (size_t)m.numElem;
+    int nl[8];
+    load_nodelist(m.nodelist, i, nl);
     double J[3][3], c[3][3], h[3][4], fa[6][3];
-};
-#define LULESH_GEO_FORM 1
-
-__device__ __forceinline__ void elem_geometry(const double x[8], const double y[8], const double z[8],
-                                              ElemGeo& g) {
-    walsh7(x, g.J[0], g.h[0]);
-    walsh7(y, g.J[1], g.h[1]);
-    walsh7(z, g.J[2], g.h[2]);
-    cofactors(g.J, g.c);
-    face_txs<0, 1, 2, 3>(x, y, z, g.fa[0]);
-    face_txs<0, 4, 5, 1>(x, y, z, g.fa[1]);
-    face_txs<1, 5, 6, 2>(x, y, z, g.fa[2]);
-    face_txs<2, 6, 7, 3>(x, y, z, g.fa[3]);
-    face_txs<3, 7, 4, 0>(x, y, z, g.fa[4]);
-    face_txs<4, 7, 6, 5>(x, y, z, g.fa[5]);
-}
-
-// Mesh::geo word q of element i is geo[q * numElem + i]: J, c, h, fa in
-// row-major order.
-__device__ __forceinline__ void geo_store(const Mesh& m, int i, const ElemGeo& g) {
-    const size_t N = (size_t)m.numElem;
-    double* o = m.geo + i;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            o[(3 * a + d) * N] = g.J[a][d];
-            o[(9 + 3 * a + d) * N] = g.c[a][d];
-        }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) o[(18 + 4 * a + k) * N] = g.h[a][k];
-#pragma unroll
-    for (int f = 0; f < 6; ++f)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[(30 + 3 * f + d) * N] = g.fa[f][d];
-}
-__device__ __forceinline__ void geo_load(const Mesh& m, int i, ElemGeo& g) {
-    const size_t N = (size_t)m.numElem;
-    const double* o = m.geo + i;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            g.J[a][d] = LD(o + (3 * a + d) * N);
-            g.c[a][d] = LD(o + (9 + 3 * a + d) * N);
-        }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) g.h[a][k] = LD(o + (18 + 4 * a + k) * N);
-#pragma unroll
-    for (int f = 0; f < 6; ++f)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) g.fa[f][d] = LD(o + (30 + 3 * f + d) * N);
-}
-
-// Stress plus hourglass corner force of element i from its geometry, summed
-// in registers and stored once (corner-major fsx, fsy, fsz). The zero test
-// on the centre Jacobian's determinant (lulesh.cc:817-821) is taken in
-// another summation order: zero for the same collapsed elements, though a
-// near-singular element may round differently. The hourglass vectors come
-// from the volume gradient (192 x dV/dx_k) and the mode sums scaled by
-// volinv / 192. The stress force (p + q) n enters through the face vectors
-// scaled by (p + q) / 8 and starts each corner's hourglass multiply-add
-// chain. Elements that fail a test store nothing: the step reports the
-// error and its state is not used.
-__device__ __forceinline__ void forces_from_geo(const Mesh& m, int i, const int nl[8], const ElemGeo& g) {
-    const size_t N = (size_t)m.numElem;
-    if (f_is_zero(g.J[0][0] * g.c[0][0] + g.J[1][0] * g.c[1][0] + g.J[2][0] * g.c[2][0]))
-        raise_error(m.result, i, PHASE_FORCES);
+    {
+        double x[8], y[8], z[8];
+        gather8(m.x, nl, x);
+        gather8(m.y, nl, y);
+        gather8(m.z, nl, z);
+        walsh7(x, J[0], h[0]);
+        walsh7(y, J[1], h[1]);
+        walsh7(z, J[2], h[2]);
+        cofactors(J, c);
+        face_txs<0, 1, 2, 3>(x, y, z, fa[0]);
+        face_txs<0, 4, 5, 1>(x, y, z, fa[1]);
+        face_txs<1, 5, 6, 2>(x, y, z, fa[2]);
+        face_txs<2, 6, 7, 3>(x, y, z, fa[3]);
+        face_txs<3, 7, 4, 0>(x, y, z, fa[4]);
+        face_txs<4, 7, 6, 5>(x, y, z, fa[5]);
+    }
+    if (f_is_zero(J[0][0] * c[0][0] + J[1][0] * c[1][0] + J[2][0] * c[2][0])) raise_error(m.result, i, PHASE_FORCES);
     const double determ = LD(m.volo + i) * LD(m.v + i);
     if (f_le(determ, 0.0)) {
         raise_error(m.result, i, PHASE_FORCES);
@@ -177,26 +128,23 @@ __device__ __forceinline__ void forces_from_geo(const Mesh& m, int i, const int 
     }
     double hg[8][4];
     {
-        double gx[8], gy[8], gz[8], hx[4], hy[4], hz[4];
-        volume_gradient(g.J, g.c, g.h[0], g.h[1], g.h[2], gx, gy, gz);
+        double gx[8], gy[8], gz[8];
+        volume_gradient(J, c, h[0], h[1], h[2], gx, gy, gz);
         const double sc = rcp(determ) * (1.0 / 192.0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            hx[k] = pmul(g.h[0][k], sc);
-            hy[k] = pmul(g.h[1][k], sc);
-            hz[k] = pmul(g.h[2][k], sc);
-        }
-        hourgam_mode_h<0>(hg, hx[0], hy[0], hz[0], gx, gy, gz);
-        hourgam_mode_h<1>(hg, hx[1], hy[1], hz[1], gx, gy, gz);
-        hourgam_mode_h<2>(hg, hx[2], hy[2], hz[2], gx, gy, gz);
-        hourgam_mode_h<3>(hg, hx[3], hy[3], hz[3], gx, gy, gz);
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) h[a][k] = pmul(h[a][k], sc);
+        hourgam_mode_h<0>(hg, h[0][0], h[1][0], h[2][0], gx, gy, gz);
+        hourgam_mode_h<1>(hg, h[0][1], h[1][1], h[2][1], gx, gy, gz);
+        hourgam_mode_h<2>(hg, h[0][2], h[1][2], h[2][2], gx, gy, gz);
+        hourgam_mode_h<3>(hg, h[0][3], h[1][3], h[2][3], gx, gy, gz);
     }
-    double fa[6][3];
     const double scale = (LD(m.p + i) + LD(m.q + i)) * kInvNormalScale;
 #pragma unroll
     for (int f = 0; f < 6; ++f)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) fa[f][d] = pmul(g.fa[f][d], scale);
+        for (int d = 0; d < 3; ++d) fa[f][d] = pmul(fa[f][d], scale);
     const double coefficient = -m.prm.hgcoef * 0.01 * LD(m.ss + i) * LD(m.elemMass + i) * rcbrt_pos(determ);
     double* outs[3] = {m.fsx, m.fsy, m.fsz};
     const double* vels[3] = {m.xd, m.yd, m.zd};
@@ -211,67 +159,51 @@ __device__ __forceinline__ void forces_from_geo(const Mesh& m, int i, const int 
     }
 }
 
-// Forces of element i from its coordinates (geometry formed here).
+// Corner forces of element i, stress plus hourglass, in block fixed point
+// (block_fixed.cuh) and stored as forces_double stores them.
 __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
+    const size_t N = (size_t)m.numElem;
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
-    ElemGeo g;
+    bf::ForceGeo g;
+    bool ok = true;
     {
-        double x[8], y[8], z[8];
+        bf::Sums s;
+        double x[8];
         gather8(m.x, nl, x);
-        gather8(m.y, nl, y);
-        gather8(m.z, nl, z);
-        elem_geometry(x, y, z, g);
+        ok &= bf::axis_sums<57>(x, 0, s);
+        gather8(m.y, nl, x);
+        ok &= bf::axis_sums<57>(x, 1, s);
+        gather8(m.z, nl, x);
+        ok &= bf::axis_sums<57>(x, 2, s);
+        ok &= bf::force_geometry(s, g);
     }
-    forces_from_geo(m, i, nl, g);
-}
-
-// Forces of element i from the stored geometry.
-__device__ __forceinline__ void forces_geo_elem(const Mesh& m, int i) {
-    int nl[8];
-    load_nodelist(m.nodelist, i, nl);
-    ElemGeo g;
-    geo_load(m, i, g);
-    forces_from_geo(m, i, nl, g);
-}
-
-// Forces of element i in lulesh_leapfrog with the geometry formed from the
-// coordinates just uploaded from the host (sx, sy, sz), the step's own.
-__device__ __forceinline__ void forces_upload_elem(const Mesh& m, const double* __restrict__ sx,
-                                                   const double* __restrict__ sy,
-                                                   const double* __restrict__ sz, int i) {
-    int nl[8];
-    load_nodelist(m.nodelist, i, nl);
-    ElemGeo g;
-    {
-        double x[8], y[8], z[8];
-        gather8(sx, nl, x);
-        gather8(sy, nl, y);
-        gather8(sz, nl, z);
-        elem_geometry(x, y, z, g);
+    const double determ = LD(m.volo + i) * LD(m.v + i);
+    ok &= f_gt(determ, 0.0);
+    bf::ForceScale sc;
+    const double coefficient = -m.prm.hgcoef * 0.01 * LD(m.ss + i) * LD(m.elemMass + i) * rcbrt_pos(determ);
+    ok &= bf::force_scale(g, rcp(determ) * (1.0 / 192.0), coefficient, LD(m.p + i) + LD(m.q + i), sc);
+    // one copy of the axis' code: three would not fit the instruction cache
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {
+        int64_t n[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) n[d] = a == 0 ? g.n[d][0] : a == 1 ? g.n[d][1] : g.n[d][2];
+        const double* v = a == 0 ? m.xd : a == 1 ? m.yd : m.zd;
+        double* out = a == 0 ? m.fsx : a == 1 ? m.fsy : m.fsz;
+        double vel[8], f[8];
+        gather8(v, nl, vel);
+        ok &= bf::force_axis(g, sc, n, a == 0 ? g.unit[0] : a == 1 ? g.unit[1] : g.unit[2], vel, f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) out[k * N + i] = f[k];
     }
-    forces_from_geo(m, i, nl, g);
-}
-
-// Stores the geometry of element i's current coordinates.
-__device__ __forceinline__ void geometry_elem(const Mesh& m, int i) {
-    int nl[8];
-    load_nodelist(m.nodelist, i, nl);
-    double x[8], y[8], z[8];
-    gather8(m.x, nl, x);
-    gather8(m.y, nl, y);
-    gather8(m.z, nl, z);
-    ElemGeo g;
-    elem_geometry(x, y, z, g);
-    geo_store(m, i, g);
+    if (!ok) forces_double(m, i);
 }
 #endif
 
 // Node n: gather in CSR order, stress then hourglass per corner
-// (combineVolumeForcesTaskFunc, lulesh.cc:838-862), then the node update
-// (of positions px, py, pz when given, see node_update).
-__device__ __forceinline__ void nodes_node(const Mesh& m, int n, double dt, const double* px = nullptr,
-                                           const double* py = nullptr, const double* pz = nullptr) {
+// (combineVolumeForcesTaskFunc, lulesh.cc:838-862), then the node update.
+__device__ __forceinline__ void nodes_node(const Mesh& m, int n, double dt) {
     const size_t N = (size_t)m.numElem;
     const int b = LD(m.nodeElemStart + n), e = LD(m.nodeElemStart + n + 1);
     double fx = 0.0, fy = 0.0, fz = 0.0;
@@ -291,7 +223,7 @@ __device__ __forceinline__ void nodes_node(const Mesh& m, int n, double dt, cons
         fz += LD(m.fsz + idx);
 #endif
     }
-    node_update(m, n, fx, fy, fz, dt, px, py, pz);
+    node_update(m, n, fx, fy, fz, dt);
 }
 
 // CalcKinematicsForElemsTask (lulesh.cc:1169-1275) and
@@ -326,45 +258,28 @@ __device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt)
     update_volume(m, i, vold, relv);
 }
 #else
-// Characteristic length 4 V / sqrt(largest face measure) from the faces'
-// t x s: the reference's face measure is 4 |t x s|^2 (Lagrange's identity),
-// so the length is 2 V / sqrt(max |t x s|^2).
-__device__ __forceinline__ double char_length_faces(const double fa[6][3], double volume) {
-    double cl = fma(fa[0][2], fa[0][2], fma(fa[0][1], fa[0][1], pmul(fa[0][0], fa[0][0])));
-#pragma unroll
-    for (int f = 1; f < 6; ++f)
-        cl = nonneg_max(cl, fma(fa[f][2], fa[f][2], fma(fa[f][1], fa[f][1], pmul(fa[f][0], fa[f][0]))));
-    return div_sqrt(2.0 * volume, cl);
-}
-
-// Kinematics of element i; STORE_GEO: also store the element geometry of the
-// updated coordinates for the next force phase (Mesh::geo).
-template <bool STORE_GEO>
-__device__ __forceinline__ void kinematics_fast(const Mesh& m, int i, double dt) {
+// Kinematics of element i in double: the path of the elements that do not fit
+// the block fixed point of kinematics_elem. The characteristic length
+// 4 V / sqrt(largest face measure) comes from the faces' t x s: the
+// reference's face measure is 4 |t x s|^2 (Lagrange's identity).
+__device__ __noinline__ void kinematics_double(const Mesh& m, int i, double dt) {
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
-    double relv, vold;
-    ElemGeo g;
-    {
-        double x[8], y[8], z[8];
-        gather8(m.x, nl, x);
-        gather8(m.y, nl, y);
-        gather8(m.z, nl, z);
-        const double volume = hex_volume(x, y, z);
-        relv = quot_refined(volume, LD(m.volo + i));
-        vold = m.v[i];
-        m.vnew[i] = relv;
-        m.delv[i] = relv - vold;
-        elem_geometry(x, y, z, g);
-        m.arealg[i] = char_length_faces(g.fa, volume);
-    }
-    if (STORE_GEO) geo_store(m, i, g);
-    double xv[8], yv[8], zv[8];
+    double x[8], y[8], z[8], xv[8], yv[8], zv[8];
+    gather8(m.x, nl, x);
+    gather8(m.y, nl, y);
+    gather8(m.z, nl, z);
+    const double volume = hex_volume(x, y, z);
+    const double relv = quot_refined(volume, LD(m.volo + i));
+    const double vold = m.v[i];
+    m.vnew[i] = relv;
+    m.delv[i] = relv - vold;
+    m.arealg[i] = char_length(x, y, z, volume);
     gather8(m.xd, nl, xv);
     gather8(m.yd, nl, yv);
     gather8(m.zd, nl, zv);
     double gr[6];
-    m.vdov[i] = gradients_vdov_xc(g.J, g.c, xv, yv, zv, pmul(LD(m.volo + i), relv), 0.5 * dt, gr);
+    m.vdov[i] = gradients_vdov(x, y, z, xv, yv, zv, pmul(LD(m.volo + i), relv), 0.5 * dt, gr);
     m.dvxi[i] = gr[0];
     m.dveta[i] = gr[1];
     m.dvzeta[i] = gr[2];
@@ -373,7 +288,70 @@ __device__ __forceinline__ void kinematics_fast(const Mesh& m, int i, double dt)
     m.dxzeta[i] = gr[5];
     update_volume(m, i, vold, relv);
 }
-__device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt) { kinematics_fast<false>(m, i, dt); }
+
+// Ulps (halved below 1) that the relative volume of an element at rest may
+// be off 1, see kinematics_elem.
+constexpr unsigned long long kUlpsBelow = 8, kUlpsAbove = 4;
+
+// Kinematics of element i in block fixed point (block_fixed.cuh). The
+// volume is closer to the exact one than the double formula that made volo,
+// so an element that has not moved would come out a few ulps from 1; a
+// relative volume within the rounding of that formula of 1 is 1, as in the
+// reference (a delv of an ulp would send its EOS passes down the compressing
+// branch).
+__device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt) {
+    int nl[8];
+    load_nodelist(m.nodelist, i, nl);
+    bf::KinGeo g;
+    bf::KinVel kv;
+    bool ok = true;
+    {
+        bf::Sums s;
+        double x[8];
+        gather8(m.x, nl, x);
+        ok &= bf::axis_sums<58>(x, 0, s);
+        gather8(m.y, nl, x);
+        ok &= bf::axis_sums<58>(x, 1, s);
+        gather8(m.z, nl, x);
+        ok &= bf::axis_sums<58>(x, 2, s);
+        ok &= bf::kin_geometry(s, g);
+    }
+    {
+        bf::VelSums v;
+        double x[8];
+        gather8(m.xd, nl, x);
+        ok &= bf::vel_sums(x, 0, v);
+        gather8(m.yd, nl, x);
+        ok &= bf::vel_sums(x, 1, v);
+        gather8(m.zd, nl, x);
+        ok &= bf::vel_sums(x, 2, v);
+        bf::kin_velocity(g, v, kv);
+    }
+    if (!ok) {
+        kinematics_double(m, i, dt);
+        return;
+    }
+    const double volo = LD(m.volo + i), vold = m.v[i];
+    const double volume = g.vol192 * (1.0 / 192.0);
+    double relv = quot_refined(volume, volo);
+    if (static_cast<unsigned long long>(dbits(relv) - dbits(1.0) + kUlpsBelow) <= kUlpsBelow + kUlpsAbove) relv = 1.0;
+    m.vnew[i] = relv;
+    m.delv[i] = relv - vold;
+    m.arealg[i] = pmul(16.0 * volume, rsqrt(g.face2));
+    const double vol = pmul(volo, relv), vol16 = 16.0 * vol;
+    const double n64 = rcp(vol + 1.e-36) * 0.015625;
+    m.dxxi[i] = pmul(vol16, rsqrt(g.cc[0] + 256.0 * 1.e-36));
+    m.dxeta[i] = pmul(vol16, rsqrt(g.cc[1] + 256.0 * 1.e-36));
+    m.dxzeta[i] = pmul(vol16, rsqrt(g.cc[2] + 256.0 * 1.e-36));
+    m.dvxi[i] = pmul(kv.cv[0], n64);
+    m.dveta[i] = pmul(kv.cv[1], n64);
+    m.dvzeta[i] = pmul(kv.cv[2], n64);
+    const double t = 0.5 * dt, b = kv.cv[0] + kv.cv[1] + kv.cv[2];
+    const double num = fma(t, fma(3.0 * t, kv.detv, -2.0 * kv.ak), b);
+    const double den = fma(-t, fma(-t, fma(-t, kv.detv, kv.ak), b), g.det);
+    m.vdov[i] = quot(num, den);
+    update_volume(m, i, vold, relv);
+}
 #endif
 
 // Material phase of an element by several lanes (material_share).
@@ -384,9 +362,16 @@ __device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int l
 
 // --- single-problem kernels -------------------------------------------------
 
+// Resident blocks of 128 per SM asked of the compiler. The fast variant's
+// block fixed point is bound by instruction issue and its dependencies, with
+// room for warps up to 128 registers: at s=150 k_forces takes 1.21, 0.98,
+// 0.92 ms with 2, 3, 4 blocks (4 spills a little), k_kinematics 1.13, 0.87,
+// 0.83 (5: 0.85).
+constexpr int kForceBlocks = LULESH_EXACT ? 1 : 4, kKinBlocks = LULESH_EXACT ? 1 : 4;
+
 // all elements, or (RANGED) elements [first, end)
 template <bool RANGED>
-__global__ void __launch_bounds__(kForceBlock) k_forces(Mesh m, int first, int end) {
+__global__ void __launch_bounds__(kForceBlock, kForceBlocks) k_forces(Mesh m, int first, int end) {
     if (m.dtime && !m.dtime->active) return;
     const int i = (RANGED ? first : 0) + blockIdx.x * blockDim.x + threadIdx.x;
     if (i < (RANGED ? end : m.numElem)) forces_elem(m, i);
@@ -403,7 +388,7 @@ __global__ void __launch_bounds__(kNodeBlock) k_nodes(Mesh m, double dt) {
 
 // all elements, or (RANGED) elements [first, end)
 template <bool RANGED>
-__global__ void __launch_bounds__(kKinBlock) k_kinematics(Mesh m, double dt, int first, int end) {
+__global__ void __launch_bounds__(kKinBlock, kKinBlocks) k_kinematics(Mesh m, double dt, int first, int end) {
     if (m.dtime) {
         if (!m.dtime->active) return;
         dt = m.dtime->deltatime;
@@ -411,72 +396,6 @@ __global__ void __launch_bounds__(kKinBlock) k_kinematics(Mesh m, double dt, int
     const int i = (RANGED ? first : 0) + blockIdx.x * blockDim.x + threadIdx.x;
     if (i < (RANGED ? end : m.numElem)) kinematics_elem(m, i, dt);
 }
-
-#if !LULESH_EXACT
-// The resident loop's form: forces from the stored geometry, kinematics that
-// store it, and the pass that forms it from the current coordinates.
-__global__ void __launch_bounds__(kForceBlock) k_forces_geo(Mesh m) {
-    if (m.dtime && !m.dtime->active) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m.numElem) forces_geo_elem(m, i);
-}
-// At least 3 blocks of 128 per SM (at most 168 registers): with the
-// integer-pipe products the compiler's own choice, 240 registers and 2
-// blocks, left the FP64 pipe waiting (2.09 -> 2.00 ms at s=150).
-template <bool RANGED>
-__global__ void __launch_bounds__(kKinBlock, 3) k_kinematics_geo(Mesh m, double dt, int first, int end) {
-    if (m.dtime) {
-        if (!m.dtime->active) return;
-        dt = m.dtime->deltatime;
-    }
-    const int i = (RANGED ? first : 0) + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (RANGED ? end : m.numElem)) kinematics_fast<true>(m, i, dt);
-}
-
-// lulesh_leapfrog's check of one slab: *flag = 1 when the host's uploaded
-// coordinates (sx, sy, sz) of a node in [first, end) differ, bit for bit,
-// from the device's own (the previous step's results). Every thread of a
-// warp reaches the vote; the flag starts at 0 (cleared by the host call).
-__global__ void __launch_bounds__(kNodeBlock) k_upload_check(Mesh m, const double* sx, const double* sy,
-                                                              const double* sz, int first, int end, int* flag) {
-    const int n = first + blockIdx.x * blockDim.x + threadIdx.x;
-    bool differs = false;
-    if (n < end)
-        differs = dbits(LD(sx + n)) != dbits(LD(m.x + n)) || dbits(LD(sy + n)) != dbits(LD(m.y + n)) ||
-                  dbits(LD(sz + n)) != dbits(LD(m.z + n));
-    if (__any_sync(0xffffffffu, differs) && (threadIdx.x & 31) == 0) *flag = 1;
-}
-// lulesh_leapfrog's node phase: every node, the positions advanced being the
-// uploaded copies sx, sy, sz (the step's own coordinates).
-__global__ void __launch_bounds__(kNodeBlock) k_nodes_upload(Mesh m, double dt, const double* sx,
-                                                              const double* sy, const double* sz) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n < m.numNode) nodes_node(m, n, dt, sx, sy, sz);
-}
-// Forces of elements [first, end) from the stored geometry, unless the
-// slab's check found a changed node (*flag).
-__global__ void __launch_bounds__(kForceBlock) k_forces_geo_unless(Mesh m, int first, int end,
-                                                                    const int* flag) {
-    if (*flag) return;
-    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < end) forces_geo_elem(m, i);
-}
-// Forces of elements [first, end) with the geometry formed from the uploaded
-// coordinates: always (flag null) or when the slab's check found a changed
-// node (*flag). The two kernels give the same bits for an unchanged element
-// (the stored geometry is formed by the same function from the same values).
-__global__ void __launch_bounds__(kForceBlock) k_forces_upload(Mesh m, const double* sx, const double* sy,
-                                                                const double* sz, int first, int end,
-                                                                const int* flag) {
-    if (flag && !*flag) return;
-    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < end) forces_upload_elem(m, sx, sy, sz, i);
-}
-__global__ void __launch_bounds__(kForceBlock) k_geometry(Mesh m) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m.numElem) geometry_elem(m, i);
-}
-#endif
 
 // Elements visited in repeat-count order so a warp's lanes run the same
 // number of EOS passes; the dt minima end in a last-block reduction.
@@ -531,47 +450,6 @@ int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s) {
     else k_material<false><<<plan.grid, kMatBlock, 0, s>>>(m, plan);
     return 1;
 }
-#if !LULESH_EXACT
-int launch_forces_geo(const Mesh& m, cudaStream_t s) {
-    k_forces_geo<<<blocks_for(m.numElem, kForceBlock), kForceBlock, 0, s>>>(m);
-    return 1;
-}
-int launch_kinematics_geo(const Mesh& m, double dt, cudaStream_t s) {
-    k_kinematics_geo<false><<<blocks_for(m.numElem, kKinBlock), kKinBlock, 0, s>>>(m, dt, 0, m.numElem);
-    return 1;
-}
-int launch_kinematics_geo_range(const Mesh& m, double dt, int first, int end, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_kinematics_geo<true><<<blocks_for(end - first, kKinBlock), kKinBlock, 0, s>>>(m, dt, first, end);
-    return 1;
-}
-int launch_nodes_upload(const Mesh& m, double dt, const double* sx, const double* sy, const double* sz,
-                        cudaStream_t s) {
-    k_nodes_upload<<<blocks_for(m.numNode, kNodeBlock), kNodeBlock, 0, s>>>(m, dt, sx, sy, sz);
-    return 1;
-}
-int launch_upload_check(const Mesh& m, const double* sx, const double* sy, const double* sz, int first, int end,
-                        int32_t* flag, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_upload_check<<<blocks_for(end - first, kNodeBlock), kNodeBlock, 0, s>>>(m, sx, sy, sz, first, end, flag);
-    return 1;
-}
-int launch_forces_geo_unless(const Mesh& m, int first, int end, const int32_t* flag, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_forces_geo_unless<<<blocks_for(end - first, kForceBlock), kForceBlock, 0, s>>>(m, first, end, flag);
-    return 1;
-}
-int launch_forces_upload(const Mesh& m, const double* sx, const double* sy, const double* sz, int first, int end,
-                         const int32_t* flag, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_forces_upload<<<blocks_for(end - first, kForceBlock), kForceBlock, 0, s>>>(m, sx, sy, sz, first, end, flag);
-    return 1;
-}
-int launch_geometry(const Mesh& m, cudaStream_t s) {
-    k_geometry<<<blocks_for(m.numElem, kForceBlock), kForceBlock, 0, s>>>(m);
-    return 1;
-}
-#endif
 
 }  // namespace LULESH_VARIANT
 }  // namespace lulesh

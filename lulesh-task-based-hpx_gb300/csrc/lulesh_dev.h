@@ -81,9 +81,6 @@ struct Mesh {
     // scratch, double path
     double *fsx, *fsy, *fsz, *fhx, *fhy, *fhz;
     double *dvxi, *dveta, *dvzeta, *dxxi, *dxeta, *dxzeta;
-    // fast double path of a single handle: the element geometry of the
-    // current coordinates, kGeoWords arrays of numElem doubles (else null)
-    double* geo;
     // mixed path: float-pair mirrors (hi, lo) of positions and velocities
     float2 *pxp, *pyp, *pzp, *vxp, *vyp, *vzp;
     // scratch, mixed path
@@ -95,10 +92,6 @@ struct Mesh {
     DevTime* dtime;  // non-null only in the graph form: kernels take dt from here
     lulesh_params prm;
 };
-
-// Words of element geometry stored per element (Mesh::geo): direction sums
-// (9), their cofactors (9), hourglass mode sums (12), face vectors (18).
-constexpr int kGeoWords = 48;
 
 // Launch configuration shared by host and device code.
 constexpr int kForceBlock = 128;
@@ -143,26 +136,6 @@ int launch_nodes(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics(const Mesh& m, double dt, cudaStream_t s);
 int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaStream_t s);  // elements
 int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s);  // the plan's matOrder positions
-// the resident loop's form: kinematics that also stores the element geometry
-// of the updated coordinates (m.geo), forces that read it, and the pass that
-// forms it from the current coordinates when it is stale
-int launch_forces_geo(const Mesh& m, cudaStream_t s);
-int launch_kinematics_geo(const Mesh& m, double dt, cudaStream_t s);
-int launch_kinematics_geo_range(const Mesh& m, double dt, int first, int end, cudaStream_t s);
-int launch_geometry(const Mesh& m, cudaStream_t s);
-// lulesh_leapfrog's force phase, slab by slab: the check of the slab's nodes
-// [first, end) (*flag = 1 when an uploaded coordinate sx, sy, sz differs from
-// m.x, m.y, m.z), then forces of its elements [first, end) from the stored
-// geometry unless *flag, and forces with the geometry formed from the
-// uploaded coordinates when *flag (always when flag is null)
-int launch_upload_check(const Mesh& m, const double* sx, const double* sy, const double* sz, int first, int end,
-                        int32_t* flag, cudaStream_t s);
-int launch_forces_geo_unless(const Mesh& m, int first, int end, const int32_t* flag, cudaStream_t s);
-// and its node phase: positions advanced from the uploaded copies
-int launch_nodes_upload(const Mesh& m, double dt, const double* sx, const double* sy, const double* sz,
-                        cudaStream_t s);
-int launch_forces_upload(const Mesh& m, const double* sx, const double* sy, const double* sz, int first, int end,
-                         const int32_t* flag, cudaStream_t s);
 }  // namespace fp64
 namespace fp64x {
 int launch_forces(const Mesh& m, cudaStream_t s);

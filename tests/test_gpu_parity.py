@@ -224,6 +224,129 @@ def test_each_phase_after_one_cycle(lulesh, oracle_mod, precision, tol):
         assert rel_err(getattr(dom, f), o.field(f)) < tol, f
 
 
+def _distorted(s, kind, rng):
+    """Fields of a distorted mesh in motion for one phase of each kernel."""
+    n = s + 1
+    h = 1.125 / s
+    z, y, x = np.meshgrid(*(np.arange(n) * h,) * 3, indexing="ij")
+    pos = [a + 0.15 * h * rng.uniform(-1, 1, a.shape) for a in (x, y, z)]
+    vel = [rng.uniform(-100, 100, x.shape) for _ in range(3)]
+    volo, press = np.full(s ** 3, h ** 3), rng.uniform(1e3, 1e4, s ** 3)
+    scale = {"tiny": 2.0 ** -210, "huge": 2.0 ** 56}.get(kind, 1.0)
+    pos, volo = [a * scale for a in pos], volo * scale ** 3
+    if kind == "flat":  # 32 times wider than high
+        pos[2], volo = pos[2] / 32, volo / 32
+    if kind == "uniform":
+        vel = [np.full_like(a, v) for a, v in zip(vel, (3.0, -70.0, 1e-3))]
+    if kind == "rest":  # a still part of the mesh, with and without pressure
+        for a in vel:
+            a[: n // 2] = 0.0
+        press[: s ** 3 // 4] = 0.0
+    if kind == "slow":  # the z velocities 1e-9 of the others, some subnormal
+        vel[2] *= 1e-9
+        vel[2][0] = 1e-310
+    if kind == "brick":
+        pos = [x, y, z]
+    if kind == "crushed":  # a corner pushed through half of its element
+        for a in pos:
+            a[1, 1, 1] += 0.6 * h
+    return [a.ravel() for a in pos], [a.ravel() for a in vel], volo, press
+
+
+def _gradients_extended(dom):
+    """The monotonic-Q gradients of the Domain's nodes in extended precision
+    (lulesh.cc:1341-1416: direction differences of coordinates and
+    velocities, their cross products as area vectors)."""
+    nl = dom.nodelist.reshape(-1, 8)
+    plus = ([1, 2, 6, 5], [2, 3, 7, 6], [4, 5, 6, 7])
+    minus = ([0, 3, 7, 4], [0, 1, 5, 4], [0, 1, 2, 3])
+
+    def directions(f):
+        v = np.asarray(getattr(dom, f), np.longdouble)[nl]
+        return [(v[:, p].sum(axis=1) - v[:, m].sum(axis=1)) / 4 for p, m in zip(plus, minus)]
+
+    X = np.array([directions(f) for f in ("x", "y", "z")])  # [axis][direction]
+    V = np.array([directions(f) for f in ("xd", "yd", "zd")])
+    vol = np.asarray(dom.volo, np.longdouble) * np.asarray(dom.vnew, np.longdouble)
+    tiny = np.longdouble(1e-36)
+    dv, dx = [], []
+    for d in range(3):
+        u, w = X[:, (d + 1) % 3], X[:, (d + 2) % 3]
+        a = [u[(k + 1) % 3] * w[(k + 2) % 3] - u[(k + 2) % 3] * w[(k + 1) % 3] for k in range(3)]
+        dx.append(vol / np.sqrt(a[0] ** 2 + a[1] ** 2 + a[2] ** 2 + tiny))
+        dv.append(sum(a[k] * V[k, d] for k in range(3)) / (vol + tiny))
+    return [np.asarray(g, np.float64) for g in dv + dx]
+
+
+@pytest.mark.parametrize("s", [3, 6])
+@pytest.mark.parametrize("kind", ["plain", "tiny", "huge", "flat", "uniform", "rest", "slow", "brick", "crushed"])
+def test_force_and_kinematics_ranges(lulesh, oracle_mod, s, kind):
+    """The double path's force and kinematics kernels work in block fixed
+    point and hand elements that do not fit (extreme magnitudes, extreme
+    aspect) to their double form: both stay at the oracle's values on
+    distorted meshes over the range of either."""
+    pos, vel, volo, press = _distorted(s, kind, np.random.default_rng(11))
+    o = oracle_mod.Oracle(s, 11, 1, 1, threads=1)
+    dom = lulesh.HostDomain(s, 11, 1, 1)
+    dt = 1e-7 * float(np.cbrt(volo[0])) * s
+    for d in (dom, o):
+        put = (lambda f, a: getattr(dom, f).__setitem__(slice(None), a)) if d is dom else \
+              (lambda f, a: o.field(f).__setitem__(slice(None), a))
+        for f, a in zip(("x", "y", "z", "xd", "yd", "zd"), pos + vel):
+            put(f, a)
+        put("volo", volo)
+        put("elemMass", volo * 1.3)
+        put("p", press)
+        put("ss", np.sqrt(press))
+    ts = dom.time_state
+    ts.deltatime = dt
+    o.set_scalar("deltatime", dt)
+    dev = lulesh.Device(dom, "fp64")
+    assert o.leapfrog() == 0
+    dev.phase(lulesh.PHASE_FORCES, dt)
+    for got, name in zip(dev.corner_forces(), ("fx_elem", "fy_elem", "fz_elem")):
+        assert rel_err(got, o.field(name)) < 1e-12, name
+    dev.phase(lulesh.PHASE_NODES, dt)
+    dev.phase(lulesh.PHASE_KINEMATICS, dt)
+    dev.download()
+    for f in ("x", "zd", "vnew", "arealg", "vdov"):
+        assert rel_err(getattr(dom, f), o.field(f)) < 1e-12, f
+    # the gradients are differences of velocities, which in a uniform flow are
+    # all rounding in a double reference: extended precision on the same nodes
+    grads = dev.gradients()
+    for got, want, name in zip(grads, _gradients_extended(dom), ("delv_xi", "delv_eta", "delv_zeta", "delx_xi",
+                                                                 "delx_eta", "delx_zeta")):
+        assert rel_err(got, want) < 1e-12, name
+    dev.close()
+
+
+@pytest.mark.parametrize("field,value", [("x", np.nan), ("zd", np.inf), ("yd", np.nan)])
+def test_non_finite_nodes_stay_local(lulesh, field, value):
+    """A NaN coordinate or an infinite velocity of one node reaches the corner
+    forces of its 8 elements, and no other element's."""
+    s, node = 4, 2 * 25 + 2 * 5 + 2
+    a, b = lulesh.HostDomain(s), lulesh.HostDomain(s)
+    rng = np.random.default_rng(3)
+    for f in ("xd", "yd", "zd"):
+        getattr(a, f)[:] = getattr(b, f)[:] = rng.uniform(-1, 1, a.numNode)
+    for d in (a, b):
+        d.p[:] = d.ss[:] = 2.0
+    getattr(b, field)[node] = value
+    near = (b.nodelist.reshape(-1, 8) == node).any(axis=1)
+    out = []
+    for d in (a, b):
+        dev = lulesh.Device(d, "fp64")
+        dev.phase(lulesh.PHASE_FORCES, 1e-6)
+        out.append([x.reshape(-1, 8) for x in dev.corner_forces()])
+        dev.close()
+    axes = range(3) if field == "x" else ["xyz".index(field[0])]
+    for k in range(3):
+        np.testing.assert_array_equal(out[0][k][~near], out[1][k][~near])
+        assert np.isfinite(out[1][k][~near]).all()
+        if k in axes:
+            assert not np.isfinite(out[1][k][near]).any()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_graph_loop_equals_host_loop(lulesh, precision):
     a, _, na = _run_device(lulesh, 12, 11, 1, 1, precision)

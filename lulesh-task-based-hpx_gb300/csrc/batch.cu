@@ -259,7 +259,7 @@ bool rebuild_tiles(lulesh_batch* b) {
             count[sl.repValue[c]] += sl.repCount[c];
     lulesh::RepClasses classes;
     for (const auto& kv : count) classes.push_back(make_int2(kv.first, kv.second));
-    const int passes = classes.empty() ? 1 : lulesh::mat_passes_per_lane(classes, b->sms);
+    const int passes = classes.empty() ? 1 : lulesh::mat_passes_per_lane(classes, b->sms, b->precision);
     for (int s = 0; s < int(b->slots.size()); ++s) {
         const Slot& sl = b->slots[s];
         if (!sl.in_use || sl.finished) continue;

@@ -213,14 +213,14 @@ void carve_mesh(Mesh& m, Arena& a, int precision, int ne, int nn) {
 
 // Most blocks of a material launch over n elements (material_plan).
 int mat_max_grid(int n, int sms) {
-    return lulesh::blocks_for(n, lulesh::kMatBlock) + lulesh::kMaxMatClasses + 8 * sms;
+    return lulesh::blocks_for(n, lulesh::kMatBlock) + lulesh::kMaxMatClasses + 24 * sms;
 }
 
 // The material launch over the classes, whose matOrder positions begin at
 // `first`, in at most max_grid blocks.
-MatPlan material_plan(const RepClasses& classes, int first, int sms, int max_grid) {
+MatPlan material_plan(const RepClasses& classes, int first, int sms, int precision, int max_grid) {
     MatPlan p{};
-    const int passes = lulesh::mat_passes_per_lane(classes, sms);
+    const int passes = lulesh::mat_passes_per_lane(classes, sms, precision);
     for (const int2& c : classes) {
         lulesh::MatClass& k = p.cls[p.n++];
         k.first = first;
@@ -239,13 +239,13 @@ MatPlan material_plan(const RepClasses& classes, int first, int sms, int max_gri
 // The handle's material launches: over all elements at most `per_sm` blocks
 // per multiprocessor, over a slab one warp per 32 / lanes elements.
 void plan_material(lulesh_dev* d, const RepClasses& classes, const std::vector<RepClasses>& slab_classes, int per_sm) {
-    d->mat = material_plan(classes, 0, d->sms, d->sms * per_sm);
+    d->mat = material_plan(classes, 0, d->sms, d->precision, d->sms * per_sm);
     d->mat_slab.clear();
     int first = 0;
     for (const RepClasses& c : slab_classes) {
         int n = 0;
         for (const int2& k : c) n += k.y;
-        d->mat_slab.push_back(material_plan(c, first, d->sms, mat_max_grid(n, d->sms)));
+        d->mat_slab.push_back(material_plan(c, first, d->sms, d->precision, mat_max_grid(n, d->sms)));
         first += n;
     }
 }
@@ -476,10 +476,12 @@ int build_graph(lulesh_dev* d) {
 }
 
 // Material blocks per SM of the grid-stride launch (elements in repeat-count
-// order; 6 blocks of 78 registers fit per SM): a sweep of 6, 8, 12 per SM and
-// one thread per element at s=150 gave the double kernel 1.38, 1.34, 1.37,
-// 1.51 ms and the mixed kernel 0.92, 0.98, 0.95, 1.08 ms
-int mat_blocks_per_sm(int precision) { return precision == LULESH_MIXED ? 6 : 8; }
+// order, so the grid's first blocks hold the long chains). At s=150 exact: 8;
+// mixed: 6, 8, 12 per SM and one thread per element gave 0.92, 0.98, 0.95,
+// 1.08 ms; fast double (6 resident): 6 and 24 gave 0.71 and 0.66.
+int mat_blocks_per_sm(int precision) {
+    return precision == LULESH_FP64 ? 24 : precision == LULESH_MIXED ? 6 : 8;
+}
 
 // A handle for ne elements and nn nodes: the arena carved, the stream and
 // the pinned result buffers created, the device result word cleared. The
@@ -1107,29 +1109,32 @@ namespace lulesh {
 
 int validate_view(const lulesh_domain_view* v) { return check_view(v); }
 
-// The time of a material phase whose lanes run at most k passes each, in
-// units of one warp's pass on a busy SM quarter (3.2 us measured at s=150):
-// the longest lane's chain (its passes and the rest of the phase as one more,
-// 1.4 units each: a lone warp's pass takes 4.3 us) and the warps' work over
-// the 4 quarters of each SM (a warp's passes and, for the Q terms and the
-// save, three more). Few elements leave the quarters idle, so more lanes per
-// element win (s=8: 87 -> 24 us, s=30: 94 -> 48 us); many keep them busy, and
-// spreading an element then only repeats its Q terms (s=91 with 4 lanes for
-// 20 passes 0.450 -> 0.483 ms, so one lane there).
-int mat_passes_per_lane(const RepClasses& classes, int sms) {
+// The time of a material phase whose lanes run at most k passes each is the
+// longest lane's chain plus the warps' work over the 4 quarters of each SM (a
+// warp's passes and, for the Q terms and the save, `rest` more). Fitted to
+// 1..20 passes per lane at s=8..120, r=16 (mean error 5 %): a chain costs
+// 0.96 us a pass and the work 0.66 (fast double), 4.2 and 4.0 (exact), 2.7
+// and 1.2 (mixed). Few elements leave the quarters idle, so more lanes per
+// element win (20 passes in one lane against the choice: s=8 37 -> 16 us, s=30
+// 40 -> 23, exact s=45 162 -> 137, mixed s=45 86 -> 51); many keep them busy,
+// and spreading an element then only repeats its Q terms (fast double s=91:
+// 188 us with one lane, 211 with 4). A split has to save a tenth.
+int mat_passes_per_lane(const RepClasses& classes, int sms, int precision) {
+    const double chain_cost = precision == LULESH_FP64 ? 1.45 : precision == LULESH_MIXED ? 2.2 : 1.05;
+    const double rest = precision == LULESH_FP64 ? 2.5 : precision == LULESH_MIXED ? 0.5 : 1.0;
     int top = 1;
     for (const int2& c : classes) top = std::max(top, c.x);
     int best = top;
-    double best_t = 0.0;  // a split has to save a tenth of the unsplit time
+    double best_t = 0.0;
     for (int k = top; k >= 1; k = std::min(k, 64) - 1) {
         double load = 0.0;
         int chain = 0;
         for (const int2& c : classes) {
             const int lanes = lanes_for_rep(c.x, k), passes = (c.x + lanes - 1) / lanes;
             chain = std::max(chain, passes);
-            load += double(blocks_for(c.y, 32 / lanes)) * (passes + 3);
+            load += double(blocks_for(c.y, 32 / lanes)) * (passes + rest);
         }
-        const double t = 1.4 * (chain + 1) + load / (4.0 * sms);
+        const double t = chain_cost * chain + load / (4.0 * sms);
         if (k == top) best_t = 0.9 * t;
         else if (t < best_t) {
             best_t = t;

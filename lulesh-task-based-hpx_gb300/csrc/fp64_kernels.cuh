@@ -398,13 +398,15 @@ __global__ void __launch_bounds__(kKinBlock, kKinBlocks) k_kinematics(Mesh m, do
 }
 
 // Elements visited in repeat-count order so a warp's lanes run the same
-// number of EOS passes; the dt minima end in a last-block reduction.
-// 8 blocks of 128 per SM (64 registers): the EOS passes are a chain of
-// dependent integer-pipe products and FP64 operations, latency-bound at 6
-// blocks per SM (1.34 -> 1.02 ms at s=150 with 8).
+// number of EOS passes; the dt minima end in a last-block reduction. Exact
+// variant: 8 blocks of 128 per SM (64 registers), the passes being a chain of
+// dependent FP64 operations. Fast variant: 6 (80 registers): its integer
+// passes are bound by the ALU pipe, and more blocks spill (s=150: 0.69 ms
+// with 8, 0.66 with 6, 0.71 with 5).
+constexpr int kMatBlocks = LULESH_EXACT ? 8 : 6;
 // SPREAD: some class has several lanes per element (MatPlan).
 template <bool SPREAD>
-__global__ void __launch_bounds__(kMatBlock, 8) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
+__global__ void __launch_bounds__(kMatBlock, kMatBlocks) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
     if (m.dtime && !m.dtime->active) return;
     double dtc = 1.0e+20, dth = 1.0e+20;  // lulesh.cc:2214-2215
     if (SPREAD) {

@@ -119,9 +119,9 @@ struct MatPlan {
 };
 // (repeat count, elements) pairs, largest repeat count first.
 using RepClasses = std::vector<int2>;
-// EOS passes a lane should run at most, for these classes on a GPU of `sms`
-// multiprocessors (lanes_for_rep gives the lanes).
-int mat_passes_per_lane(const RepClasses& classes, int sms);
+// EOS passes a lane should run at most, for these classes in this arithmetic
+// on a GPU of `sms` multiprocessors (lanes_for_rep gives the lanes).
+int mat_passes_per_lane(const RepClasses& classes, int sms, int precision);
 inline int lanes_for_rep(int rep, int passes) {
     const int l = (rep + passes - 1) / passes;
     return l < 1 ? 1 : l > 32 ? 32 : l;

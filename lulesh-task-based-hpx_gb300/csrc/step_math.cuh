@@ -12,6 +12,14 @@
 // operation as the reference does.
 #pragma once
 
+// LULESH_FIXED_EOS: the EOS in integers (eos_fixed.cuh), for the fast double
+// variant.
+#ifndef LULESH_FIXED_EOS
+#define LULESH_FIXED_EOS 0
+#endif
+#if LULESH_FIXED_EOS
+#include "eos_fixed.cuh"
+#endif
 #include "fp64_emu.cuh"
 #include "lulesh_dev.h"
 #include "portable_cbrt.h"
@@ -1024,6 +1032,51 @@ __device__ __forceinline__ void q_terms(const Mesh& m, int i, const R* dvxi, con
     qq = double(qquad);
 }
 
+#if LULESH_FIXED_EOS
+// The double q terms: the path of what q_sums does not take (limiter
+// parameters other than the reference's, values that are infinite, NaN or of
+// extreme magnitude).
+__device__ __noinline__ double2 q_terms_double(const Mesh& m, int i, double vnew, double vdov) {
+    double ql, qq;
+    q_terms<double>(m, i, m.dvxi, m.dveta, m.dvzeta, m.dxxi, m.dxeta, m.dxzeta, vnew, vdov, ql, qq);
+    return make_double2(ql, qq);
+}
+
+// q_terms with the limiters and sums in integers (eos_fixed.cuh).
+__device__ __forceinline__ void q_terms_fixed(const Mesh& m, int i, double vnew, double vdov, double& ql, double& qq) {
+    const lulesh_params& P = m.prm;
+    const int bc = LD(m.elemBC + i);
+    double dv[3], dm[3], dp[3], dx[3];
+    auto direction = [&](int d, const double* f, const double* fx, int minus, int plus, int symm_m, int comm_m, int symm_p,
+                         int comm_p, int nm, int np) {
+        dv[d] = LD(f + i);
+        dx[d] = LD(fx + i);
+        const double m1 = LD(f + nm), p1 = LD(f + np);
+        dm[d] = minus == comm_m || minus == 0 ? m1 : minus == symm_m ? dv[d] : 0.0;
+        dp[d] = plus == comm_p || plus == 0 ? p1 : plus == symm_p ? dv[d] : 0.0;
+    };
+    direction(0, m.dvxi, m.dxxi, bc & XI_M, bc & XI_P, XI_M_SYMM, XI_M_COMM, XI_P_SYMM, XI_P_COMM, LD(m.lxim + i),
+              LD(m.lxip + i));
+    direction(1, m.dveta, m.dxeta, bc & ETA_M, bc & ETA_P, ETA_M_SYMM, ETA_M_COMM, ETA_P_SYMM, ETA_P_COMM,
+              LD(m.letam + i), LD(m.letap + i));
+    direction(2, m.dvzeta, m.dxzeta, bc & ZETA_M, bc & ZETA_P, ZETA_M_SYMM, ZETA_M_COMM, ZETA_P_SYMM, ZETA_P_COMM,
+              LD(m.lzetam + i), LD(m.lzetap + i));
+    double lin, quad;
+    bool ok = bf::q_sums(dv, dm, dp, dx, lin, quad);
+    ok &= P.monoq_limiter_mult == 2.0 && P.monoq_max_slope == 1.0;
+    if (!ok) {
+        const double2 q = q_terms_double(m, i, vnew, vdov);
+        ql = q.x;
+        qq = q.y;
+        return;
+    }
+    const double rho = LD(m.elemMass + i) * rcp(LD(m.volo + i) * vnew);
+    const bool opening = f_gt(vdov, 0.);
+    ql = opening ? 0. : P.qlc_monoq * rho * lin;
+    qq = opening ? 0. : P.qqc_monoq * rho * quad;
+}
+#endif
+
 // CalcPressureForElemsTask for one element (lulesh.cc:1671-1690).
 __device__ __forceinline__ double eos_pressure(double& bvc, double& pbvc, double e, double comp,
                                                double vnewc, const lulesh_params& P) {
@@ -1216,9 +1269,36 @@ __device__ __forceinline__ EosState eos_body(const Mesh& m, int i, double vnewc,
 }
 #endif
 
+#if LULESH_FIXED_EOS
+// The double evaluations: the path of what eos_pass does not take (parameters
+// other than the reference's kind, overridden volumes, values that are
+// infinite, NaN or of extreme magnitude).
+__device__ __noinline__ EosState eos_double(const Mesh& m, int i, double vnewc, int passes) {
+    return m.prm.refdens == 1.0 ? eos_body<true>(m, i, vnewc, passes) : eos_body<false>(m, i, vnewc, passes);
+}
+
+__device__ __forceinline__ EosState eos_element(const Mesh& m, int i, double vnewc, int passes) {
+    const lulesh_params& P = m.prm;
+    const bf::EosCuts cuts = bf::eos_cuts(P.e_cut, P.p_cut, P.q_cut, P.pmin, P.emin, P.refdens);
+    bool ok = cuts.ok && f_lt(vnewc, P.eosvmax) && (f_is_zero(P.eosvmin) || f_gt(vnewc, P.eosvmin));
+    EosState s{0., 0., 0., 0.};
+    double delvc = 0.;
+    for (int r = 0; ok && r < passes; ++r) {
+        // inputs re-read for each evaluation, as in eos_body
+        asm volatile("" ::: "memory");
+        asm volatile("" : "+d"(vnewc));
+        delvc = m.delv[i];
+        ok = bf::eos_pass(m.e[i], m.p[i], m.q[i], m.ql[i], m.qq[i], delvc, vnewc, cuts, s.e, s.p, s.q, s.ss);
+    }
+    if (!ok) return eos_double(m, i, vnewc, passes);
+    if (f_le(delvc, 0.) && f_abs_lt(s.q, P.q_cut)) s.q = 0.;
+    return s;
+}
+#else
 __device__ __forceinline__ EosState eos_element(const Mesh& m, int i, double vnewc, int passes) {
     return m.prm.refdens == 1.0 ? eos_body<true>(m, i, vnewc, passes) : eos_body<false>(m, i, vnewc, passes);
 }
+#endif
 
 // Courant and hydro candidates of one element (lulesh.cc:1938-1974); false
 // where vdov == 0 (the element does not constrain).
@@ -1263,7 +1343,11 @@ __device__ __forceinline__ void material_share(const Mesh& m, int t, int r, int 
     const int i = LD(m.matOrder + t);
     const double vnew = LD(m.vnew + i), vdov = LD(m.vdov + i);
     double ql, qq;
+#if LULESH_FIXED_EOS
+    q_terms_fixed(m, i, vnew, vdov, ql, qq);
+#else
     q_terms<R>(m, i, dvxi, dveta, dvzeta, dxxi, dxeta, dxzeta, vnew, vdov, ql, qq);
+#endif
     if (!SPREAD || r == 0) {
         m.qq[i] = qq;
         m.ql[i] = ql;

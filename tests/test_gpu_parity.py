@@ -320,6 +320,65 @@ def test_force_and_kinematics_ranges(lulesh, oracle_mod, s, kind):
     dev.close()
 
 
+MATERIAL_KINDS = ["plain", "cold", "opening", "closing", "still", "huge", "faint", "negative", "half_cold", "folded"]
+
+
+@pytest.mark.parametrize("params", [{}, {"pmin": 5.0}, {"eosvmax": 0.95}, {"eosvmin": 0.97}, {"refdens": 2.0},
+                                    {"monoq_limiter_mult": 1.5}, {"q_cut": 0.0}],
+                         ids=lambda p: next(iter(p), "default"))
+@pytest.mark.parametrize("kind", MATERIAL_KINDS)
+def test_material_ranges(lulesh, kind, params):
+    """The double path's material kernel evaluates the Q terms and the EOS in
+    integers and hands what does not fit (parameters of another kind,
+    extreme magnitudes) to its double form: both stay within rounding of the
+    exact variant's double arithmetic on the same gradients and state."""
+    s = 6
+    rng = np.random.default_rng(5)
+    pos, vel, volo, press = _distorted(s, "plain", rng)
+    ne = s ** 3
+    e = press * 1.5
+    vnew = rng.uniform(0.9, 1.1, ne)
+    delv = rng.uniform(-0.05, 0.05, ne)
+    q = rng.uniform(0, 0.2, ne) * press
+    if kind == "cold":
+        e, press, q = np.zeros(ne), np.zeros(ne), np.zeros(ne)
+    if kind == "half_cold":
+        for a in (e, press, q):
+            a[::2] = 0.0
+    if kind in ("opening", "closing"):
+        delv = np.abs(delv) * (1 if kind == "opening" else -1)
+    if kind == "still":
+        delv[:] = 0.0
+    if kind == "huge":
+        e, press, q = e * 1e270, press * 1e270, q * 1e270
+    if kind == "faint":  # around the cutoffs of 1e-7
+        e, press, q = e * 1e-11, press * 1e-11, q * 1e-11
+    if kind == "negative":
+        e[::3] *= -1
+    if kind == "folded":  # steps longer than the relative volume
+        delv[::4] = -1.5
+    out = {}
+    for precision in ("fp64_exact", "fp64"):
+        dom = lulesh.HostDomain(s, 11)
+        for f, a in zip(("x", "y", "z", "xd", "yd", "zd"), pos + vel):
+            getattr(dom, f)[:] = a
+        dom.volo[:], dom.elemMass[:] = volo, volo * 1.3
+        for k, v in params.items():
+            setattr(dom.view.params, k, v)
+        dev = lulesh.Device(dom, precision)
+        dev.phase(lulesh.PHASE_KINEMATICS, 1e-7)
+        dev.download()
+        dom.vnew[:], dom.delv[:], dom.e[:], dom.p[:], dom.q[:] = vnew, delv, e, press, q
+        dev.upload(lulesh.F_KIN | lulesh.F_EPQ)
+        dev.phase(lulesh.PHASE_MATERIAL)
+        dev.download()
+        out[precision] = {f: getattr(dom, f).copy() for f in ("e", "p", "q", "ql", "qq", "ss")}
+        dev.close()
+        dom.close()
+    for f, want in out["fp64_exact"].items():
+        assert rel_err(out["fp64"][f], want) < 1e-12, f
+
+
 @pytest.mark.parametrize("field,value", [("x", np.nan), ("zd", np.inf), ("yd", np.nan)])
 def test_non_finite_nodes_stay_local(lulesh, field, value):
     """A NaN coordinate or an infinite velocity of one node reaches the corner

@@ -72,8 +72,9 @@ struct lulesh_dev {
     StepResult* h_result = nullptr;  // pinned: [0] the step's, [1 + k] material slab k's (lulesh_leapfrog)
     DevTime* d_time = nullptr;
     DevTime* h_time = nullptr;       // pinned
-    cudaGraphExec_t graph = nullptr;
-    int graph_kernels = 0;
+    // the graph form's cycle, once and kGraphCycles times
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    int graph_kernels = 0;  // of one cycle
     int64_t launches = 0;
     int32_t err_elem = -1;
     int32_t nx = 0;                  // edge of the cube (Domain::sizeX)
@@ -398,18 +399,22 @@ int upload_mesh(const Mesh& m, const lulesh_domain_view* v, int precision, cudaS
 // current cycle's dt minima (lulesh_dev_run). `set` picks the profiling
 // events of the cycle (two sets: a cycle's and the next one's forces).
 //
-// The force phase: the error word cleared, forces.
+// The error word cleared, before the first cycle of a call (a cycle that
+// raises an error ends the call).
+int clear_error(lulesh_dev* d) {
+    CK(cudaMemsetAsync(&d->m.result->err, 0, 3 * sizeof(int32_t), d->stream));
+    return LULESH_OK;
+}
+// The force phase.
 int queue_forces(lulesh_dev* d, int set) {
-    const Mesh& m = d->m;
     const bool prof = d->profiling;
-    CK(cudaMemsetAsync(&m.result->err, 0, 3 * sizeof(int32_t), d->stream));
     if (prof) CK(cudaEventRecord(d->ev[set][0], d->stream));
-    d->launches += d->L.forces(m, d->stream);
+    d->launches += d->L.forces(d->m, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][1], d->stream));
     return LULESH_OK;
 }
-// The rest of the cycle with time step dt, then the readback of its dt
-// minima and error word (event ev_done).
+// The rest of the cycle with time step dt. Its last block writes the dt minima
+// and the error word to the host's h_result (event ev_done).
 int queue_rest(lulesh_dev* d, double dt, int set) {
     const Mesh& m = d->m;
     const bool prof = d->profiling;
@@ -421,12 +426,10 @@ int queue_rest(lulesh_dev* d, double dt, int set) {
     d->launches += d->L.material(m, d->mat, d->stream);
     if (prof) CK(cudaEventRecord(d->ev[set][4], d->stream));
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(d->h_result, m.result, sizeof(StepResult), cudaMemcpyDeviceToHost, d->stream));
     CK(cudaEventRecord(d->ev_done, d->stream));
     return LULESH_OK;
 }
-// Waits for the cycle's readback (not for work queued after it) and returns
-// its status.
+// Waits for the cycle (not for work queued after it) and returns its status.
 int finish_cycle(lulesh_dev* d, int set) {
     CK(cudaEventSynchronize(d->ev_done));
     if (d->profiling) {
@@ -445,30 +448,36 @@ int finish_cycle(lulesh_dev* d, int set) {
 }
 
 int run_cycle(lulesh_dev* d, double dt) {
-    int st = queue_forces(d, 0);
+    int st = clear_error(d);
+    if (st == LULESH_OK) st = queue_forces(d, 0);
     if (st == LULESH_OK) st = queue_rest(d, dt, 0);
     return st == LULESH_OK ? finish_cycle(d, 0) : st;
 }
 
-int build_graph(lulesh_dev* d) {
-    if (d->graph) return LULESH_OK;
+// Cycles of the longer graph: 8 to one host launch (cycles after the loop's
+// end return at once, as in the one-cycle graph).
+constexpr int kGraphCycles = 8;
+
+int build_graph(lulesh_dev* d, int which) {
+    if (d->graph[which]) return LULESH_OK;
     Mesh gm = d->m;
     gm.dtime = d->d_time;
+    gm.report = nullptr;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
     int k = 0;
-    k += lulesh::launch_time_increment(d->d_time, gm.result, d->stream);
-    k += d->L.forces(gm, d->stream);
-    k += d->L.nodes(gm, 0.0, d->stream);
-    k += d->L.kinematics(gm, 0.0, d->stream);
-    k += d->L.material(gm, d->mat, d->stream);
-    k += lulesh::launch_time_finish(d->d_time, gm.result, d->stream);
+    for (int c = 0; c < (which ? kGraphCycles : 1); ++c) {
+        k = d->L.forces(gm, d->stream);
+        k += d->L.nodes(gm, 0.0, d->stream);
+        k += d->L.kinematics(gm, 0.0, d->stream);
+        k += d->L.material(gm, d->mat, d->stream);
+    }
     cudaError_t ce = cudaStreamEndCapture(d->stream, &g);
     if (ce != cudaSuccess) return LULESH_ECUDA;
-    ce = cudaGraphInstantiate(&d->graph, g, 0);
+    ce = cudaGraphInstantiate(&d->graph[which], g, 0);
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) {
-        d->graph = nullptr;
+        d->graph[which] = nullptr;
         return LULESH_ECUDA;
     }
     d->graph_kernels = k;
@@ -518,6 +527,7 @@ int new_handle(int32_t precision, int ne, int nn, lulesh_dev** out) {
         return fail(LULESH_ECUDA);
     if (cudaMallocHost(&d->h_result, sizeof(StepResult) * (1 + kLeapfrogSlabs)) != cudaSuccess)
         return fail(LULESH_ENOMEM);
+    m.report = d->h_result;
     if (cudaMallocHost(&d->h_time, sizeof(DevTime)) != cudaSuccess) return fail(LULESH_ENOMEM);
     if (cudaMallocHost(&d->h_verify, 4 * sizeof(double)) != cudaSuccess) return fail(LULESH_ENOMEM);
     if (cudaMemsetAsync(m.result, 0, sizeof(StepResult), d->stream) != cudaSuccess)
@@ -591,7 +601,8 @@ void lulesh_dev_destroy(lulesh_dev* d) {
         if (e) cudaEventDestroy(e);
     if (d->ev_begin) cudaEventDestroy(d->ev_begin);
     if (d->ev_end) cudaEventDestroy(d->ev_end);
-    if (d->graph) cudaGraphExecDestroy(d->graph);
+    for (cudaGraphExec_t g : d->graph)
+        if (g) cudaGraphExecDestroy(g);
     if (d->arena) cudaFree(d->arena);
     if (d->h_result) cudaFreeHost(d->h_result);
     if (d->h_time) cudaFreeHost(d->h_time);
@@ -862,6 +873,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     CK(cudaStreamWaitEvent(d->stream, d->ev_e, 0));
     CK(cudaStreamWaitEvent(d->stream2, d->ev_e, 0));
     Mesh ms = m;  // the slab-major material order: positions [e_lo, e_hi) are the slab's elements
+    ms.report = nullptr;  // the slabs' results come back together below
     if (slabs > 1) ms.matOrder = d->matOrderSlab;
     int part = 0;  // first block partial of the slab
     for (int sl = 0; sl < slabs; ++sl) {
@@ -932,7 +944,10 @@ int lulesh_dev_run(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycles, int
     int set = 0;
     while (ts->time < ts->stoptime && ts->cycle < max_cycles) {
         lulesh_time_increment(ts);
-        if (!forces_queued) st = queue_forces(d, set);
+        if (!forces_queued) {
+            st = clear_error(d);
+            if (st == LULESH_OK) st = queue_forces(d, set);
+        }
         if (st == LULESH_OK) st = queue_rest(d, ts->deltatime, set);
         if (st != LULESH_OK) break;
         forces_queued = ts->time < ts->stoptime && ts->cycle < max_cycles;
@@ -951,8 +966,6 @@ int lulesh_dev_run(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycles, int
 int lulesh_dev_run_graph(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycles,
                          int32_t sync_every, int32_t* cycles_run) {
     if (!d || !ts || sync_every < 1) return LULESH_EINVAL;
-    int st = build_graph(d);
-    if (st != LULESH_OK) return st;
     DevTime& h = *d->h_time;
     h = DevTime{};
     h.time = ts->time;
@@ -970,10 +983,16 @@ int lulesh_dev_run_graph(lulesh_dev* d, lulesh_time_state* ts, int32_t max_cycle
     const int32_t start = ts->cycle;
     CK(cudaMemsetAsync(d->m.result, 0, sizeof(StepResult), d->stream));
     CK(cudaMemcpyAsync(d->d_time, d->h_time, sizeof(DevTime), cudaMemcpyHostToDevice, d->stream));
+    d->launches += lulesh::launch_time_increment(d->d_time, d->m.result, d->stream);
+    CK(cudaGetLastError());
     for (;;) {
-        for (int k = 0; k < sync_every; ++k) {
-            CK(cudaGraphLaunch(d->graph, d->stream));
-            d->launches += d->graph_kernels;
+        for (int k = 0; k < sync_every;) {
+            const int which = sync_every - k >= kGraphCycles, cycles = which ? kGraphCycles : 1;
+            const int st = build_graph(d, which);
+            if (st != LULESH_OK) return st;
+            CK(cudaGraphLaunch(d->graph[which], d->stream));
+            d->launches += int64_t(d->graph_kernels) * cycles;
+            k += cycles;
         }
         CK(cudaMemcpyAsync(d->h_time, d->d_time, sizeof(DevTime), cudaMemcpyDeviceToHost, d->stream));
         CK(cudaMemcpyAsync(d->h_result, d->m.result, sizeof(StepResult), cudaMemcpyDeviceToHost, d->stream));

@@ -90,6 +90,7 @@ struct Mesh {
     DtPartial* partials;  // one per block of a material launch
     StepResult* result;
     DevTime* dtime;  // non-null only in the graph form: kernels take dt from here
+    StepResult* report;  // pinned host memory that the cycle's result goes to as well, or null
     lulesh_params prm;
 };
 
@@ -158,7 +159,6 @@ int launch_mirror_range(const Mesh& m, int first, int end, cudaStream_t s);  // 
 
 // Device-side TimeIncrement for the graph form (time_increment.cu).
 int launch_time_increment(DevTime* t, StepResult* r, cudaStream_t s);
-int launch_time_finish(DevTime* t, StepResult* r, cudaStream_t s);
 
 // --- batched form -------------------------------------------------------------
 // Many independent problems ("instances"), each with its own Mesh in a slot

@@ -23,6 +23,7 @@
 #include "fp64_emu.cuh"
 #include "lulesh_dev.h"
 #include "portable_cbrt.h"
+#include "time_advance.cuh"
 
 #ifndef LULESH_VARIANT
 #error "define LULESH_VARIANT"
@@ -1416,7 +1417,8 @@ __device__ __forceinline__ void block_min2(double& a, double& b) {
 }
 
 // Publishes this block's (dtc, dth) minima; the last block to arrive reduces
-// all partials into m.result and re-arms the counter. One pass, no second
+// all partials into m.result, re-arms the counter and ends the cycle (the
+// graph form's time, the host's report). One pass, no second
 // launch. Every thread of the block must call it.
 __device__ __forceinline__ void finish_dt_reduction(const Mesh& m, double dtc, double dth) {
     block_min2(dtc, dth);
@@ -1439,9 +1441,15 @@ __device__ __forceinline__ void finish_dt_reduction(const Mesh& m, double dtc, d
     __syncthreads();  // block_min2's shared scratch is reused
     block_min2(a, b);
     if (threadIdx.x == 0) {
-        m.result->dtcourant = a;
-        m.result->dthydro = b;
-        m.result->blocks_done = 0u;
+        StepResult* r = m.result;
+        r->dtcourant = a;
+        r->dthydro = b;
+        r->blocks_done = 0u;
+        if (m.dtime) {  // the graph form: hand the minima over, take the next cycle's step
+            finish_time(m.dtime, r);
+            advance_time(m.dtime, r);
+        }
+        if (m.report) *m.report = *r;
     }
 }
 

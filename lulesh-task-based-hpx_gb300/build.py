@@ -44,6 +44,7 @@ UNITS = [
     ("device_init.cu", ["--fmad=false"]),
     ("capi.cu", []),
     ("noalloc.cu", []),
+    ("host_copy.cu", []),
     ("batch.cu", []),
     ("serve.cu", []),
     ("domain.cpp", ["-x", "cu", "--fmad=false"]),

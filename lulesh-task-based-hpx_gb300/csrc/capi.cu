@@ -273,6 +273,23 @@ struct Copy {
     size_t bytes;
 };
 
+// Elements [a, b) of each array as a list for copy_segments.
+std::vector<lulesh::HostCopy> segments(const std::vector<Copy>& c, int64_t a, int64_t b) {
+    std::vector<lulesh::HostCopy> out;
+    for (const Copy& k : c)
+        out.push_back({static_cast<double*>(k.dev) + a, const_cast<double*>(static_cast<const double*>(k.host)) + a,
+                       sizeof(double) * size_t(b - a)});
+    return out;
+}
+// Queues whole-array copies on s.
+int copy_whole(const std::vector<Copy>& c, bool to_device, cudaStream_t s, int64_t* launches) {
+    std::vector<lulesh::HostCopy> list;
+    for (const Copy& k : c) list.push_back({k.dev, const_cast<void*>(k.host), k.bytes});
+    const int n = int(list.size());
+    return lulesh::copy_segments(list.data(), n, to_device, lulesh::host_mapped(list.data(), n), lulesh::kKernelCopyBytes,
+                                 s, launches);
+}
+
 // The (device, host) pairs of the field groups in `mask`.
 std::vector<Copy> groups(const Mesh& m, const lulesh_domain_view* v, uint32_t mask) {
     const size_t nb = sizeof(double) * size_t(m.numNode), eb = sizeof(double) * size_t(m.numElem);
@@ -646,10 +663,10 @@ int lulesh_dev_verify(lulesh_dev* d, int32_t cycle, lulesh_verify_result* out) {
 int lulesh_dev_upload(lulesh_dev* d, const lulesh_domain_view* v, uint32_t mask) {
     if (!d || !v || v->numElem != d->m.numElem || v->numNode != d->m.numNode) return LULESH_EINVAL;
     if (mask & LULESH_F_MESH) return LULESH_EINVAL;  // the mesh is fixed at creation
-    for (const Copy& c : groups(d->m, v, mask)) {
+    const auto list = groups(d->m, v, mask);
+    for (const Copy& c : list)
         if (!c.host) return LULESH_EINVAL;
-        CK(cudaMemcpyAsync(c.dev, c.host, c.bytes, cudaMemcpyHostToDevice, d->stream));
-    }
+    if (int st = copy_whole(list, true, d->stream, &d->launches)) return st;
     if (d->precision == LULESH_MIXED && (mask & (LULESH_F_POS | LULESH_F_VEL))) {
         d->launches += lulesh::mixed::launch_mirror(d->m, d->stream);
         CK(cudaGetLastError());
@@ -660,10 +677,10 @@ int lulesh_dev_upload(lulesh_dev* d, const lulesh_domain_view* v, uint32_t mask)
 
 int lulesh_dev_download(lulesh_dev* d, lulesh_domain_view* v, uint32_t mask) {
     if (!d || !v || v->numElem != d->m.numElem || v->numNode != d->m.numNode) return LULESH_EINVAL;
-    for (const Copy& c : groups(d->m, v, mask)) {
+    const auto list = groups(d->m, v, mask);
+    for (const Copy& c : list)
         if (!c.host) return LULESH_EINVAL;
-        CK(cudaMemcpyAsync(const_cast<void*>(c.host), c.dev, c.bytes, cudaMemcpyDeviceToHost, d->stream));
-    }
+    if (int st = copy_whole(list, false, d->stream, &d->launches)) return st;
     CK(cudaStreamSynchronize(d->stream));
     return LULESH_OK;
 }
@@ -681,13 +698,21 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     if (!d || !v || !v->time || v->numElem != d->m.numElem || v->numNode != d->m.numNode)
         return LULESH_EINVAL;
     if (!(v->time->deltatime > 0.0)) return LULESH_EINVAL;
-    const auto in = groups(d->m, v, LULESH_F_STEP_IN);
+    const auto in_nodes = groups(d->m, v, LULESH_F_POS | LULESH_F_VEL);
+    auto in_elems = groups(d->m, v, LULESH_F_EPQ | LULESH_F_V | LULESH_F_SS);
     const auto out_nodes = groups(d->m, v, LULESH_F_POS | LULESH_F_VEL | LULESH_F_ACC | LULESH_F_FORCE);
     const auto out_kin = groups(d->m, v, LULESH_F_V | LULESH_F_KIN);
     const auto out_mat = groups(d->m, v, LULESH_F_EPQ | LULESH_F_QLQQ | LULESH_F_SS);
-    for (const auto* g : {&in, &out_nodes, &out_kin, &out_mat})
+    using List = const std::vector<Copy>*;
+    for (List g : {List(&in_nodes), List(&in_elems), List(&out_nodes), List(&out_kin), List(&out_mat)})
         for (const Copy& c : *g)
             if (!c.host) return LULESH_EINVAL;
+    // the energy, read only by the material phase, goes up last
+    in_elems.erase(std::find_if(in_elems.begin(), in_elems.end(), [&](const Copy& c) { return c.dev == d->m.e; }));
+    std::vector<lulesh::HostCopy> all;  // every array of the call, once
+    for (const auto* g : {&out_nodes, &out_kin, &out_mat})
+        for (const Copy& c : *g) all.push_back({c.dev, const_cast<void*>(c.host), c.bytes});
+    const bool mapped = lulesh::host_mapped(all.data(), int(all.size()));
     if (!d->cstream) {
         CK(cudaStreamCreateWithFlags(&d->cstream, cudaStreamNonBlocking));
         CK(cudaStreamCreateWithFlags(&d->mstream, cudaStreamNonBlocking));
@@ -770,16 +795,13 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     // compute stream st is done (event ev), on st's download stream.
     // (stage and index: the timeline's marks of the work and of its download)
     auto elem_down = [&](const std::vector<Copy>& out, int64_t e0, int64_t e1, cudaEvent_t ev,
-                         cudaStream_t st, int stage, int index) -> int {
+                         cudaStream_t st, size_t limit, int stage, int index) -> int {
         cudaStream_t down = st == d->stream2 ? d->mstream2 : d->mstream;
         CK(cudaEventRecord(ev, st));
         if (int r = mark(stage, index, st)) return r;
         CK(cudaStreamWaitEvent(down, ev, 0));
-        const size_t off = size_t(e0), cnt = size_t(e1 - e0);
-        for (const Copy& c : out)
-            CK(cudaMemcpyAsync(static_cast<double*>(const_cast<void*>(c.host)) + off,
-                               static_cast<const double*>(c.dev) + off, sizeof(double) * cnt,
-                               cudaMemcpyDeviceToHost, down));
+        const auto list = segments(out, e0, e1);
+        if (int r = lulesh::copy_segments(list.data(), int(list.size()), false, mapped, limit, down, &d->launches)) return r;
         return mark(stage + 1, index, down);
     };
 
@@ -805,16 +827,15 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         CK(cudaEventRecord(ev, d->nstream));
         if (int st = mark(LULESH_TL_NODES, r, d->nstream)) return st;
         CK(cudaStreamWaitEvent(d->mstream, ev, 0));
-        for (const Copy& c : out_nodes)
-            CK(cudaMemcpyAsync(static_cast<double*>(const_cast<void*>(c.host)) + a,
-                               static_cast<const double*>(c.dev) + a, sizeof(double) * size_t(b - a),
-                               cudaMemcpyDeviceToHost, d->mstream));
+        const auto list = segments(out_nodes, a, b);
+        if (int st = lulesh::copy_segments(list.data(), int(list.size()), false, mapped, lulesh::kKernelGroupBytes,
+                                           d->mstream, &d->launches))
+            return st;
         return mark(LULESH_TL_NODES_DOWN, r, d->mstream);
     };
     int64_t node_next = 0;  // first node not yet updated
     int nranges = 0;
 
-    const Copy* e_in = nullptr;
     int64_t node_done = 0;
     for (int sl = 0; sl < slabs; ++sl) {
         if (cube && sl > 0 && (sl & 1) == 0) {  // the node planes below slab sl's
@@ -823,18 +844,13 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
             node_next = n_lo[sl];
         }
         const int64_t e0 = e_lo[sl], e1 = e_hi[sl], n1 = n_hi[sl];
-        for (const Copy& c : in) {
-            if (c.dev == m.e) {
-                e_in = &c;
-                continue;
-            }
-            const bool node = c.bytes == sizeof(double) * size_t(m.numNode);
-            const int64_t a = node ? node_done : e0, b = node ? n1 : e1;
-            double* dst = static_cast<double*>(c.dev);
-            if (b > a)
-                CK(cudaMemcpyAsync(dst + a, static_cast<const double*>(c.host) + a, sizeof(double) * size_t(b - a),
-                                   cudaMemcpyHostToDevice, d->cstream));
+        auto up = segments(in_elems, e0, e1);
+        if (n1 > node_done) {
+            const auto nodes = segments(in_nodes, node_done, n1);
+            up.insert(up.end(), nodes.begin(), nodes.end());
         }
+        if (int st = lulesh::copy_segments(up.data(), int(up.size()), true, mapped, lulesh::kKernelCopyBytes, d->cstream,
+                                           &d->launches)) return st;
         CK(cudaEventRecord(d->ev_slab[sl], d->cstream));
         if (int st = mark(LULESH_TL_UPLOAD, sl, d->cstream)) return st;
         cudaStream_t cs = (sl & 1) ? d->stream2 : d->stream;
@@ -851,7 +867,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         node_done = n1;
     }
 
-    if (e_in) CK(cudaMemcpyAsync(e_in->dev, e_in->host, e_in->bytes, cudaMemcpyHostToDevice, d->cstream));
+    CK(cudaMemcpyAsync(m.e, v->e, sizeof(double) * size_t(m.numElem), cudaMemcpyHostToDevice, d->cstream));
     CK(cudaEventRecord(d->ev_e, d->cstream));
     if (int st = mark(LULESH_TL_ENERGY_UP, 0, d->cstream)) return st;
     if (int st = node_range(node_next, m.numNode, d->ev_node[nranges], nranges)) return st;
@@ -862,7 +878,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         const int64_t e0 = e_lo[k], e1 = e_hi[std::min(k + 1, slabs - 1)];
         cudaStream_t cs = (k & 2) ? d->stream2 : d->stream;
         d->launches += d->L.kinematics_range(m, dt, int(e0), int(e1), cs);
-        if (int st = elem_down(out_kin, e0, e1, d->ev_kin[k], cs, LULESH_TL_KIN, k / 2)) return st;
+        if (int st = elem_down(out_kin, e0, e1, d->ev_kin[k], cs, lulesh::kKernelGroupBytes, LULESH_TL_KIN, k / 2)) return st;
     }
     // the material phase reads the kinematics of both compute streams (the
     // Q limiter reads neighbouring elements' gradients) and the energy
@@ -884,7 +900,7 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
         ms.result = d->slab_result + sl;
         part += d->mat_slab[sl].grid;
         d->launches += d->L.material(ms, d->mat_slab[sl], cs);
-        if (int st = elem_down(out_mat, e_lo[sl], e_hi[sl], d->ev_mat[sl], cs, LULESH_TL_MAT, sl)) return st;
+        if (int st = elem_down(out_mat, e_lo[sl], e_hi[sl], d->ev_mat[sl], cs, lulesh::kKernelCopyBytes, LULESH_TL_MAT, sl)) return st;
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(d->ev_s2, d->stream2));
@@ -1326,11 +1342,10 @@ int mesh_init_problem(Mesh& m, char* base, const lulesh_problem* p, int precisio
 
 int copy_fields(const Mesh& m, const lulesh_domain_view* v, uint32_t mask, bool to_device, cudaStream_t s) {
     if (to_device && (mask & LULESH_F_MESH)) return LULESH_EINVAL;  // the mesh is fixed at admission
-    for (const Copy& c : groups(m, v, mask)) {
+    const auto list = groups(m, v, mask);
+    for (const Copy& c : list)
         if (!c.host) return LULESH_EINVAL;
-        if (to_device) CK(cudaMemcpyAsync(c.dev, c.host, c.bytes, cudaMemcpyHostToDevice, s));
-        else CK(cudaMemcpyAsync(const_cast<void*>(c.host), c.dev, c.bytes, cudaMemcpyDeviceToHost, s));
-    }
+    if (int st = copy_whole(list, to_device, s, nullptr)) return st;
     CK(cudaStreamSynchronize(s));
     return LULESH_OK;
 }

@@ -249,6 +249,31 @@ int launch_build(const Mesh& m, int s, double einit, const RegionRun* runs, int 
 // entries, device memory) into an element order out[numElem].
 int launch_build_order(int32_t* out, int numElem, const int2* ranges, const int32_t* off, int n, cudaStream_t st);
 
+// --- copies to and from the caller's host arrays (host_copy.cu) --------------------
+
+struct HostCopy {
+    void* dev;
+    void* host;
+    size_t bytes;
+};
+// Lists of up to this many bytes per copy go through one kernel when the host
+// arrays are page-locked; larger ones through the copy engines, which leave
+// the multiprocessors to the step. Download of all 23 arrays: s=8 48 -> 13 us,
+// s=30 76 -> 44, s=45 (712 KB each) 139 -> 117, s=60 (1.7 MB) 271 -> 259. Drop-in
+// call: s=8 341 -> 206 us, s=45 473 -> 318; s=90 1.42 -> 1.18 ms with the slabs'
+// uploads and material results (729 KB) in kernels and the node ranges and
+// kinematics groups (twice that) left to the engines, 1.40 with all of them
+// in kernels; likewise s=60 671 -> 478 us so divided, 532 undivided. So the
+// groups of two slabs keep to the engines from a quarter of the size on.
+constexpr size_t kKernelCopyBytes = 1 << 20;
+constexpr size_t kKernelGroupBytes = kKernelCopyBytes / 4;
+// Are all host arrays of the list page-locked and mapped for kernels?
+bool host_mapped(const HostCopy* c, int n);
+// Queues the copies on s, in a kernel if `mapped` (as host_mapped says) and of
+// at most `limit` bytes per copy, and counts the launches it made.
+int copy_segments(const HostCopy* c, int n, bool to_device, bool mapped, size_t limit, cudaStream_t s,
+                  int64_t* launches);
+
 // Handle-independent instance set-up shared by the single-problem handle and
 // the batch pool (capi.cu).
 size_t mesh_bytes(int precision, int numElem, int numNode);

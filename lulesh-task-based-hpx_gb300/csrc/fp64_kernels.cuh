@@ -98,8 +98,9 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
 // (192 x dV/dx_k) and the mode sums scaled by volinv / 192. The stress force
 // (p + q) n enters through the face vectors scaled by (p + q) / 8 and starts
 // each corner's hourglass multiply-add chain. Elements that fail a test store
-// nothing: the step reports the error and its state is not used.
-__device__ __noinline__ void forces_double(const Mesh& m, int i) {
+// nothing: the step reports the error and its state is not used. Bit a of
+// `axes`: form and store the forces along axis a.
+__device__ __noinline__ void forces_double(const Mesh& m, int i, int axes) {
     const size_t N = (size_t)m.numElem;
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
@@ -150,6 +151,7 @@ __device__ __noinline__ void forces_double(const Mesh& m, int i) {
     const double* vels[3] = {m.xd, m.yd, m.zd};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        if (!(axes >> a & 1)) continue;
         double st[8], vel[8], f[8];
         corner_sums(fa, a, st);
         gather8(vels[a], nl, vel);
@@ -159,9 +161,12 @@ __device__ __noinline__ void forces_double(const Mesh& m, int i) {
     }
 }
 
-// Corner forces of element i, stress plus hourglass, in block fixed point
-// (block_fixed.cuh) and stored as forces_double stores them.
-__device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
+// Corner forces of element i, stress plus hourglass, along axes [first, end),
+// in block fixed point (block_fixed.cuh) and stored as forces_double stores
+// them. Which form an axis takes depends on the geometry and on that axis'
+// velocities alone, so an element's forces are the same bits however its
+// axes are divided.
+__device__ __forceinline__ void forces_axes(const Mesh& m, int i, int first, int end) {
     const size_t N = (size_t)m.numElem;
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
@@ -183,9 +188,10 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
     bf::ForceScale sc;
     const double coefficient = -m.prm.hgcoef * 0.01 * LD(m.ss + i) * LD(m.elemMass + i) * rcbrt_pos(determ);
     ok &= bf::force_scale(g, rcp(determ) * (1.0 / 192.0), coefficient, LD(m.p + i) + LD(m.q + i), sc);
+    int again = ok ? 0 : 7;
     // one copy of the axis' code: three would not fit the instruction cache
 #pragma unroll 1
-    for (int a = 0; a < 3; ++a) {
+    for (int a = first; a < end; ++a) {
         int64_t n[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) n[d] = a == 0 ? g.n[d][0] : a == 1 ? g.n[d][1] : g.n[d][2];
@@ -193,12 +199,15 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
         double* out = a == 0 ? m.fsx : a == 1 ? m.fsy : m.fsz;
         double vel[8], f[8];
         gather8(v, nl, vel);
-        ok &= bf::force_axis(g, sc, n, a == 0 ? g.unit[0] : a == 1 ? g.unit[1] : g.unit[2], vel, f);
+        const bool fits = bf::force_axis(g, sc, n, a == 0 ? g.unit[0] : a == 1 ? g.unit[1] : g.unit[2], vel, f);
+        again |= fits ? 0 : 1 << a;
 #pragma unroll
         for (int k = 0; k < 8; ++k) out[k * N + i] = f[k];
     }
-    if (!ok) forces_double(m, i);
+    again &= (1 << end) - (1 << first);
+    if (again) forces_double(m, i, again);
 }
+__device__ __forceinline__ void forces_elem(const Mesh& m, int i) { forces_axes(m, i, 0, 3); }
 #endif
 
 // Node n: gather in CSR order, stress then hourglass per corner
@@ -262,31 +271,39 @@ __device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt)
 // the block fixed point of kinematics_elem. The characteristic length
 // 4 V / sqrt(largest face measure) comes from the faces' t x s: the
 // reference's face measure is 4 |t x s|^2 (Lagrange's identity).
-__device__ __noinline__ void kinematics_double(const Mesh& m, int i, double dt) {
+// Parts: kKinGeometry stores what follows from the coordinates (and v),
+// kKinVelocity what needs the velocities too.
+constexpr int kKinGeometry = 1, kKinVelocity = 2;
+__device__ __noinline__ void kinematics_double(const Mesh& m, int i, double dt, int parts) {
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
     double x[8], y[8], z[8], xv[8], yv[8], zv[8];
     gather8(m.x, nl, x);
     gather8(m.y, nl, y);
     gather8(m.z, nl, z);
-    const double volume = hex_volume(x, y, z);
-    const double relv = quot_refined(volume, LD(m.volo + i));
-    const double vold = m.v[i];
-    m.vnew[i] = relv;
-    m.delv[i] = relv - vold;
-    m.arealg[i] = char_length(x, y, z, volume);
     gather8(m.xd, nl, xv);
     gather8(m.yd, nl, yv);
     gather8(m.zd, nl, zv);
+    const double volume = hex_volume(x, y, z);
+    const double relv = quot_refined(volume, LD(m.volo + i));
     double gr[6];
-    m.vdov[i] = gradients_vdov(x, y, z, xv, yv, zv, pmul(LD(m.volo + i), relv), 0.5 * dt, gr);
-    m.dvxi[i] = gr[0];
-    m.dveta[i] = gr[1];
-    m.dvzeta[i] = gr[2];
-    m.dxxi[i] = gr[3];
-    m.dxeta[i] = gr[4];
-    m.dxzeta[i] = gr[5];
-    update_volume(m, i, vold, relv);
+    const double vdov = gradients_vdov(x, y, z, xv, yv, zv, pmul(LD(m.volo + i), relv), 0.5 * dt, gr);
+    if (parts & kKinGeometry) {
+        const double vold = m.v[i];
+        m.vnew[i] = relv;
+        m.delv[i] = relv - vold;
+        m.arealg[i] = char_length(x, y, z, volume);
+        m.dxxi[i] = gr[3];
+        m.dxeta[i] = gr[4];
+        m.dxzeta[i] = gr[5];
+        update_volume(m, i, vold, relv);
+    }
+    if (parts & kKinVelocity) {
+        m.vdov[i] = vdov;
+        m.dvxi[i] = gr[0];
+        m.dveta[i] = gr[1];
+        m.dvzeta[i] = gr[2];
+    }
 }
 
 // Ulps (halved below 1) that the relative volume of an element at rest may
@@ -299,58 +316,69 @@ constexpr unsigned long long kUlpsBelow = 8, kUlpsAbove = 4;
 // relative volume within the rounding of that formula of 1 is 1, as in the
 // reference (a delv of an ulp would send its EOS passes down the compressing
 // branch).
-__device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt) {
+// PARTS: the parts to form and store (kinematics_double). Which form a part
+// takes depends on its own inputs alone, so an element's values are the same
+// bits however its parts are divided.
+template <int PARTS>
+__device__ __forceinline__ void kinematics_parts(const Mesh& m, int i, double dt) {
     int nl[8];
     load_nodelist(m.nodelist, i, nl);
     bf::KinGeo g;
-    bf::KinVel kv;
-    bool ok = true;
+    bool geo = true, vel = true;
     {
         bf::Sums s;
         double x[8];
         gather8(m.x, nl, x);
-        ok &= bf::axis_sums<58>(x, 0, s);
+        geo &= bf::axis_sums<58>(x, 0, s);
         gather8(m.y, nl, x);
-        ok &= bf::axis_sums<58>(x, 1, s);
+        geo &= bf::axis_sums<58>(x, 1, s);
         gather8(m.z, nl, x);
-        ok &= bf::axis_sums<58>(x, 2, s);
-        ok &= bf::kin_geometry(s, g);
+        geo &= bf::axis_sums<58>(x, 2, s);
+        geo &= bf::kin_geometry(s, g);
     }
-    {
-        bf::VelSums v;
-        double x[8];
-        gather8(m.xd, nl, x);
-        ok &= bf::vel_sums(x, 0, v);
-        gather8(m.yd, nl, x);
-        ok &= bf::vel_sums(x, 1, v);
-        gather8(m.zd, nl, x);
-        ok &= bf::vel_sums(x, 2, v);
-        bf::kin_velocity(g, v, kv);
-    }
-    if (!ok) {
-        kinematics_double(m, i, dt);
-        return;
-    }
-    const double volo = LD(m.volo + i), vold = m.v[i];
+    const double volo = LD(m.volo + i);
     const double volume = g.vol192 * (1.0 / 192.0);
     double relv = quot_refined(volume, volo);
     if (static_cast<unsigned long long>(dbits(relv) - dbits(1.0) + kUlpsBelow) <= kUlpsBelow + kUlpsAbove) relv = 1.0;
-    m.vnew[i] = relv;
-    m.delv[i] = relv - vold;
-    m.arealg[i] = pmul(16.0 * volume, rsqrt(g.face2));
-    const double vol = pmul(volo, relv), vol16 = 16.0 * vol;
-    const double n64 = rcp(vol + 1.e-36) * 0.015625;
-    m.dxxi[i] = pmul(vol16, rsqrt(g.cc[0] + 256.0 * 1.e-36));
-    m.dxeta[i] = pmul(vol16, rsqrt(g.cc[1] + 256.0 * 1.e-36));
-    m.dxzeta[i] = pmul(vol16, rsqrt(g.cc[2] + 256.0 * 1.e-36));
-    m.dvxi[i] = pmul(kv.cv[0], n64);
-    m.dveta[i] = pmul(kv.cv[1], n64);
-    m.dvzeta[i] = pmul(kv.cv[2], n64);
-    const double t = 0.5 * dt, b = kv.cv[0] + kv.cv[1] + kv.cv[2];
-    const double num = fma(t, fma(3.0 * t, kv.detv, -2.0 * kv.ak), b);
-    const double den = fma(-t, fma(-t, fma(-t, kv.detv, kv.ak), b), g.det);
-    m.vdov[i] = quot(num, den);
-    update_volume(m, i, vold, relv);
+    const double vol = pmul(volo, relv);
+    if ((PARTS & kKinGeometry) && geo) {
+        const double vold = m.v[i], vol16 = 16.0 * vol;
+        m.vnew[i] = relv;
+        m.delv[i] = relv - vold;
+        m.arealg[i] = pmul(16.0 * volume, rsqrt(g.face2));
+        m.dxxi[i] = pmul(vol16, rsqrt(g.cc[0] + 256.0 * 1.e-36));
+        m.dxeta[i] = pmul(vol16, rsqrt(g.cc[1] + 256.0 * 1.e-36));
+        m.dxzeta[i] = pmul(vol16, rsqrt(g.cc[2] + 256.0 * 1.e-36));
+        update_volume(m, i, vold, relv);
+    }
+    if (PARTS & kKinVelocity) {
+        bf::VelSums v;
+        double x[8];
+        gather8(m.xd, nl, x);
+        vel &= bf::vel_sums(x, 0, v);
+        gather8(m.yd, nl, x);
+        vel &= bf::vel_sums(x, 1, v);
+        gather8(m.zd, nl, x);
+        vel &= bf::vel_sums(x, 2, v);
+        vel &= geo;
+        bf::KinVel kv;
+        bf::kin_velocity(g, v, kv);
+        if (vel) {
+            const double n64 = rcp(vol + 1.e-36) * 0.015625;
+            m.dvxi[i] = pmul(kv.cv[0], n64);
+            m.dveta[i] = pmul(kv.cv[1], n64);
+            m.dvzeta[i] = pmul(kv.cv[2], n64);
+            const double t = 0.5 * dt, b = kv.cv[0] + kv.cv[1] + kv.cv[2];
+            const double num = fma(t, fma(3.0 * t, kv.detv, -2.0 * kv.ak), b);
+            const double den = fma(-t, fma(-t, fma(-t, kv.detv, kv.ak), b), g.det);
+            m.vdov[i] = quot(num, den);
+        }
+    }
+    const int again = PARTS & ((geo ? 0 : kKinGeometry) | (vel ? 0 : kKinVelocity));
+    if (again) kinematics_double(m, i, dt, again);
+}
+__device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt) {
+    kinematics_parts<kKinGeometry | kKinVelocity>(m, i, dt);
 }
 #endif
 
@@ -368,6 +396,27 @@ __device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int l
 // 0.92 ms with 2, 3, 4 blocks (4 spills a little), k_kinematics 1.13, 0.87,
 // 0.83 (5: 0.85).
 constexpr int kForceBlocks = LULESH_EXACT ? 1 : 4, kKinBlocks = LULESH_EXACT ? 1 : 4;
+
+#if !LULESH_EXACT
+// The same for few elements: one axis of an element to a thread (blockIdx.y),
+// and one part of its kinematics. The geometry is formed again for each, but
+// a mesh that leaves the multiprocessors idle takes as long as one thread.
+__global__ void __launch_bounds__(kForceBlock, kForceBlocks) k_forces_axis(Mesh m, int first, int end) {
+    if (m.dtime && !m.dtime->active) return;
+    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < end) forces_axes(m, i, blockIdx.y, blockIdx.y + 1);
+}
+__global__ void __launch_bounds__(kKinBlock, kKinBlocks) k_kinematics_part(Mesh m, double dt, int first, int end) {
+    if (m.dtime) {
+        if (!m.dtime->active) return;
+        dt = m.dtime->deltatime;
+    }
+    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= end) return;
+    if (blockIdx.y == 0) kinematics_parts<kKinGeometry>(m, i, dt);
+    else kinematics_parts<kKinVelocity>(m, i, dt);
+}
+#endif
 
 // all elements, or (RANGED) elements [first, end)
 template <bool RANGED>
@@ -425,27 +474,46 @@ __global__ void __launch_bounds__(kMatBlock, kMatBlocks) k_material(Mesh m, cons
     finish_dt_reduction(m, dtc, dth);
 }
 
-int launch_forces(const Mesh& m, cudaStream_t s) {
-    k_forces<false><<<blocks_for(m.numElem, kForceBlock), kForceBlock, 0, s>>>(m, 0, m.numElem);
-    return 1;
-}
+// Up to this many elements the forces' axes, and the kinematics' parts, go to
+// threads of their own: forces s=8 16.7 -> 10.5 us, s=16 16.6 -> 12.5, s=24
+// (13,824) the same, s=30 20.7 -> 22.8; kinematics s=8 14.3 -> 11.9, s=30
+// (27,000) 18.4 -> 16.4, s=34 20.6 -> 22.5.
+constexpr int kSplitElems = LULESH_EXACT ? 0 : 12000, kSplitKinElems = LULESH_EXACT ? 0 : 30000;
+
 int launch_forces_range(const Mesh& m, int first, int end, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_forces<true><<<blocks_for(end - first, kForceBlock), kForceBlock, 0, s>>>(m, first, end);
+    const int n = end - first, blocks = blocks_for(n, kForceBlock);
+    if (n <= 0) return 0;
+#if !LULESH_EXACT
+    if (n <= kSplitElems) {
+        k_forces_axis<<<dim3(blocks, 3), kForceBlock, 0, s>>>(m, first, end);
+        return 1;
+    }
+#endif
+    if (n == m.numElem) k_forces<false><<<blocks, kForceBlock, 0, s>>>(m, 0, n);
+    else k_forces<true><<<blocks, kForceBlock, 0, s>>>(m, first, end);
     return 1;
 }
+int launch_forces(const Mesh& m, cudaStream_t s) { return launch_forces_range(m, 0, m.numElem, s); }
 int launch_nodes(const Mesh& m, double dt, cudaStream_t s) {
-    k_nodes<<<blocks_for(m.numNode, kNodeBlock), kNodeBlock, 0, s>>>(m, dt);
-    return 1;
-}
-int launch_kinematics(const Mesh& m, double dt, cudaStream_t s) {
-    k_kinematics<false><<<blocks_for(m.numElem, kKinBlock), kKinBlock, 0, s>>>(m, dt, 0, m.numElem);
+    const int blocks = blocks_for(m.numNode, kNodeBlock);
+    k_nodes<<<blocks, kNodeBlock, 0, s>>>(m, dt);
     return 1;
 }
 int launch_kinematics_range(const Mesh& m, double dt, int first, int end, cudaStream_t s) {
-    if (end <= first) return 0;
-    k_kinematics<true><<<blocks_for(end - first, kKinBlock), kKinBlock, 0, s>>>(m, dt, first, end);
+    const int n = end - first, blocks = blocks_for(n, kKinBlock);
+    if (n <= 0) return 0;
+#if !LULESH_EXACT
+    if (n <= kSplitKinElems) {
+        k_kinematics_part<<<dim3(blocks, 2), kKinBlock, 0, s>>>(m, dt, first, end);
+        return 1;
+    }
+#endif
+    if (n == m.numElem) k_kinematics<false><<<blocks, kKinBlock, 0, s>>>(m, dt, 0, n);
+    else k_kinematics<true><<<blocks, kKinBlock, 0, s>>>(m, dt, first, end);
     return 1;
+}
+int launch_kinematics(const Mesh& m, double dt, cudaStream_t s) {
+    return launch_kinematics_range(m, dt, 0, m.numElem, s);
 }
 int launch_material(const Mesh& m, const MatPlan& plan, cudaStream_t s) {
     if (plan.spread) k_material<true><<<plan.grid, kMatBlock, 0, s>>>(m, plan);

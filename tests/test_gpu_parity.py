@@ -353,6 +353,36 @@ def test_pinned_and_pageable_copies_agree(lulesh, s, precision):
         dev.close()
 
 
+@pytest.mark.parametrize("s", [8, 22, 23, 31, 32])
+def test_split_kernels_equal_whole_ones(lulesh, s):
+    """Few elements give each axis of the forces and each part of the
+    kinematics a thread of its own (up to 12,000 and 30,000 elements: s=22 and
+    s=31 are the last). The drop-in call's slabs are below those sizes where
+    the whole mesh is not: same bits, with some elements outside the fixed
+    point's range (a flat and a fast one)."""
+    a, b = lulesh.HostDomain(s, 11), lulesh.HostDomain(s, 11)
+    rng = np.random.default_rng(s)
+    h = 1.125 / s
+    for f in ("x", "y", "z", "xd", "yd", "zd"):
+        v = getattr(a, f)
+        v += rng.uniform(-0.1, 0.1, v.size) * (h if len(f) == 1 else 50.0)
+        getattr(b, f)[:] = v
+    en = s + 1
+    for d in (a, b):
+        d.z[d.nodelist[4:8]] = d.z[d.nodelist[0:4]] + h / 40  # element 0: 40 times wider than high
+        d.yd[en * en * en // 2] = 1e200  # velocity outside the range
+        d.p[:] = d.ss[:] = 1.0
+        d.time_state.deltatime = 1e-9
+    dev_a, dev_b = lulesh.Device(a, "fp64"), lulesh.Device(b, "fp64")
+    dev_a.step(1e-9)
+    dev_a.download()
+    dev_b.leapfrog()
+    for f in NODE + ELEM:
+        np.testing.assert_array_equal(getattr(a, f), getattr(b, f), err_msg=f)
+    dev_a.close()
+    dev_b.close()
+
+
 MATERIAL_KINDS = ["plain", "cold", "opening", "closing", "still", "huge", "faint", "negative", "half_cold", "folded"]
 
 

@@ -1,8 +1,8 @@
 // Block fixed point: sums and products of doubles on the integer pipes.
 //
 // GB300's FP64 pipe takes 62 cycles for a warp's double multiply-add and 73
-// for an add (per SM quarter); a 64-bit integer add takes 2 and a 32 x 32 +
-// 64 bit multiply-add (mad.wide) 2. The element kernels' vector arithmetic,
+// for an add (per SM quarter); a 64-bit integer add takes 2 and a 32 x 32 bit
+// product of 64 bits (mul.wide) 3. The element kernels' vector arithmetic,
 // sums of corner values and products of such sums, therefore runs in
 // 64-bit integers that share one power-of-two unit per block of values:
 //
@@ -10,7 +10,7 @@
 //     by the largest of them. Corners within a factor 2 (4) of it are exact
 //     (53 bits), so sums of corners are exact where a double sum would round.
 //   * a value splits into limbs h * 2^29 + l; a product adds h h' to one
-//     64-bit sum and h l' + l h' to another (3 mad.wide), and their value, in
+//     64-bit sum and h l' + l h' to another (3 mul.wide), and their value, in
 //     units of 2^58 of the product, is off by about one unit: some 2^-56 of
 //     the block's largest product, against 2^-53 of each product and each
 //     sum in double.
@@ -61,11 +61,14 @@ LULESH_BF double up_exponent(double x, int k) { return __hiloint2double(__double
 LULESH_BF int64_t round_to_int(double x) { return __double2ll_rn(x); }
 LULESH_BF double to_double(int64_t v) { return __ll2double_rn(v); }
 LULESH_BF int lead_zeros(uint32_t v) { return __clz(int(v)); }
-// Written out: the compiler turns (-a) * b + c into a product and a subtraction.
+// Product and sum apart: a multiply-add with a 64-bit addend takes 6.2 cycles
+// of its pipe, the product alone 3.3 and the addition, two to three of which
+// go together, runs on others (s=150: forces 0.90 -> 0.78 ms, kinematics
+// 0.69 -> 0.65, material 0.66 -> 0.63).
 LULESH_BF int64_t wide(int32_t a, int32_t b, int64_t c) {
     int64_t r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+    return r + c;
 }
 // v << s as limbs for 0 <= s < 29
 LULESH_BF Limb limb_up(int64_t v, int s) {
@@ -96,24 +99,53 @@ LULESH_BF void mac(Acc& s, Limb a, Limb b) {
     s.hh = wide(a.h, b.h, s.hh);
     s.mid = wide(a.l, b.h, wide(a.h, b.l, s.mid));
 }
+LULESH_BF Acc self_product(Limb a) { return {wide(a.h, a.h, 0), wide(a.l, 2 * a.h, int64_t(1) << (kLow - 1))}; }
+LULESH_BF void mac_self(Acc& s, Limb a) {
+    s.hh = wide(a.h, a.h, s.hh);
+    s.mid = wide(a.l, 2 * a.h, s.mid);
+}
 LULESH_BF int64_t value(Acc s) { return s.hh + (s.mid >> kLow); }
 LULESH_BF int64_t mul(Limb a, Limb b) { return value(product(a, b)); }
+// The same with the middle products' sum cut at its high word: off by up to 4
+// units (some 2^-54 of the block's largest product, still below what double
+// sums of them lose), for two instructions in place of four.
+LULESH_BF int64_t near(Acc s) { return wide(int32_t((s.mid + (int64_t(1) << 31)) >> 32), 8, s.hh); }
+LULESH_BF int64_t mul_near(Limb a, Limb b) { return near(product(a, b)); }
 
-// The width of a block: the high words of its magnitudes OR-ed together.
-LULESH_BF uint32_t top_bits(int64_t v) {
-    const int32_t h = int32_t(v >> 32);
-    return uint32_t(h ^ (h >> 31));
-}
-// Left shift that brings a block of values below 2^top, whose OR-ed top bits
-// are m, to at least 2^(top - 1) (or by top - 32, when all are below 2^32).
-LULESH_BF int room(uint32_t m, int top) { return lead_zeros(m) - (64 - top); }
+// The width of a block: the largest high word of its values or of their
+// complements, two values to an instruction.
+#ifdef __CUDACC__
+LULESH_BF int32_t max3(int32_t a, int32_t b, int32_t c) { return __vimax3_s32(a, b, c); }
+LULESH_BF int32_t min3(int32_t a, int32_t b, int32_t c) { return __vimin3_s32(a, b, c); }
+#else
+LULESH_BF int32_t max3(int32_t a, int32_t b, int32_t c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
+LULESH_BF int32_t min3(int32_t a, int32_t b, int32_t c) { return a < b ? (a < c ? a : c) : (b < c ? b : c); }
+#endif
+struct Top {
+    int32_t hi = 0, lo = 0;
+#ifdef __CUDACC__
+    __device__ __forceinline__
+#endif
+    void add(int64_t v, int64_t w) {
+        hi = max3(hi, int32_t(v >> 32), int32_t(w >> 32));
+        lo = min3(lo, int32_t(v >> 32), int32_t(w >> 32));
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__
+#endif
+    void add(int64_t v) { add(v, v); }
+};
+LULESH_BF uint32_t top_bits(Top t) { return uint32_t(t.hi > ~t.lo ? t.hi : ~t.lo); }
+// Left shift that brings a block of values below 2^top to at least 2^(top - 1)
+// (or by top - 32, when all are below 2^32).
+LULESH_BF int room(Top m, int top) { return lead_zeros(top_bits(m)) - (64 - top); }
 LULESH_BF int64_t down(int64_t v, int s) { return v >> s; }
 LULESH_BF int clamp63(int s) { return s < 63 ? s : 63; }
 
 // 8 doubles as integers up to 2^(WIDTH - 3), so that their signed sums stay
 // below 2^WIDTH, times 2^unit. False where they do not fit. A block of zeros
 // (or of values below 2^-1042) is all zero.
-template <int WIDTH>
+template <int WIDTH, bool CVT>
 LULESH_BF bool fix8(const double v[8], int64_t q[8], int& unit) {
     int32_t top = 0;
     LULESH_UNROLL
@@ -123,8 +155,24 @@ LULESH_BF bool fix8(const double v[8], int64_t q[8], int& unit) {
     }
     const int e = top >> 20;
     unit = e - (kBias + WIDTH);
+    // CVT: by the FP64 pipe's conversion, 62 cycles. Else the significand is
+    // shifted into place by 15 integer instructions. The kernels take what
+    // balances their pipes: kinematics, with 80 FP64 instructions of other
+    // kinds, the latter (s=150: 0.717 -> 0.633 ms), forces the former for the
+    // velocities only (0.780; 0.790 with integers for all, 0.819 with
+    // conversions for all, 0.803 the other way round).
     LULESH_UNROLL
-    for (int k = 0; k < 8; ++k) q[k] = round_to_int(up_exponent(v[k], kBias + WIDTH - e));
+    for (int k = 0; k < 8; ++k) {
+        if (CVT) {
+            q[k] = round_to_int(up_exponent(v[k], kBias + WIDTH - e));
+            continue;
+        }
+        const int64_t b = bits_of(v[k]);
+        const int n = e - (int(b >> 52) & 0x7ff);
+        const uint64_t m = uint64_t((b & 0xfffffffffffffll) | 0x10000000000000ll) << (WIDTH - 56);
+        const int64_t a = int64_t(m >> clamp63(n)), s = b >> 63;
+        q[k] = (a ^ s) - s;
+    }
     return top == 0 || (e >= 64 && e <= kBias + WIDTH);
 }
 
@@ -203,16 +251,16 @@ struct Sums {
     int unit[3];
 };
 
-template <int WIDTH>
+template <int WIDTH, bool CVT>
 LULESH_BF bool axis_sums(const double x[8], int a, Sums& s) {
     int64_t q[8], d[3], h[4];
-    const bool ok = fix8<WIDTH>(x, q, s.unit[a]);
+    const bool ok = fix8<WIDTH, CVT>(x, q, s.unit[a]);
     walsh(q, d, h);
-    uint32_t m = 0;
-    LULESH_UNROLL
-    for (int k = 0; k < 3; ++k) m |= top_bits(d[k]);
-    LULESH_UNROLL
-    for (int k = 0; k < 4; ++k) m |= top_bits(h[k]);
+    Top m;
+    m.add(d[0], d[1]);
+    m.add(d[2], h[0]);
+    m.add(h[1], h[2]);
+    m.add(h[3]);
     const int up = room(m, WIDTH);
     s.unit[a] -= up;
     LULESH_UNROLL
@@ -250,7 +298,7 @@ struct ForceGeo {
 // or near zero.
 LULESH_BF bool force_geometry(const Sums& s, ForceGeo& o) {
     int64_t g[6][3];
-    uint32_t m = 0;
+    Top m;
     bool ok = true;
     LULESH_UNROLL
     for (int d = 0; d < 3; ++d) {
@@ -263,7 +311,7 @@ LULESH_BF bool force_geometry(const Sums& s, ForceGeo& o) {
             o.n[d][a] = c + e;
             g[d][a] = (o.n[d][a] + 2 * c) >> 1;  // up to 2^58
             g[3 + d][a] = value(cross2(s.H[j], s.A[i], s.A[j], s.H[i], a)) >> 1;
-            m |= top_bits(g[d][a]) | top_bits(g[3 + d][a]);
+            m.add(g[d][a], g[3 + d][a]);
             if (d == 0) {
                 if (a == 0) det = product(s.A[0][a], limb(c));
                 else mac(det, s.A[0][a], limb(c));
@@ -320,14 +368,14 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
                           double out[8]) {
     int64_t q[8], v[3], amp[4];
     int unit;
-    bool ok = fix8<kUnit - 1>(vel, q, unit);
+    bool ok = fix8<kUnit - 1, true>(vel, q, unit);
     const bool still = unit == -(kBias + kUnit - 1);  // all zero
     walsh(q, v, amp);
-    uint32_t m = 0;
-    LULESH_UNROLL
-    for (int d = 0; d < 3; ++d) m |= top_bits(v[d]);
-    LULESH_UNROLL
-    for (int k = 0; k < 4; ++k) m |= top_bits(amp[k]);
+    Top m;
+    m.add(v[0], v[1]);
+    m.add(v[2], amp[0]);
+    m.add(amp[1], amp[2]);
+    m.add(amp[3]);
     const int up = room(m, kUnit - 1);
     unit -= up;
     Limb vl[6];  // below 2^57
@@ -339,48 +387,46 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
     for (int k = 0; k < 4; ++k) amp[k] <<= up;
     // T, up to 6 2^57 / 2
     int64_t t[3];
-    m = 0;
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) {
         Acc s = product(o.g[0][a], vl[0]);
         LULESH_UNROLL
         for (int j = 1; j < 6; ++j) mac(s, o.g[j][a], vl[j]);
-        t[a] = value(s) >> 1;
-        m |= top_bits(t[a]);
+        t[a] = near(s) >> 1;
     }
-    const int nt = room(m, kUnit + 1);
+    Top mt;
+    mt.add(t[0], t[1]);
+    mt.add(t[2]);
+    const int nt = room(mt, kUnit + 1);
     Limb tl[3];  // below 2^59
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) tl[a] = limb_up(t[a], nt);
     // H_m . T, up to 3 2^58, then times sc; a correction that does not fit
     // beside W takes the double path
     int64_t r[4];
-    m = 0;
     LULESH_UNROLL
     for (int k = 0; k < 4; ++k) {
         Acc s = product(o.H[k][0], tl[0]);
         mac(s, o.H[k][1], tl[1]);
         mac(s, o.H[k][2], tl[2]);
-        r[k] = value(s);
-        m |= top_bits(r[k]);
+        r[k] = near(s);
     }
-    const int np = room(m, kUnit + 2);
-    m = 0;
+    Top mp, mr, ma;
+    mp.add(r[0], r[1]);
+    mp.add(r[2], r[3]);
+    const int np = room(mp, kUnit + 2);
     LULESH_UNROLL
-    for (int k = 0; k < 4; ++k) {
-        r[k] = mul(limb_up(r[k], np), f.sc);
-        m |= top_bits(r[k]);
-    }
+    for (int k = 0; k < 4; ++k) r[k] = mul_near(limb_up(r[k], np), f.sc);
+    mr.add(r[0], r[1]);
+    mr.add(r[2], r[3]);
     int right = nt - 1 + np - f.kappa;
-    ok &= right >= 0 && lead_zeros(m) + right >= 6;  // below 2^58
+    ok &= right >= 0 && lead_zeros(top_bits(mr)) + right >= 6;  // below 2^58
     right = clamp63(right);
-    m = 0;
     LULESH_UNROLL
-    for (int k = 0; k < 4; ++k) {
-        amp[k] -= down(r[k], right);
-        m |= top_bits(amp[k]);
-    }
-    const int na = room(m, kUnit + 1);
+    for (int k = 0; k < 4; ++k) amp[k] -= down(r[k], right);
+    ma.add(amp[0], amp[1]);
+    ma.add(amp[2], amp[3]);
+    const int na = room(ma, kUnit + 1);
     unit -= na;
     Limb al[4];  // below 2^59
     LULESH_UNROLL
@@ -389,16 +435,17 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
         amp[k] <<= na;
     }
     // U, up to 4 2^58, then times sc
-    m = 0;
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) {
         Acc s = product(o.H[0][a], al[0]);
         LULESH_UNROLL
         for (int k = 1; k < 4; ++k) mac(s, o.H[k][a], al[k]);
-        t[a] = mul(limb(value(s)), f.sc);
-        m |= top_bits(t[a]);
+        t[a] = mul_near(limb(near(s)), f.sc);
     }
-    const int nu = room(m, kUnit + 2);
+    Top mu;
+    mu.add(t[0], t[1]);
+    mu.add(t[2]);
+    const int nu = room(mu, kUnit + 2);
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) tl[a] = limb_up(t[a], nu);
     // coefficients of the force in the Walsh basis
@@ -406,28 +453,32 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
     right = nu - f.kappa;
     ok &= right >= 0;
     right = clamp63(right);
-    uint32_t mr = 0;
-    m = 0;
+    Top mc, mw;
     LULESH_UNROLL
     for (int j = 0; j < 6; ++j) {
         Acc s = product(o.g[j][0], tl[0]);
         mac(s, o.g[j][1], tl[1]);
         mac(s, o.g[j][2], tl[2]);
-        const int64_t p = down(value(s), right);
-        mr |= top_bits(p);
-        w[j] = (j >= 3 ? amp[j - 3] : 0) - p;
-        m |= top_bits(w[j]);
+        w[j] = near(s);
     }
+    mc.add(w[0], w[1]);
+    mc.add(w[2], w[3]);
+    mc.add(w[4], w[5]);
+    ok &= lead_zeros(top_bits(mc)) + right >= 5;  // below 2^59, so w stays below 2^60
+    LULESH_UNROLL
+    for (int j = 0; j < 6; ++j) w[j] = (j >= 3 ? amp[j - 3] : 0) - down(w[j], right);
     w[6] = amp[3];
-    m |= top_bits(w[6]);
-    ok &= lead_zeros(mr) >= 5;  // below 2^59, so w stays below 2^60
-    const int nw = room(m, kUnit + 2);
+    mw.add(w[0], w[1]);
+    mw.add(w[2], w[3]);
+    mw.add(w[4], w[5]);
+    mw.add(w[6]);
+    const int nw = room(mw, kUnit + 2);
     const int u1 = still ? kNone : kUnit + unit + f.ucoef - nw;
     // stress
-    m = 0;
-    LULESH_UNROLL
-    for (int d = 0; d < 3; ++d) m |= top_bits(n[d]);
-    const int ns = room(m, kUnit + 2);
+    Top mn;
+    mn.add(n[0], n[1]);
+    mn.add(n[2]);
+    const int ns = room(mn, kUnit + 2);
     const int u2 = f.upress - unit_a - ns;
     const int u = u1 > u2 ? u1 : u2, s1 = clamp63(u - u1), s2 = clamp63(u - u2);
     int64_t x[3], h[4];  // up to 2 2^60 and 2^60: a quarter of it in the corner sums
@@ -473,7 +524,7 @@ LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {
     o.cross = s.unit[0] + s.unit[1] + s.unit[2];
     const int square = kUnit + 2 * (kUnit + o.cross - lo);  // unit of a square of vectors in the coarsest unit
     int64_t n[3][3];
-    uint32_t mn = 0;
+    Top mn;
     int coarse[3];
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) coarse[a] = clamp63(s.unit[a] - lo);
@@ -481,21 +532,23 @@ LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {
     for (int d = 0; d < 3; ++d) {
         const int i = (d + 1) % 3, j = (d + 2) % 3;
         int64_t cs[3];
-        uint32_t m = 0;
         LULESH_UNROLL
         for (int a = 0; a < 3; ++a) {
             const int64_t c = value(cross(s.A[i], s.A[j], a));  // up to 2^59
             n[d][a] = (c + value(cross(s.H[j], s.H[i], a))) >> 2;
-            mn |= top_bits(n[d][a]);
             o.c[d][a] = limb(c);
             cs[a] = down(c, clamp63(coarse[a] + 1));
-            m |= top_bits(cs[a]);
         }
+        mn.add(n[d][0], n[d][1]);
+        mn.add(n[d][2]);
+        Top m;
+        m.add(cs[0], cs[1]);
+        m.add(cs[2]);
         const int up = room(m, kUnit);
         const Limb l0 = limb_up(cs[0], up), l1 = limb_up(cs[1], up), l2 = limb_up(cs[2], up);
-        Acc sq = product(l0, l0);
-        mac(sq, l1, l1);
-        mac(sq, l2, l2);
+        Acc sq = self_product(l0);
+        mac_self(sq, l1);
+        mac_self(sq, l2);
         o.cc[d] = scaled(value(sq), square - 2 * (up - 1));
     }
     const int nv = room(mn, kUnit);
@@ -514,7 +567,7 @@ LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {
     o.vol192 = scaled(value(vol), 2 * kUnit + o.cross + 2 - nv);
     // faces: an eighth of n and of the differences of P in the coarsest unit, up to 2^57
     int64_t p[3][3];
-    uint32_t m = 0;
+    Top m;
     LULESH_UNROLL
     for (int a = 0; a < 3; ++a) {
         const int64_t p0 = value(cross(s.A[0], s.H[0], a)), p1 = value(cross(s.A[1], s.H[1], a)),
@@ -526,7 +579,7 @@ LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {
         LULESH_UNROLL
         for (int d = 0; d < 3; ++d) {
             n[d][a] = down(n[d][a], down1);
-            m |= top_bits(p[d][a]) | top_bits(n[d][a]);
+            m.add(p[d][a], n[d][a]);
         }
     }
     const int nf = room(m, kUnit - 1);
@@ -538,11 +591,11 @@ LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {
         for (int a = 0; a < 3; ++a) {
             const Limb lp = limb_up(n[d][a] + p[d][a], nf), lm = limb_up(n[d][a] - p[d][a], nf);
             if (a == 0) {
-                plus = product(lp, lp);
-                minus = product(lm, lm);
+                plus = self_product(lp);
+                minus = self_product(lm);
             } else {
-                mac(plus, lp, lp);
-                mac(minus, lm, lm);
+                mac_self(plus, lp);
+                mac_self(minus, lm);
             }
         }
         const int64_t vp = value(plus), vm = value(minus);
@@ -567,9 +620,11 @@ struct VelSums {
 LULESH_BF bool vel_sums(const double v[8], int a, VelSums& o) {
     int64_t q[8], d[3], h[4];
     int unit;
-    const bool ok = fix8<kUnit>(v, q, unit);
+    const bool ok = fix8<kUnit, false>(v, q, unit);
     walsh(q, d, h);
-    const uint32_t m = top_bits(d[0]) | top_bits(d[1]) | top_bits(d[2]);
+    Top m;
+    m.add(d[0], d[1]);
+    m.add(d[2]);
     const int up = room(m, kUnit);
     LULESH_UNROLL
     for (int k = 0; k < 3; ++k) o.V[k][a] = limb_up(d[k], up);

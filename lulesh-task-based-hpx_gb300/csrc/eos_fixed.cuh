@@ -6,7 +6,7 @@
 // pipe that takes 5,000 per pass. Here energies are integers in one unit and
 // pressures (p, q and their sums) in another, both chosen per evaluation
 // from the exponents of its inputs so that nothing can grow out of 60 bits:
-// sums are integer adds, products 3 mad.wide and a shift. Reciprocals and
+// sums are integer adds, products 3 mul.wide and a shift. Reciprocals and
 // square roots start from the float unit's approximation and take one
 // third-order step. Energies keep 2^-57 of the larger of the old energy and
 // the work done, so the result's error is below the double chain's; the

@@ -176,11 +176,11 @@ __device__ __forceinline__ void forces_axes(const Mesh& m, int i, int first, int
         bf::Sums s;
         double x[8];
         gather8(m.x, nl, x);
-        ok &= bf::axis_sums<57>(x, 0, s);
+        ok &= bf::axis_sums<57, false>(x, 0, s);
         gather8(m.y, nl, x);
-        ok &= bf::axis_sums<57>(x, 1, s);
+        ok &= bf::axis_sums<57, false>(x, 1, s);
         gather8(m.z, nl, x);
-        ok &= bf::axis_sums<57>(x, 2, s);
+        ok &= bf::axis_sums<57, false>(x, 2, s);
         ok &= bf::force_geometry(s, g);
     }
     const double determ = LD(m.volo + i) * LD(m.v + i);
@@ -329,11 +329,11 @@ __device__ __forceinline__ void kinematics_parts(const Mesh& m, int i, double dt
         bf::Sums s;
         double x[8];
         gather8(m.x, nl, x);
-        geo &= bf::axis_sums<58>(x, 0, s);
+        geo &= bf::axis_sums<58, false>(x, 0, s);
         gather8(m.y, nl, x);
-        geo &= bf::axis_sums<58>(x, 1, s);
+        geo &= bf::axis_sums<58, false>(x, 1, s);
         gather8(m.z, nl, x);
-        geo &= bf::axis_sums<58>(x, 2, s);
+        geo &= bf::axis_sums<58, false>(x, 2, s);
         geo &= bf::kin_geometry(s, g);
     }
     const double volo = LD(m.volo + i);
@@ -391,11 +391,10 @@ __device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int l
 // --- single-problem kernels -------------------------------------------------
 
 // Resident blocks of 128 per SM asked of the compiler. The fast variant's
-// block fixed point is bound by instruction issue and its dependencies, with
-// room for warps up to 128 registers: at s=150 k_forces takes 1.21, 0.98,
-// 0.92 ms with 2, 3, 4 blocks (4 spills a little), k_kinematics 1.13, 0.87,
-// 0.83 (5: 0.85).
-constexpr int kForceBlocks = LULESH_EXACT ? 1 : 4, kKinBlocks = LULESH_EXACT ? 1 : 4;
+// block fixed point is bound by the integer multiply and add pipes, with room
+// for warps up to 128 registers: at s=150 k_forces takes 0.78, 0.82, 0.83 ms
+// with 4, 5, 6 blocks, k_kinematics 0.643, 0.633, 0.641.
+constexpr int kForceBlocks = LULESH_EXACT ? 1 : 4, kKinBlocks = LULESH_EXACT ? 1 : 5;
 
 #if !LULESH_EXACT
 // The same for few elements: one axis of an element to a thread (blockIdx.y),

@@ -69,22 +69,22 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 1) kb_phase(BatchCtl c, int gr
             }
             if (!s_active) continue;
             if (PHASE == 3) {
-                double dtc = 1.0e+20, dth = 1.0e+20;
+                DtMin<LULESH_EXACT> dt;
                 const MatClass cls{tile.first, tile.count, tile.lanes, 0};
                 const int per_warp = 32 / cls.lanes;
                 for (int w = threadIdx.x >> 5; w * per_warp < cls.count; w += blockDim.x >> 5) {
                     int pos, r;
                     material_place(cls, w, pos, r);
-                    material_elem<true>(m, pos, r, cls.lanes, dtc, dth);
+                    material_elem<true>(m, pos, r, cls.lanes, dt);
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
-                    dtc = fmin(dtc, __shfl_down_sync(0xffffffffu, dtc, o));
-                    dth = fmin(dth, __shfl_down_sync(0xffffffffu, dth, o));
+                    dt.dtc = fmin(dt.dtc, __shfl_down_sync(0xffffffffu, dt.dtc, o));
+                    dt.dth = fmin(dt.dth, __shfl_down_sync(0xffffffffu, dt.dth, o));
                 }
                 if ((threadIdx.x & 31) == 0) {
-                    atomic_min_pos(&m.result->dtcourant, dtc);
-                    atomic_min_pos(&m.result->dthydro, dth);
+                    atomic_min_pos(&m.result->dtcourant, dt.dtc);
+                    atomic_min_pos(&m.result->dthydro, dt.dth);
                 }
             } else {
                 for (int k = threadIdx.x; k < tile.count; k += blockDim.x) {

@@ -92,8 +92,9 @@ LULESH_BF EosCuts eos_cuts(double e_cut, double p_cut, double q_cut, double pmin
     c.up = exponent(p_cut) - 1080;
     c.emin = exponent(emin);
     // cutoffs in [2^-300, 2^300], as far from the flushed 2^-1022 as from overflow
-    c.ok = e_cut >= 4.9e-91 && e_cut <= 2.0e90 && p_cut >= 4.9e-91 && p_cut <= 2.0e90 && q_cut >= 4.9e-91 &&
-           q_cut <= 2.0e90 && pmin == 0.0 && emin < 0.0 && refdens == 1.0;
+    auto sane = [](double x) { return bits_of(x) >= bits_of(4.9e-91) && bits_of(x) <= bits_of(2.0e90); };
+    c.ok = sane(e_cut) && sane(p_cut) && sane(q_cut) && bits_of(pmin) << 1 == 0 && bits_of(emin) < 0 && bits_of(emin) << 1 != 0 &&
+           uint64_t(bits_of(emin)) <= 0xfff0000000000000ull && bits_of(refdens) == bits_of(1.0);
     return c;
 }
 
@@ -127,7 +128,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
               xd = exponent(delv), xv = exponent(v);
     // everything normal or zero, of sane magnitude; |delv| below v
     bool ok = xe < 1800 && xp < 1800 && xq < 1800 && xl < 1800 && xqq < 1800 && xd <= xv && xv > 700 && xv < 1400 &&
-              v > 0.0;
+              bits_of(v) >= 0;
     // |x| < 2^(exponent - 1022): tops of the pressures (tp) and energies (te)
     const int tb = 1024 - xv;     // of 2/3 / v and 2/3 / vhalf
     const int th = xd - 1023;     // of delv / 2
@@ -158,7 +159,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     const int nw = ue - (xd - 1081 + up + 58);
     ok &= nph >= 0 && npv >= 0 && nw >= 2;
     const int sph = clamp63(nph), spv = clamp63(npv), sw = clamp63(nw), sw2 = clamp63(nw - 2);
-    const bool opening = delv > 0.0;
+    const bool opening = bits_of(delv) > 0;
     const Limb lf = limb(mul(mantissa(ql), kRootFull)), lc = limb(mul(mantissa(ql), kRootCut));
     const int ul = xl - 1080 + 1, ql_unit = up - (ul + 58);
     const int64_t pq = po + qo;
@@ -203,7 +204,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     const double lin = scaled(mul(limb(s), off ? lc : lf), us + ul + 58);
     q_new = opening ? 0.0 : (warm ? lin : .3333333e-18 * ql) + qq;
     ss = scaled(mul(s, off ? kRootCut : kRootFull), us + 1);
-    ss = warm && ss > .33333331e-18 ? ss : .3333333e-18;
+    ss = warm && bits_of(ss) > bits_of(.33333331e-18) ? ss : .3333333e-18;
     return ok;
 }
 

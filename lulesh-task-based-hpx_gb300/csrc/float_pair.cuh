@@ -19,12 +19,12 @@ __device__ __noinline__ float2 split_convert(double v) {
 }
 
 __device__ __forceinline__ float2 split(double v) {
-    const unsigned long long b = __double_as_longlong(v);
+    const unsigned long long b = dmul_bits(v);
     const unsigned e = unsigned(b >> 52) & 0x7ffu;
     if ((b << 1) == 0ull) return make_float2(__uint_as_float(unsigned(b >> 32)), 0.0f);  // +-0
     if (e < 949u || e > 1150u) return split_convert(v);
     const unsigned long long hb = round_to_float_bits(b);
-    const unsigned long long lb = __double_as_longlong(v - __longlong_as_double(hb));
+    const unsigned long long lb = dmul_bits(v - __longlong_as_double(hb));
     return make_float2(float_from_rounded(hb), (lb << 1) == 0ull ? 0.0f : float_from_rounded(round_to_float_bits(lb)));
 }
 

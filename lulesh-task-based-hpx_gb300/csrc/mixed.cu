@@ -71,7 +71,7 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
         }
     }
     const double determ = LD(m.volo + i) * LD(m.v + i);
-    if (determ <= 0.0) {
+    if (f_le(determ, 0.0)) {
         raise_error(m.result, i, PHASE_FORCES);
         return;
     }
@@ -163,9 +163,9 @@ __device__ __forceinline__ void kinematics_elem(const Mesh& m, int i, double dt)
 }
 
 // Material phase of an element by several lanes (material_share).
-template <bool SPREAD>
-__device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int lanes, double& dtc, double& dth) {
-    material_share<SPREAD>(m, t, r, lanes, m.gvxi, m.gveta, m.gvzeta, m.gxxi, m.gxeta, m.gxzeta, dtc, dth);
+template <bool SPREAD, class Dt>
+__device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int lanes, Dt& dt) {
+    material_share<SPREAD>(m, t, r, lanes, m.gvxi, m.gveta, m.gvzeta, m.gxxi, m.gxeta, m.gxzeta, dt);
 }
 
 // --- single-problem kernels -------------------------------------------------
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kKinBlock) k_kinematics(Mesh m, double dt, int
 template <bool SPREAD>
 __global__ void __launch_bounds__(kMatBlock) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
     if (m.dtime && !m.dtime->active) return;
-    double dtc = 1.0e+20, dth = 1.0e+20;
+    DtMin<true> dt;
     if (SPREAD) {
         const int nwarps = gridDim.x * (kMatBlock / 32);
         for (int w = blockIdx.x * (kMatBlock / 32) + (threadIdx.x >> 5); w < plan.warps; w += nwarps) {
@@ -219,13 +219,14 @@ __global__ void __launch_bounds__(kMatBlock) k_material(Mesh m, const __grid_con
             while (k + 1 < plan.n && w >= plan.cls[k + 1].warp0) ++k;
             int t, r;
             material_place(plan.cls[k], w - plan.cls[k].warp0, t, r);
-            material_elem<true>(m, t, r, plan.cls[k].lanes, dtc, dth);
+            material_elem<true>(m, t, r, plan.cls[k].lanes, dt);
         }
     } else {
-        for (int t = blockIdx.x * kMatBlock + threadIdx.x; t < plan.count; t += gridDim.x * kMatBlock)
-            material_elem<false>(m, plan.cls[0].first + t, 0, 1, dtc, dth);
+        const int lane = threadIdx.x & 31;
+        for (int t = blockIdx.x * kMatBlock + threadIdx.x - lane; t < plan.count; t += gridDim.x * kMatBlock)
+            material_elem<false>(m, plan.cls[0].first + min(t + lane, plan.count - 1), t + lane < plan.count ? 0 : 1, 1, dt);
     }
-    finish_dt_reduction(m, dtc, dth);
+    finish_dt_reduction(m, dt.dtc, dt.dth);
 }
 
 int launch_mirror(const Mesh& m, cudaStream_t s) {

@@ -49,10 +49,10 @@ __global__ void __launch_bounds__(kBlock)
     // value, and a NaN candidate is then ignored as fmin ignores it
     double dtc = 1.0e+20, dth = 1.0e+20;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double courant, hydro;
-    if (i < n && dt_candidates(prm, __ldg(ss + i), __ldg(vdov + i), __ldg(arealg + i), courant, hydro)) {
-        dtc = fmin(dtc, courant);
-        dth = fmin(dth, hydro);
+    const double vd = i < n ? __ldg(vdov + i) : 0.0;
+    if (!f_is_zero(vd)) {
+        dtc = fmin(dtc, courant_bound(prm, __ldg(ss + i), vd, __ldg(arealg + i)));
+        dth = fmin(dth, hydro_bound(prm, vd));
     }
     block_min2(dtc, dth);
     __shared__ bool last;

@@ -273,7 +273,10 @@ __device__ __forceinline__ double quot_refined(double a, double b) {
 // Comparisons. On GB300 a double compare (DSETP) occupies the FP64 pipe,
 // which issues at 1/60 the integer rate. The fast variants compare the
 // doubles' bit patterns on the integer pipe instead: positive doubles order
-// like their 64-bit patterns, negative ones in reverse. For non-NaN inputs
+// like their 64-bit patterns, negative ones in reverse (through dmul_bits:
+// of bits that it sees to be a double's the compiler makes FP64 compares
+// again, which held the mixed material kernel at 117 FP64 instructions per
+// warp where 86 are left, 0.46 -> 0.37 ms at s=120). For non-NaN inputs
 // these give the IEEE results, except that -0 may compare below +0 (a test
 // that then stores the constant turns a -0 into +0). The exact variant keeps
 // the IEEE compares.
@@ -288,7 +291,7 @@ __device__ __forceinline__ bool f_abs_lt(double x, double c) { return fabs(x) < 
 __device__ __forceinline__ bool f_is_zero(double x) { return x == 0.0; }
 #else
 constexpr long long kMag = 0x7fffffffffffffffLL;
-__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ long long dbits(double x) { return static_cast<long long>(dmul_bits(x)); }
 __device__ __forceinline__ bool f_lt(double x, double c) {
     const long long bx = dbits(x), bc = dbits(c);
     return bc >= 0 ? bx < bc : (bx < 0 && (bx & kMag) > (bc & kMag));
@@ -343,7 +346,7 @@ __device__ __forceinline__ float float_from_rounded(unsigned long long b) {
 __device__ __noinline__ float narrow_convert(double v) { return __double2float_rn(v); }
 __device__ __noinline__ double widen_convert(float f) { return double(f); }
 __device__ __forceinline__ float narrow(double v) {
-    const unsigned long long b = __double_as_longlong(v);
+    const unsigned long long b = dmul_bits(v);
     const unsigned e = unsigned(b >> 52) & 0x7ffu;
     if ((b << 1) == 0ull) return __uint_as_float(unsigned(b >> 32));  // +-0
     if (e < 897u || e > 1150u) return narrow_convert(v);
@@ -994,6 +997,12 @@ __device__ __forceinline__ R limiter(const R* __restrict__ dv, int i, int bm, in
     return phi;
 }
 
+// Between double and a variant's Q type, on the integer pipes.
+__device__ __forceinline__ float to_real(double v, float) { return narrow(v); }
+__device__ __forceinline__ double to_real(double v, double) { return v; }
+__device__ __forceinline__ double to_double(float v) { return widen(v); }
+__device__ __forceinline__ double to_double(double v) { return v; }
+
 // Linear and quadratic q of one element (lulesh.cc:1448-1656). dv/dx are the
 // six gradient arrays.
 template <class R>
@@ -1022,15 +1031,15 @@ __device__ __forceinline__ void q_terms(const Mesh& m, int i, const R* dvxi, con
     if (f_gt(dxi, R(0.))) dxi = R(0.);
     if (f_gt(deta, R(0.))) deta = R(0.);
     if (f_gt(dzeta, R(0.))) dzeta = R(0.);
-    const R rho = R(quot(LD(m.elemMass + i), pmul(LD(m.volo + i), vnew)));
+    const R rho = to_real(quot(LD(m.elemMass + i), pmul(LD(m.volo + i), vnew)), R());
     const R qlin = pmul(pmul(-R(P.qlc_monoq), rho),
                         pmul(dxi, R(1.) - phixi) + pmul(deta, R(1.) - phieta) + pmul(dzeta, R(1.) - phizeta));
     const R qquad = pmul(pmul(R(P.qqc_monoq), rho),
                          pmul(pmul(dxi, dxi), R(1.) - pmul(phixi, phixi)) +
                          pmul(pmul(deta, deta), R(1.) - pmul(phieta, phieta)) +
                          pmul(pmul(dzeta, dzeta), R(1.) - pmul(phizeta, phizeta)));
-    ql = double(qlin);
-    qq = double(qquad);
+    ql = to_double(qlin);
+    qq = to_double(qquad);
 }
 
 #if LULESH_FIXED_EOS
@@ -1101,17 +1110,27 @@ __device__ __forceinline__ double ss_guard(double ssc) {
 // Square root of the q terms' sound-speed expression (ss_guard's guard and
 // value). The mixed variant forms the linear and quadratic q coefficients
 // (ql, qq) in float, so its q terms take a float square root of the double
-// expression (two conversions and a float reciprocal square root instead of
-// the double sequence); the sound speed saved for the dt constraints stays
-// double.
+// expression (a float reciprocal square root instead of the double sequence,
+// and both conversions on the integer pipes); the sound speed saved for the
+// dt constraints stays double.
 #ifndef LULESH_FLOAT_Q
 #define LULESH_FLOAT_Q 0
+#endif
+#if LULESH_FLOAT_Q
+__device__ __noinline__ double q_sound_convert(double ssc) {
+    const float f = float(ssc);
+    return double(f * rsqrtf(f));
+}
 #endif
 __device__ __forceinline__ double q_sound(double ssc) {
 #if LULESH_FLOAT_Q
     if (f_le(ssc, .1111111e-36)) return .3333333e-18;
-    const float f = float(ssc);
-    return double(f * rsqrtf(f));
+    const unsigned long long b = static_cast<unsigned long long>(dbits(ssc));
+    if (b >= 0x47e0000000000000ull) return q_sound_convert(ssc);
+    // a normal float, as is its square root
+    const float f = float_from_rounded(round_to_float_bits(b));
+    const unsigned u = __float_as_uint(f * rsqrtf(f));
+    return __hiloint2double(int((u >> 3) + 0x38000000u), int(u << 29));
 #else
     return ss_guard(ssc);
 #endif
@@ -1301,11 +1320,8 @@ __device__ __forceinline__ EosState eos_element(const Mesh& m, int i, double vne
 }
 #endif
 
-// Courant and hydro candidates of one element (lulesh.cc:1938-1974); false
-// where vdov == 0 (the element does not constrain).
-__device__ __forceinline__ bool dt_candidates(const lulesh_params& P, double ss, double vdov,
-                                              double arealg, double& courant, double& hydro) {
-    if (f_is_zero(vdov)) return false;
+// Courant and hydro candidates of one element with vdov != 0 (lulesh.cc:1938-1974).
+__device__ __forceinline__ double courant_bound(const lulesh_params& P, double ss, double vdov, double arealg) {
     const double qqc2 = 64.0 * P.qqc * P.qqc;
 #if LULESH_EXACT
     double dtf = ss * ss;
@@ -1314,33 +1330,77 @@ __device__ __forceinline__ bool dt_candidates(const lulesh_params& P, double ss,
     double dtf = pmul(ss, ss);
     if (f_lt(vdov, 0.0)) dtf = fma(pmul(qqc2, pmul(arealg, arealg)), pmul(vdov, vdov), dtf);
 #endif
-    courant = div_sqrt(arealg, dtf);  // arealg / sqrt(dtf)
-    hydro = quot(P.dvovmax, fabs(vdov) + 1.e-20);
-    return true;
+    return div_sqrt(arealg, dtf);  // arealg / sqrt(dtf)
+}
+__device__ __forceinline__ double hydro_bound(const lulesh_params& P, double vdov) {
+    return quot(P.dvovmax, fabs(vdov) + 1.e-20);
 }
 
-// The same constraints folded into running minima (the candidates of the
-// step's own state are non-negative: ss, arealg >= 0).
-__device__ __forceinline__ void dt_constraints(const lulesh_params& P, double ss, double vdov,
-                                               double arealg, double& dtc, double& dth) {
-    double courant, hydro;
-    if (!dt_candidates(P, ss, vdov, arealg, courant, hydro)) return;
-    dtc = nonneg_min(dtc, courant);
-    dth = nonneg_min(dth, hydro);
+// Magnitude of a double within the floats' normal range, truncated to a float
+// (relative error below 2^-23); others set `off`.
+__device__ __forceinline__ float float_near(double v, bool& off) {
+    const unsigned hi = unsigned(dmul_bits(v) >> 32) & 0x7fffffffu;
+    off |= hi - 0x38100000u >= 0x47e00000u - 0x38100000u;
+    return __uint_as_float(__funnelshift_l(unsigned(__double2loint(v)), hi, 3) - (896u << 23));
 }
+
+// Running minima of the dt constraints in one warp. A candidate costs a
+// double square root and two reciprocals, some 60 slots of the FP64 pipe in
+// the exact variant and 13 in the fast ones, and only the least ones matter,
+// so an element whose candidate must be above one seen before in the warp
+// does not form it: the Courant bound is compared by its square in float
+// (off by some 2^-20, kept within 2^-15), the hydro bound, which falls with
+// |vdov|, by the high word of |vdov| (one more is 2^-20 of it). What the
+// comparison cannot tell (values beyond the float range, NaN) is formed. The
+// minima are those over all candidates (the candidates of the step's own
+// state are non-negative: ss, arealg >= 0).
+template <bool PRUNED>
+struct DtMin {
+    double dtc = 1.0e+20, dth = 1.0e+20;  // lulesh.cc:2214-2215
+    unsigned courant2 = 0x7f800000u;      // least square of a Courant bound seen, as float bits
+    int speed = 0;                        // greatest high word of |vdov| seen
+
+    // Every lane of the warp must call it; one without an element passes has
+    // = false.
+    __device__ __forceinline__ void add(const lulesh_params& P, bool has, double ss, double vdov, double arealg) {
+        has = has && !f_is_zero(vdov);
+        if (!PRUNED) {
+            if (has) fold(P, ss, vdov, arealg, true, true);
+            return;
+        }
+        if (!__any_sync(0xffffffffu, has)) return;
+        bool off = static_cast<long long>(dmul_bits(arealg)) < 0;
+        const float a = float_near(arealg, off), c = float_near(ss, off);
+        const float v = float_near(P.qqc, off) * 8.0f * a * float_near(vdov, off);
+        const float dtf = f_neg(vdov) ? c * c + v * v : c * c, est = __fdividef(a * a, dtf);
+        off |= !(a * a > 1e-30f && dtf > 1e-30f && dtf < 1e30f && est > 1e-30f && est < 1e30f);
+        const int hi = int(dmul_bits(vdov) >> 32) & 0x7fffffff;
+        courant2 = min(courant2, __reduce_min_sync(0xffffffffu, has && !off ? __float_as_uint(est) : 0x7f800000u));
+        speed = max(speed, __reduce_max_sync(0xffffffffu, has && hi < 0x7ff00000 ? hi : 0));
+        if (!has) return;
+        // below 2^-20 the 1e-20 may count
+        fold(P, ss, vdov, arealg, off || !(est > __uint_as_float(courant2) * (1.0f + 1.0f / 32768.0f)),
+             hi >= speed - 1 || speed < 0x3eb00000 || !(P.dvovmax > 0.0));
+    }
+    __device__ __forceinline__ void fold(const lulesh_params& P, double ss, double vdov, double arealg, bool courant,
+                                         bool hydro) {
+        if (courant) dtc = nonneg_min(dtc, courant_bound(P, ss, vdov, arealg));
+        if (hydro) dth = nonneg_min(dth, hydro_bound(P, vdov));
+    }
+};
 
 // Material phase of the element at position t of the repeat-count order
 // (matOrder) by `lanes` lanes of one warp, of which this is lane r: Q limiter
 // and q terms, this lane's share of the element's EOS passes, then (lane 0,
 // whose share is the largest) the save (lulesh.cc:1881-1904) and the
-// element's Courant and hydro constraints folded into dtc, dth. dv and dx are
-// the Q gradients, R their type. Every lane of the warp must call it; one
-// with r >= lanes runs no pass and saves nothing. Without SPREAD each lane
-// has an element of its own (r = 0, lanes = 1).
-template <bool SPREAD, class R>
+// element's Courant and hydro constraints folded into dt. dv and dx are the Q
+// gradients, R their type. Every lane of the warp must call it; one with
+// r >= lanes runs no pass and saves nothing. Without SPREAD each lane has an
+// element of its own (lanes = 1, and r = 0 or, in a lane without, 1).
+template <bool SPREAD, class R, class Dt>
 __device__ __forceinline__ void material_share(const Mesh& m, int t, int r, int lanes, const R* dvxi, const R* dveta,
                                                const R* dvzeta, const R* dxxi, const R* dxeta, const R* dxzeta,
-                                               double& dtc, double& dth) {
+                                               Dt& dt) {
     const int i = LD(m.matOrder + t);
     const double vnew = LD(m.vnew + i), vdov = LD(m.vdov + i);
     double ql, qq;
@@ -1349,7 +1409,7 @@ __device__ __forceinline__ void material_share(const Mesh& m, int t, int r, int 
 #else
     q_terms<R>(m, i, dvxi, dveta, dvzeta, dxxi, dxeta, dxzeta, vnew, vdov, ql, qq);
 #endif
-    if (!SPREAD || r == 0) {
+    if (r == 0) {
         m.qq[i] = qq;
         m.ql[i] = ql;
     }
@@ -1360,15 +1420,14 @@ __device__ __forceinline__ void material_share(const Mesh& m, int t, int r, int 
     const int rep = LD(m.elemRep + i);
     const int passes = !SPREAD || lanes == 1 ? (r == 0 ? rep : 0) : r < lanes ? (rep - r + lanes - 1) / lanes : 0;
     const EosState s = eos_element(m, i, vnewc, passes);
-    if (SPREAD) {
-        __syncwarp();  // no lane reads e, p, q of this element any more
-        if (r != 0) return;
+    if (SPREAD) __syncwarp();  // no lane reads e, p, q of this element any more
+    if (r == 0) {
+        m.ss[i] = s.ss;
+        m.p[i] = s.p;
+        m.e[i] = s.e;
+        m.q[i] = s.q;
     }
-    m.ss[i] = s.ss;
-    m.p[i] = s.p;
-    m.e[i] = s.e;
-    m.q[i] = s.q;
-    dt_constraints(m.prm, s.ss, vdov, LD(m.arealg + i), dtc, dth);
+    dt.add(m.prm, r == 0, s.ss, vdov, LD(m.arealg + i));
 }
 
 // The lane's element and share in warp w of a class: position t (the last

@@ -749,3 +749,40 @@ def test_mixed_size_sweep_against_double(lulesh):
     print("mixed vs double e(0), s=8..30:", " ".join(f"{e:.2e}" for e in errs))
     assert max(errs) <= E0_TOL_MIXED_ANY_SIZE, errs
     assert float(np.median(errs)) <= 1e-7, errs
+
+
+@pytest.mark.parametrize("precision", ["fp64_exact", "mixed"])
+@pytest.mark.parametrize("kind", ["random", "slow", "fast", "alike", "closing"])
+def test_time_step_bounds_of_many_elements(lulesh, precision, kind):
+    """A warp that takes several elements forms only the dt bounds that can be
+    the least: the minima are those over all elements (bit for bit in the
+    exact variant, within the rounding of the fast square root and reciprocal
+    otherwise), with velocity gradients below, within and beyond the float
+    range of its comparison, and almost equal ones."""
+    s = 64  # more elements than lanes in flight
+    rng = np.random.default_rng(3)
+    dom = lulesh.HostDomain(s, 11)
+    scale = {"slow": 1e-9, "fast": 1e25}.get(kind, 1.0)
+    for f, x in zip(("xd", "yd", "zd"), ("x", "y", "z")):
+        v = np.asarray(getattr(dom, x)).copy()
+        if kind == "random":
+            v *= rng.uniform(-1.0, 1.0, v.size)
+        elif kind != "alike":
+            v = rng.uniform(-1.0, 1.0, v.size)
+        getattr(dom, f)[:] = v * (-scale if kind == "closing" else scale)
+    dom.e[:] = rng.uniform(0.5, 1.0, s ** 3) * min(scale, 1e3)
+    dom.view.params.u_cut = 0.0
+    dev = lulesh.Device(dom, precision)
+    dtc, dth = dev.step(1e-9 / max(scale, 1.0))
+    dev.download(lulesh.F_SS | lulesh.F_KIN)
+    prm, a, vd = dom.view.params, np.asarray(dom.arealg), np.asarray(dom.vdov)
+    a, vd, ss = a[vd != 0.0], vd[vd != 0.0], np.asarray(dom.ss)[vd != 0.0]
+    dtf = ss * ss
+    closing = vd < 0.0
+    dtf[closing] += (64.0 * prm.qqc * prm.qqc * a * a * vd * vd)[closing]
+    # NaN (of a float that overflowed) is no bound, as in the reference's compares
+    want = [np.fmin.reduce(b, initial=1e20) for b in (a / np.sqrt(dtf), prm.dvovmax / (np.abs(vd) + 1e-20))]
+    assert vd.size > 0.9 * s ** 3
+    # fast: dtf 2, its reciprocal root 2, the product 1; 1 / |vdov| 2, the product 1 (half ulps and numpy's own 2)
+    np.testing.assert_allclose([dtc, dth], want, rtol=0 if precision == "fp64_exact" else 8 * 2.0 ** -53)
+    dev.close()

@@ -393,8 +393,11 @@ __device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int l
 // Resident blocks of 128 per SM asked of the compiler. The fast variant's
 // block fixed point is bound by the integer multiply and add pipes, with room
 // for warps up to 128 registers: at s=150 k_forces takes 0.78, 0.82, 0.83 ms
-// with 4, 5, 6 blocks, k_kinematics 0.643, 0.633, 0.641.
-constexpr int kForceBlocks = LULESH_EXACT ? 1 : 4, kKinBlocks = LULESH_EXACT ? 1 : 5;
+// with 4, 5, 6 blocks, k_kinematics 0.643, 0.633, 0.641. The exact variant's
+// out-of-line products leave a warp waiting on their chains: at s=60 k_forces
+// takes 0.594, 0.62, 0.536, 0.661 ms with 1 to 4 blocks, k_kinematics 0.274,
+// 0.274, 0.277, 0.282 (and 0.273 with 3 and its compares in integers).
+constexpr int kForceBlocks = LULESH_EXACT ? 3 : 4, kKinBlocks = LULESH_EXACT ? 3 : 5;
 
 #if !LULESH_EXACT
 // The same for few elements: one axis of an element to a thread (blockIdx.y),

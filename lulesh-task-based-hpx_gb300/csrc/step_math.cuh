@@ -46,6 +46,20 @@ __device__ __forceinline__ double pmul(double a, double b) { return dmul_ipipe(a
 #endif
 __device__ __forceinline__ float pmul(float a, float b) { return a * b; }
 
+// A product of the exact variant on the integer pipes (the same bits,
+// dmul_ipipe). Its kernels are bound by the FP64 pipe, 1,640 instructions an
+// element in k_forces, of which 680 products go here. Out of line, as so many
+// do not fit the instruction cache: inlined for the hourglass forces alone
+// k_forces takes 0.60 ms at s=60, with two products to a call 0.567, this way
+// 0.527 (0.609 without; k_kinematics 0.331 -> 0.273, material with its
+// compares in integers 0.341 -> 0.266). Plain in the other variants.
+#if LULESH_EXACT
+__device__ __noinline__ double xmul(double a, double b) { return dmul_ipipe(a, b); }
+#else
+template <class R>
+__device__ __forceinline__ R xmul(R a, R b) { return a * b; }
+#endif
+
 __device__ __forceinline__ void raise_error(StepResult* r, int elem, int phase) {
     if (atomicCAS(&r->err, 0, LULESH_EVOLUME) == 0) {
         r->err_elem = elem;
@@ -71,7 +85,7 @@ __device__ __forceinline__ void gather8(const double* __restrict__ f, const int 
 template <class R>
 __device__ __forceinline__ R triple(R x1, R y1, R z1, R x2, R y2, R z2, R x3, R y3, R z3) {
 #if LULESH_EXACT
-    return x1 * (y2 * z3 - z2 * y3) + x2 * (z1 * y3 - y1 * z3) + x3 * (y1 * z2 - z1 * y2);
+    return xmul(x1, xmul(y2, z3) - xmul(z2, y3)) + xmul(x2, xmul(z1, y3) - xmul(y1, z3)) + xmul(x3, xmul(y1, z2) - xmul(z1, y2));
 #else
     // the first product of each pair and of the sum on the integer pipes
     return fma(x3, fma(-z1, y2, pmul(y1, z2)),
@@ -101,7 +115,9 @@ __device__ __forceinline__ R hex_volume(const R x[8], const R y[8], const R z[8]
     return pmul(vol, twelveth);
 }
 
-// Centre Jacobian of CalcElemShapeFunctionDerivatives (lulesh.cc:277-305).
+// 8 times the centre Jacobian of CalcElemShapeFunctionDerivatives
+// (lulesh.cc:277-305): the powers of two of its determinant and shape
+// derivatives commute with rounding and cancel in the velocity gradient.
 template <class R>
 struct Jac {
     R fjxxi, fjxet, fjxze, fjyxi, fjyet, fjyze, fjzxi, fjzet, fjzze;
@@ -109,27 +125,26 @@ struct Jac {
 
 template <class R>
 __device__ __forceinline__ Jac<R> jacobian(const R x[8], const R y[8], const R z[8]) {
-    const R c = R(.125);
     Jac<R> j;
-    j.fjxxi = c * ((x[6] - x[0]) + (x[5] - x[3]) - (x[7] - x[1]) - (x[4] - x[2]));
-    j.fjxet = c * ((x[6] - x[0]) - (x[5] - x[3]) + (x[7] - x[1]) - (x[4] - x[2]));
-    j.fjxze = c * ((x[6] - x[0]) + (x[5] - x[3]) + (x[7] - x[1]) + (x[4] - x[2]));
-    j.fjyxi = c * ((y[6] - y[0]) + (y[5] - y[3]) - (y[7] - y[1]) - (y[4] - y[2]));
-    j.fjyet = c * ((y[6] - y[0]) - (y[5] - y[3]) + (y[7] - y[1]) - (y[4] - y[2]));
-    j.fjyze = c * ((y[6] - y[0]) + (y[5] - y[3]) + (y[7] - y[1]) + (y[4] - y[2]));
-    j.fjzxi = c * ((z[6] - z[0]) + (z[5] - z[3]) - (z[7] - z[1]) - (z[4] - z[2]));
-    j.fjzet = c * ((z[6] - z[0]) - (z[5] - z[3]) + (z[7] - z[1]) - (z[4] - z[2]));
-    j.fjzze = c * ((z[6] - z[0]) + (z[5] - z[3]) + (z[7] - z[1]) + (z[4] - z[2]));
+    j.fjxxi = (x[6] - x[0]) + (x[5] - x[3]) - (x[7] - x[1]) - (x[4] - x[2]);
+    j.fjxet = (x[6] - x[0]) - (x[5] - x[3]) + (x[7] - x[1]) - (x[4] - x[2]);
+    j.fjxze = (x[6] - x[0]) + (x[5] - x[3]) + (x[7] - x[1]) + (x[4] - x[2]);
+    j.fjyxi = (y[6] - y[0]) + (y[5] - y[3]) - (y[7] - y[1]) - (y[4] - y[2]);
+    j.fjyet = (y[6] - y[0]) - (y[5] - y[3]) + (y[7] - y[1]) - (y[4] - y[2]);
+    j.fjyze = (y[6] - y[0]) + (y[5] - y[3]) + (y[7] - y[1]) + (y[4] - y[2]);
+    j.fjzxi = (z[6] - z[0]) + (z[5] - z[3]) - (z[7] - z[1]) - (z[4] - z[2]);
+    j.fjzet = (z[6] - z[0]) - (z[5] - z[3]) + (z[7] - z[1]) - (z[4] - z[2]);
+    j.fjzze = (z[6] - z[0]) + (z[5] - z[3]) + (z[7] - z[1]) + (z[4] - z[2]);
     return j;
 }
 
-// Determinant only (lulesh.cc:308-373 without the B matrix).
+// 64 times the determinant only (lulesh.cc:308-373 without the B matrix).
 template <class R>
 __device__ __forceinline__ R jac_det(const Jac<R>& j) {
     const R cjxet = -(j.fjyxi * j.fjzze) + (j.fjzxi * j.fjyze);
     const R cjyet = (j.fjxxi * j.fjzze) - (j.fjzxi * j.fjxze);
     const R cjzet = -(j.fjxxi * j.fjyze) + (j.fjyxi * j.fjxze);
-    return R(8.) * (j.fjxet * cjxet + j.fjyet * cjyet + j.fjzet * cjzet);
+    return j.fjxet * cjxet + j.fjyet * cjyet + j.fjzet * cjzet;
 }
 
 #if !LULESH_EXACT
@@ -187,19 +202,19 @@ __device__ __forceinline__ bool jacobian_singular(const R x[8], const R y[8], co
 #endif
 }
 
-// Shape-function derivatives b[a][0..3] (b[a][4..7] are their negatives,
-// lulesh.cc:337-364) and the determinant.
+// 64 times the shape-function derivatives b[a][0..3] (b[a][4..7] are their
+// negatives, lulesh.cc:337-364) and 64 times the determinant.
 template <class R>
 __device__ __forceinline__ R shape_derivs(const Jac<R>& j, R b[3][4]) {
-    const R cjxxi = (j.fjyet * j.fjzze) - (j.fjzet * j.fjyze);
-    const R cjxet = -(j.fjyxi * j.fjzze) + (j.fjzxi * j.fjyze);
-    const R cjxze = (j.fjyxi * j.fjzet) - (j.fjzxi * j.fjyet);
-    const R cjyxi = -(j.fjxet * j.fjzze) + (j.fjzet * j.fjxze);
-    const R cjyet = (j.fjxxi * j.fjzze) - (j.fjzxi * j.fjxze);
-    const R cjyze = -(j.fjxxi * j.fjzet) + (j.fjzxi * j.fjxet);
-    const R cjzxi = (j.fjxet * j.fjyze) - (j.fjyet * j.fjxze);
-    const R cjzet = -(j.fjxxi * j.fjyze) + (j.fjyxi * j.fjxze);
-    const R cjzze = (j.fjxxi * j.fjyet) - (j.fjyxi * j.fjxet);
+    const R cjxxi = xmul(j.fjyet, j.fjzze) - xmul(j.fjzet, j.fjyze);
+    const R cjxet = -xmul(j.fjyxi, j.fjzze) + xmul(j.fjzxi, j.fjyze);
+    const R cjxze = xmul(j.fjyxi, j.fjzet) - xmul(j.fjzxi, j.fjyet);
+    const R cjyxi = -xmul(j.fjxet, j.fjzze) + xmul(j.fjzet, j.fjxze);
+    const R cjyet = xmul(j.fjxxi, j.fjzze) - xmul(j.fjzxi, j.fjxze);
+    const R cjyze = -xmul(j.fjxxi, j.fjzet) + xmul(j.fjzxi, j.fjxet);
+    const R cjzxi = xmul(j.fjxet, j.fjyze) - xmul(j.fjyet, j.fjxze);
+    const R cjzet = -xmul(j.fjxxi, j.fjyze) + xmul(j.fjyxi, j.fjxze);
+    const R cjzze = xmul(j.fjxxi, j.fjyet) - xmul(j.fjyxi, j.fjxet);
     b[0][0] = -cjxxi - cjxet - cjxze;
     b[0][1] = cjxxi - cjxet - cjxze;
     b[0][2] = cjxxi + cjxet - cjxze;
@@ -212,7 +227,7 @@ __device__ __forceinline__ R shape_derivs(const Jac<R>& j, R b[3][4]) {
     b[2][1] = cjzxi - cjzet - cjzze;
     b[2][2] = cjzxi + cjzet - cjzze;
     b[2][3] = -cjzxi + cjzet - cjzze;
-    return R(8.) * (j.fjxet * cjxet + j.fjyet * cjyet + j.fjzet * cjzet);
+    return xmul(j.fjxet, cjxet) + xmul(j.fjyet, cjyet) + xmul(j.fjzet, cjzet);
 }
 
 // Division helpers. x / refdens is x itself when refdens is 1 (the
@@ -271,24 +286,37 @@ __device__ __forceinline__ double quot_refined(double a, double b) {
 }
 
 // Comparisons. On GB300 a double compare (DSETP) occupies the FP64 pipe,
-// which issues at 1/60 the integer rate. The fast variants compare the
+// which issues at 1/60 the integer rate. All variants compare the
 // doubles' bit patterns on the integer pipe instead: positive doubles order
 // like their 64-bit patterns, negative ones in reverse (through dmul_bits:
 // of bits that it sees to be a double's the compiler makes FP64 compares
 // again, which held the mixed material kernel at 117 FP64 instructions per
 // warp where 86 are left, 0.46 -> 0.37 ms at s=120). For non-NaN inputs
 // these give the IEEE results, except that -0 may compare below +0 (a test
-// that then stores the constant turns a -0 into +0). The exact variant keeps
-// the IEEE compares.
+// that then stores the constant turns a -0 into +0). The exact variant's give
+// them for every input: in an order of the bits where -0 is +0, and false for
+// NaN (some 10 integer instructions; s=60 material 0.341 -> 0.304 ms).
 #if LULESH_EXACT
-__device__ __forceinline__ bool f_lt(double x, double c) { return x < c; }
-__device__ __forceinline__ bool f_le(double x, double c) { return x <= c; }
-__device__ __forceinline__ bool f_neg(double x) { return x < 0.0; }
+constexpr long long kMag = 0x7fffffffffffffffLL;
+__device__ __forceinline__ long long number_order(double x) {
+    const long long b = static_cast<long long>(dmul_bits(x)), s = b >> 63;
+    return ((b & kMag) ^ s) - s;
+}
+__device__ __forceinline__ bool is_number(double x) {
+    return (static_cast<long long>(dmul_bits(x)) & kMag) <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool f_lt(double x, double c) {
+    return number_order(x) < number_order(c) && is_number(x) && is_number(c);
+}
+__device__ __forceinline__ bool f_le(double x, double c) {
+    return number_order(x) <= number_order(c) && is_number(x) && is_number(c);
+}
+__device__ __forceinline__ bool f_neg(double x) { return f_lt(x, 0.0); }
 __device__ __forceinline__ double nonneg_min(double a, double b) { return fmin(a, b); }
-__device__ __forceinline__ bool f_gt(double x, double c) { return x > c; }
-__device__ __forceinline__ bool f_ge(double x, double c) { return x >= c; }
-__device__ __forceinline__ bool f_abs_lt(double x, double c) { return fabs(x) < c; }
-__device__ __forceinline__ bool f_is_zero(double x) { return x == 0.0; }
+__device__ __forceinline__ bool f_gt(double x, double c) { return f_lt(c, x); }
+__device__ __forceinline__ bool f_ge(double x, double c) { return f_le(c, x); }
+__device__ __forceinline__ bool f_abs_lt(double x, double c) { return f_lt(fabs(x), c); }
+__device__ __forceinline__ bool f_is_zero(double x) { return dmul_bits(x) << 1 == 0; }
 #else
 constexpr long long kMag = 0x7fffffffffffffffLL;
 __device__ __forceinline__ long long dbits(double x) { return static_cast<long long>(dmul_bits(x)); }
@@ -314,7 +342,7 @@ __device__ __forceinline__ double nonneg_min(double a, double b) {
 // two variables (the limiter); floats compare on the float pipe
 __device__ __forceinline__ bool f_vlt(double a, double b) {
 #if LULESH_EXACT
-    return a < b;
+    return f_lt(a, b);
 #else
     const long long ba = dbits(a), bb = dbits(b);
     const long long ka = ba ^ ((ba >> 63) & kMag), kb = bb ^ ((bb >> 63) & kMag);
@@ -410,9 +438,9 @@ __device__ __forceinline__ void face_normal(R nx[8], R ny[8], R nz[8], const R x
     const R bisX1 = (x[C] + x[B] - x[D] - x[A]);
     const R bisY1 = (y[C] + y[B] - y[D] - y[A]);
     const R bisZ1 = (z[C] + z[B] - z[D] - z[A]);
-    const R ax = (bisY0 * bisZ1 - bisZ0 * bisY1);
-    const R ay = (bisZ0 * bisX1 - bisX0 * bisZ1);
-    const R az = (bisX0 * bisY1 - bisY0 * bisX1);
+    const R ax = xmul(bisY0, bisZ1) - xmul(bisZ0, bisY1);
+    const R ay = xmul(bisZ0, bisX1) - xmul(bisX0, bisZ1);
+    const R az = xmul(bisX0, bisY1) - xmul(bisY0, bisX1);
     const int c[4] = {A, B, C, D};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -498,12 +526,12 @@ __device__ __forceinline__ void volu_der(R dvdx[8], R dvdy[8], R dvdz[8], const 
     const R x0 = x[P0], x1 = x[P1], x2 = x[P2], x3 = x[P3], x4 = x[P4], x5 = x[P5];
     const R y0 = y[P0], y1 = y[P1], y2 = y[P2], y3 = y[P3], y4 = y[P4], y5 = y[P5];
     const R z0 = z[P0], z1 = z[P1], z2 = z[P2], z3 = z[P3], z4 = z[P4], z5 = z[P5];
-    const R dx = (y1 + y2) * (z0 + z1) - (y0 + y1) * (z1 + z2) + (y0 + y4) * (z3 + z4) -
-                 (y3 + y4) * (z0 + z4) - (y2 + y5) * (z3 + z5) + (y3 + y5) * (z2 + z5);
-    const R dy = -(x1 + x2) * (z0 + z1) + (x0 + x1) * (z1 + z2) - (x0 + x4) * (z3 + z4) +
-                 (x3 + x4) * (z0 + z4) + (x2 + x5) * (z3 + z5) - (x3 + x5) * (z2 + z5);
-    const R dz = -(y1 + y2) * (x0 + x1) + (y0 + y1) * (x1 + x2) - (y0 + y4) * (x3 + x4) +
-                 (y3 + y4) * (x0 + x4) + (y2 + y5) * (x3 + x5) - (y3 + y5) * (x2 + x5);
+    const R dx = xmul(y1 + y2, z0 + z1) - xmul(y0 + y1, z1 + z2) + xmul(y0 + y4, z3 + z4) -
+                 xmul(y3 + y4, z0 + z4) - xmul(y2 + y5, z3 + z5) + xmul(y3 + y5, z2 + z5);
+    const R dy = -xmul(x1 + x2, z0 + z1) + xmul(x0 + x1, z1 + z2) - xmul(x0 + x4, z3 + z4) +
+                 xmul(x3 + x4, z0 + z4) + xmul(x2 + x5, z3 + z5) - xmul(x3 + x5, z2 + z5);
+    const R dz = -xmul(y1 + y2, x0 + x1) + xmul(y0 + y1, x1 + x2) - xmul(y0 + y4, x3 + x4) +
+                 xmul(y3 + y4, x0 + x4) + xmul(y2 + y5, x3 + x5) - xmul(y3 + y5, x2 + x5);
 #if LULESH_EXACT
     dvdx[K] = dx * twelfth;
     dvdy[K] = dy * twelfth;
@@ -667,7 +695,7 @@ __device__ __forceinline__ void hourgam_mode(R hg[8][4], const R x[8], const R y
     const R hx = hourmod<M>(x), hy = hourmod<M>(y), hz = hourmod<M>(z);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        hg[k][M] = R(gamma_sign(M, k)) - volinv * (dvdx[k] * hx + dvdy[k] * hy + dvdz[k] * hz);
+        hg[k][M] = R(gamma_sign(M, k)) - volinv * (xmul(dvdx[k], hx) + xmul(dvdy[k], hy) + xmul(dvdz[k], hz));
 }
 
 // volinv = 1 / (volo v); in the fast variants the volume derivatives come
@@ -707,12 +735,13 @@ __device__ __forceinline__ void fb_force_axis(const R hg[8][4], const R vel[8], 
     R h[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m)
-        h[m] = hg[0][m] * vel[0] + hg[1][m] * vel[1] + hg[2][m] * vel[2] + hg[3][m] * vel[3] +
-               hg[4][m] * vel[4] + hg[5][m] * vel[5] + hg[6][m] * vel[6] + hg[7][m] * vel[7];
+        h[m] = xmul(hg[0][m], vel[0]) + xmul(hg[1][m], vel[1]) + xmul(hg[2][m], vel[2]) + xmul(hg[3][m], vel[3]) +
+               xmul(hg[4][m], vel[4]) + xmul(hg[5][m], vel[5]) + xmul(hg[6][m], vel[6]) + xmul(hg[7][m], vel[7]);
 #if LULESH_EXACT
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        out[k] = coefficient * (hg[k][0] * h[0] + hg[k][1] * h[1] + hg[k][2] * h[2] + hg[k][3] * h[3]);
+        out[k] = coefficient * (xmul(hg[k][0], h[0]) + xmul(hg[k][1], h[1]) + xmul(hg[k][2], h[2]) +
+                                xmul(hg[k][3], h[3]));
 #else
     // fast variants: the coefficient scales the 4 mode amplitudes, not the 8 corners
 #pragma unroll
@@ -752,13 +781,13 @@ __device__ __forceinline__ R face_area(const R x[8], const R y[8], const R z[8])
     const R gx = (x[C] - x[A]) + (x[D] - x[B]);
     const R gy = (y[C] - y[A]) + (y[D] - y[B]);
     const R gz = (z[C] - z[A]) + (z[D] - z[B]);
-    return (fx * fx + fy * fy + fz * fz) * (gx * gx + gy * gy + gz * gz) -
-           (fx * gx + fy * gy + fz * gz) * (fx * gx + fy * gy + fz * gz);
+    const R fg = xmul(fx, gx) + xmul(fy, gy) + xmul(fz, gz);
+    return (xmul(fx, fx) + xmul(fy, fy) + xmul(fz, fz)) * (xmul(gx, gx) + xmul(gy, gy) + xmul(gz, gz)) - fg * fg;
 }
 
 template <class R>
 __device__ __forceinline__ R max_ref(R a, R cl) {
-    return (a < cl) ? cl : a;  // std::max(a, cl)
+    return f_lt(a, cl) ? cl : a;  // std::max(a, cl)
 }
 
 #if !LULESH_EXACT
@@ -817,61 +846,62 @@ __device__ __forceinline__ R max_face_area(const R x[8], const R y[8], const R z
 // Monotonic-Q gradients of CalcMonotonicQGradientsForElemsTask
 // (lulesh.cc:1341-1416). vol = volo * vnew. Outputs
 // g[0..2] = delv_xi, delv_eta, delv_zeta and g[3..5] = delx_xi, delx_eta, delx_zeta.
+// The reference's factors 0.25 of the differences are left to the end, where
+// there are fewer: powers of two commute with rounding.
 template <class R>
 __device__ __forceinline__ void q_gradients(const R x[8], const R y[8], const R z[8], const R xv[8],
                                             const R yv[8], const R zv[8], R vol, R g[6]) {
     const R ptiny = R(1.e-36);
-    const R q = R(0.25), mq = R(-0.25);
-    const R norm = rcp(vol + ptiny);
-    const R dxj = mq * ((x[0] + x[1] + x[5] + x[4]) - (x[3] + x[2] + x[6] + x[7]));
-    const R dyj = mq * ((y[0] + y[1] + y[5] + y[4]) - (y[3] + y[2] + y[6] + y[7]));
-    const R dzj = mq * ((z[0] + z[1] + z[5] + z[4]) - (z[3] + z[2] + z[6] + z[7]));
-    const R dxi = q * ((x[1] + x[2] + x[6] + x[5]) - (x[0] + x[3] + x[7] + x[4]));
-    const R dyi = q * ((y[1] + y[2] + y[6] + y[5]) - (y[0] + y[3] + y[7] + y[4]));
-    const R dzi = q * ((z[1] + z[2] + z[6] + z[5]) - (z[0] + z[3] + z[7] + z[4]));
-    const R dxk = q * ((x[4] + x[5] + x[6] + x[7]) - (x[0] + x[1] + x[2] + x[3]));
-    const R dyk = q * ((y[4] + y[5] + y[6] + y[7]) - (y[0] + y[1] + y[2] + y[3]));
-    const R dzk = q * ((z[4] + z[5] + z[6] + z[7]) - (z[0] + z[1] + z[2] + z[3]));
+    const R norm = rcp(vol + ptiny), pt = R(256.0) * ptiny, vol16 = R(16.0) * vol, scale = R(0.015625);
+    const R dxj = -((x[0] + x[1] + x[5] + x[4]) - (x[3] + x[2] + x[6] + x[7]));
+    const R dyj = -((y[0] + y[1] + y[5] + y[4]) - (y[3] + y[2] + y[6] + y[7]));
+    const R dzj = -((z[0] + z[1] + z[5] + z[4]) - (z[3] + z[2] + z[6] + z[7]));
+    const R dxi = (x[1] + x[2] + x[6] + x[5]) - (x[0] + x[3] + x[7] + x[4]);
+    const R dyi = (y[1] + y[2] + y[6] + y[5]) - (y[0] + y[3] + y[7] + y[4]);
+    const R dzi = (z[1] + z[2] + z[6] + z[5]) - (z[0] + z[3] + z[7] + z[4]);
+    const R dxk = (x[4] + x[5] + x[6] + x[7]) - (x[0] + x[1] + x[2] + x[3]);
+    const R dyk = (y[4] + y[5] + y[6] + y[7]) - (y[0] + y[1] + y[2] + y[3]);
+    const R dzk = (z[4] + z[5] + z[6] + z[7]) - (z[0] + z[1] + z[2] + z[3]);
     R ax, ay, az, dxv, dyv, dzv;
 
     // zeta: i cross j
-    ax = dyi * dzj - dzi * dyj;
-    ay = dzi * dxj - dxi * dzj;
-    az = dxi * dyj - dyi * dxj;
-    g[5] = div_sqrt(vol, ax * ax + ay * ay + az * az + ptiny);
+    ax = xmul(dyi, dzj) - xmul(dzi, dyj);
+    ay = xmul(dzi, dxj) - xmul(dxi, dzj);
+    az = xmul(dxi, dyj) - xmul(dyi, dxj);
+    g[5] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = q * ((xv[4] + xv[5] + xv[6] + xv[7]) - (xv[0] + xv[1] + xv[2] + xv[3]));
-    dyv = q * ((yv[4] + yv[5] + yv[6] + yv[7]) - (yv[0] + yv[1] + yv[2] + yv[3]));
-    dzv = q * ((zv[4] + zv[5] + zv[6] + zv[7]) - (zv[0] + zv[1] + zv[2] + zv[3]));
-    g[2] = ax * dxv + ay * dyv + az * dzv;
+    dxv = (xv[4] + xv[5] + xv[6] + xv[7]) - (xv[0] + xv[1] + xv[2] + xv[3]);
+    dyv = (yv[4] + yv[5] + yv[6] + yv[7]) - (yv[0] + yv[1] + yv[2] + yv[3]);
+    dzv = (zv[4] + zv[5] + zv[6] + zv[7]) - (zv[0] + zv[1] + zv[2] + zv[3]);
+    g[2] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
 
     // xi: j cross k
-    ax = dyj * dzk - dzj * dyk;
-    ay = dzj * dxk - dxj * dzk;
-    az = dxj * dyk - dyj * dxk;
-    g[3] = div_sqrt(vol, ax * ax + ay * ay + az * az + ptiny);
+    ax = xmul(dyj, dzk) - xmul(dzj, dyk);
+    ay = xmul(dzj, dxk) - xmul(dxj, dzk);
+    az = xmul(dxj, dyk) - xmul(dyj, dxk);
+    g[3] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = q * ((xv[1] + xv[2] + xv[6] + xv[5]) - (xv[0] + xv[3] + xv[7] + xv[4]));
-    dyv = q * ((yv[1] + yv[2] + yv[6] + yv[5]) - (yv[0] + yv[3] + yv[7] + yv[4]));
-    dzv = q * ((zv[1] + zv[2] + zv[6] + zv[5]) - (zv[0] + zv[3] + zv[7] + zv[4]));
-    g[0] = ax * dxv + ay * dyv + az * dzv;
+    dxv = (xv[1] + xv[2] + xv[6] + xv[5]) - (xv[0] + xv[3] + xv[7] + xv[4]);
+    dyv = (yv[1] + yv[2] + yv[6] + yv[5]) - (yv[0] + yv[3] + yv[7] + yv[4]);
+    dzv = (zv[1] + zv[2] + zv[6] + zv[5]) - (zv[0] + zv[3] + zv[7] + zv[4]);
+    g[0] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
 
     // eta: k cross i
-    ax = dyk * dzi - dzk * dyi;
-    ay = dzk * dxi - dxk * dzi;
-    az = dxk * dyi - dyk * dxi;
-    g[4] = div_sqrt(vol, ax * ax + ay * ay + az * az + ptiny);
+    ax = xmul(dyk, dzi) - xmul(dzk, dyi);
+    ay = xmul(dzk, dxi) - xmul(dxk, dzi);
+    az = xmul(dxk, dyi) - xmul(dyk, dxi);
+    g[4] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = mq * ((xv[0] + xv[1] + xv[5] + xv[4]) - (xv[3] + xv[2] + xv[6] + xv[7]));
-    dyv = mq * ((yv[0] + yv[1] + yv[5] + yv[4]) - (yv[3] + yv[2] + yv[6] + yv[7]));
-    dzv = mq * ((zv[0] + zv[1] + zv[5] + zv[4]) - (zv[3] + zv[2] + zv[6] + zv[7]));
-    g[1] = ax * dxv + ay * dyv + az * dzv;
+    dxv = -((xv[0] + xv[1] + xv[5] + xv[4]) - (xv[3] + xv[2] + xv[6] + xv[7]));
+    dyv = -((yv[0] + yv[1] + yv[5] + yv[4]) - (yv[3] + yv[2] + yv[6] + yv[7]));
+    dzv = -((zv[0] + zv[1] + zv[5] + zv[4]) - (zv[3] + zv[2] + zv[6] + zv[7]));
+    g[1] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
 }
 
 // Trace of the velocity gradient at the half-step geometry
@@ -883,12 +913,12 @@ __device__ __forceinline__ R vel_grad_trace(const R xh[8], const R yh[8], const 
     R b[3][4];
     const R detJ = shape_derivs(jacobian(xh, yh, zh), b);
     const R inv = rcp(detJ);
-    const R dxx = inv * (b[0][0] * (xv[0] - xv[6]) + b[0][1] * (xv[1] - xv[7]) +
-                         b[0][2] * (xv[2] - xv[4]) + b[0][3] * (xv[3] - xv[5]));
-    const R dyy = inv * (b[1][0] * (yv[0] - yv[6]) + b[1][1] * (yv[1] - yv[7]) +
-                         b[1][2] * (yv[2] - yv[4]) + b[1][3] * (yv[3] - yv[5]));
-    const R dzz = inv * (b[2][0] * (zv[0] - zv[6]) + b[2][1] * (zv[1] - zv[7]) +
-                         b[2][2] * (zv[2] - zv[4]) + b[2][3] * (zv[3] - zv[5]));
+    const R dxx = inv * (xmul(b[0][0], xv[0] - xv[6]) + xmul(b[0][1], xv[1] - xv[7]) +
+                         xmul(b[0][2], xv[2] - xv[4]) + xmul(b[0][3], xv[3] - xv[5]));
+    const R dyy = inv * (xmul(b[1][0], yv[0] - yv[6]) + xmul(b[1][1], yv[1] - yv[7]) +
+                         xmul(b[1][2], yv[2] - yv[4]) + xmul(b[1][3], yv[3] - yv[5]));
+    const R dzz = inv * (xmul(b[2][0], zv[0] - zv[6]) + xmul(b[2][1], zv[1] - zv[7]) +
+                         xmul(b[2][2], zv[2] - zv[4]) + xmul(b[2][3], zv[3] - zv[5]));
     return dxx + dyy + dzz;
 }
 
@@ -1093,7 +1123,7 @@ __device__ __forceinline__ double eos_pressure(double& bvc, double& pbvc, double
     const double cls = 2.0 / 3.0;
     bvc = cls * (comp + 1.0);
     pbvc = cls;
-    double nv = bvc * e;
+    double nv = xmul(bvc, e);
     if (f_abs_lt(nv, P.p_cut) || f_ge(vnewc, P.eosvmax)) nv = 0.0;
     if (f_lt(nv, P.pmin)) nv = P.pmin;
     return nv;
@@ -1175,17 +1205,17 @@ __device__ __forceinline__ EosState eos_body(const Mesh& m, int i, double vnewc,
             compHalf = 0.;
         }
         // predictor
-        e_new = e_old - 0.5 * delvc * (p_old + q_old) LULESH_PLUS_ZERO_WORK;
+        e_new = e_old - xmul(0.5 * delvc, p_old + q_old) LULESH_PLUS_ZERO_WORK;
         if (f_lt(e_new, P.emin)) e_new = P.emin;
         const double pHalf = eos_pressure(bvc, pbvc, e_new, compHalf, vnewc, P);
         const double vhalf = rcp(1. + compHalf);
         if (f_gt(delvc, 0.)) {
             q_new = 0.;
         } else {
-            const double ssc = ss_guard(over_rho<UNIT_RHO>((pbvc * e_new + vhalf * vhalf * bvc * pHalf), P));
-            q_new = (ssc * ql_old + qq_old);
+            const double ssc = ss_guard(over_rho<UNIT_RHO>((xmul(pbvc, e_new) + xmul(xmul(xmul(vhalf, vhalf), bvc), pHalf)), P));
+            q_new = (xmul(ssc, ql_old) + qq_old);
         }
-        e_new = e_new + 0.5 * delvc * (3.0 * (p_old + q_old) - 4.0 * (pHalf + q_new));
+        e_new = e_new + xmul(0.5 * delvc, 3.0 * (p_old + q_old) - 4.0 * (pHalf + q_new));
         e_new = e_new LULESH_PLUS_ZERO_WORK;
         if (f_abs_lt(e_new, P.e_cut)) e_new = 0.0;
         if (f_lt(e_new, P.emin)) e_new = P.emin;
@@ -1197,18 +1227,18 @@ __device__ __forceinline__ EosState eos_body(const Mesh& m, int i, double vnewc,
             if (f_gt(delvc, 0.)) {
                 q_tilde = 0.;
             } else {
-                const double ssc = ss_guard(over_rho<UNIT_RHO>((pbvc * e_new + vnewc * vnewc * bvc * p_new), P));
-                q_tilde = (ssc * ql_old + qq_old);
+                const double ssc = ss_guard(over_rho<UNIT_RHO>((xmul(pbvc, e_new) + xmul(xmul(xmul(vnewc, vnewc), bvc), p_new)), P));
+                q_tilde = (xmul(ssc, ql_old) + qq_old);
             }
             e_new = e_new -
-                    (7.0 * (p_old + q_old) - 8.0 * (pHalf + q_new) + (p_new + q_tilde)) * delvc * sixth;
+                    xmul(xmul(7.0 * (p_old + q_old) - 8.0 * (pHalf + q_new) + (p_new + q_tilde), delvc), sixth);
             if (f_abs_lt(e_new, P.e_cut)) e_new = 0.;
             if (f_lt(e_new, P.emin)) e_new = P.emin;
         }
         p_new = eos_pressure(bvc, pbvc, e_new, comp, vnewc, P);
         if (f_le(delvc, 0.)) {
-            const double ssc = ss_guard(over_rho<UNIT_RHO>((pbvc * e_new + vnewc * vnewc * bvc * p_new), P));
-            q_new = (ssc * ql_old + qq_old);
+            const double ssc = ss_guard(over_rho<UNIT_RHO>((xmul(pbvc, e_new) + xmul(xmul(xmul(vnewc, vnewc), bvc), p_new)), P));
+            q_new = (xmul(ssc, ql_old) + qq_old);
             if (f_abs_lt(q_new, P.q_cut)) q_new = 0.;
         }
     }

@@ -786,3 +786,74 @@ def test_time_step_bounds_of_many_elements(lulesh, precision, kind):
     # fast: dtf 2, its reciprocal root 2, the product 1; 1 / |vdov| 2, the product 1 (half ulps and numpy's own 2)
     np.testing.assert_allclose([dtc, dth], want, rtol=0 if precision == "fp64_exact" else 8 * 2.0 ** -53)
     dev.close()
+
+
+def _eos_plain(P, e0, p0, q0, ql, qq, v, delv):
+    """The reference's EOS passes (lulesh.cc:1692-1904), each operation rounded on its own."""
+    cls, work = 2.0 / 3.0, 0.5 * 0.0
+
+    def guard(x):
+        return np.where(x <= .1111111e-36, .3333333e-18, np.sqrt(np.maximum(x, 0.0)))
+
+    def pressure(comp, e):
+        bvc = cls * (comp + 1.0)
+        p = bvc * e
+        p = np.where((np.abs(p) < P.p_cut) | (v >= P.eosvmax), 0.0, p)
+        return bvc, np.where(p < P.pmin, P.pmin, p)
+
+    def least(e, cut=True):
+        e = np.where(np.abs(e) < P.e_cut, 0.0, e) if cut else e
+        return np.where(e < P.emin, P.emin, e)
+
+    comp, half = 1.0 / v - 1.0, 1.0 / (v - delv * .5) - 1.0
+    e = least(e0 - 0.5 * delv * (p0 + q0) + work, cut=False)
+    bvc, ph = pressure(half, e)
+    vhalf = 1.0 / (1.0 + half)
+    q = np.where(delv > 0.0, 0.0, guard(cls * e + vhalf * vhalf * bvc * ph) * ql + qq)
+    e = least(e + 0.5 * delv * (3.0 * (p0 + q0) - 4.0 * (ph + q)) + work)
+    bvc, p = pressure(comp, e)
+    qt = np.where(delv > 0.0, 0.0, guard(cls * e + v * v * bvc * p) * ql + qq)
+    e = least(e - (7.0 * (p0 + q0) - 8.0 * (ph + q) + (p + qt)) * delv * (1.0 / 6.0))
+    bvc, p = pressure(comp, e)
+    last = guard(cls * e + v * v * bvc * p) * ql + qq
+    q = np.where(delv <= 0.0, np.where(np.abs(last) < P.q_cut, 0.0, last), q)
+    return {"e": e, "p": p, "q": q, "ss": guard(cls * e + v * v * bvc * p)}
+
+
+@pytest.mark.parametrize("params", [{}, {"pmin": -0.0, "q_cut": 0.0}, {"emin": -0.0}, {"p_cut": 1e-310}],
+                         ids=lambda p: next(iter(p), "default"))
+def test_exact_compares_and_products(lulesh, params):
+    """The exact variant compares and multiplies in integers: over zeros of
+    both signs, subnormals, infinities, NaN and values at the cutoffs its EOS
+    gives the bits of plain double arithmetic."""
+    s = 12
+    rng = np.random.default_rng(11)
+    dom = lulesh.HostDomain(s, 11)
+    special = np.array([0.0, -0.0, 5e-324, -5e-324, 1e-310, 1e-7, -1e-7, np.nextafter(1e-7, 0), np.inf, -np.inf,
+                        np.nan, 1e300, -1e300, 1.0])
+    ne = s ** 3
+
+    def mixed(a):
+        return np.where(rng.uniform(size=ne) < 0.3, rng.choice(special, ne), a)
+
+    e, p, q = (mixed(rng.uniform(-1.0, 10.0, ne)) for _ in range(3))
+    delv = mixed(rng.uniform(-0.05, 0.05, ne))
+    v = rng.uniform(0.9, 1.1, ne)
+    dom.xd[:] = np.asarray(dom.x) * rng.uniform(-1.0, 1.0, dom.numNode)  # some close, some open
+    for k, x in params.items():
+        setattr(dom.view.params, k, x)
+    dev = lulesh.Device(dom, "fp64_exact")
+    dev.phase(lulesh.PHASE_KINEMATICS, 1e-7)
+    dev.download()
+    dom.vnew[:], dom.delv[:], dom.e[:], dom.p[:], dom.q[:] = v, delv, e, p, q
+    dev.upload(lulesh.F_KIN | lulesh.F_EPQ)
+    dev.phase(lulesh.PHASE_MATERIAL)
+    dev.download()
+    with np.errstate(all="ignore"):
+        want = _eos_plain(dom.view.params, e, p, q, np.asarray(dom.ql), np.asarray(dom.qq), v, delv)
+    for f, w in want.items():
+        got = np.asarray(getattr(dom, f))
+        np.testing.assert_array_equal(got, w, err_msg=f)
+        live = ~np.isnan(w)
+        np.testing.assert_array_equal(np.signbit(got)[live], np.signbit(w)[live], err_msg=f)
+    dev.close()

@@ -230,18 +230,20 @@ BatchLaunch shape(const lulesh_batch* b, int phase) {
 }
 
 // Tile size for the problems still running: the tuned size, halved (down to
-// 64) while the running problems' elements would give each resident block
-// of the widest phase fewer than 4 tiles. When the first problems of an
-// ensemble finish, the rest then still spread over every SM instead of a few
-// long tiles.
+// 128, a block's threads) while the running problems' elements would give each
+// resident block of the widest phase (in blocks of 128) fewer than 4 tiles.
+// When the first problems of an ensemble finish, the rest then still spread
+// over every SM instead of a few long tiles. us per cycle of 10 problems of
+// s=18-40: at least 64 a tile 343 double, 245 mixed; 128 251, 236; 256 318,
+// 358. 14 of 16-64: 2, 4, 8 tiles a block 830, 768, 797 double.
 int effective_tile(const lulesh_batch* b) {
     int64_t elems = 0;
     for (const Slot& sl : b->slots)
         if (sl.in_use && !sl.finished) elems += sl.numElem;
     int blocks = 1;
-    for (int p = 0; p < 4; ++p) blocks = std::max(blocks, shape(b, p).grid);
+    for (int p = 0; p < 4; ++p) blocks = std::max(blocks, shape(b, p).grid * shape(b, p).block / 128);
     int T = std::max(32, b->tuning.tile);
-    while (T > 64 && elems < int64_t(4) * blocks * T) T /= 2;
+    while (T > 128 && elems < int64_t(4) * blocks * T) T /= 2;
     return T;
 }
 
@@ -260,6 +262,17 @@ bool rebuild_tiles(lulesh_batch* b) {
     lulesh::RepClasses classes;
     for (const auto& kv : count) classes.push_back(make_int2(kv.first, kv.second));
     const int passes = classes.empty() ? 1 : lulesh::mat_passes_per_lane(classes, b->sms, b->precision);
+    // Material tiles: as many rounds of a block's warps as take half a warp's
+    // share of the phase (counted in passes, the Q terms as 3), so that the
+    // queue ends evenly whatever the class. In place of the other phases'
+    // tiles: 10 problems of s=18-40 244 -> 243 us double, 225 -> 182 mixed,
+    // 1500 -> 1313 exact; a quarter of the share is the same.
+    const BatchLaunch mat = shape(b, 3);
+    const int warps = mat.block / 32;
+    auto cost = [&](int rep) { return 3 + (rep + lulesh::lanes_for_rep(rep, passes) - 1) / lulesh::lanes_for_rep(rep, passes); };
+    double share = 0.0;
+    for (const int2& c : classes) share += double(c.y) * lulesh::lanes_for_rep(c.x, passes) / 32 * cost(c.x);
+    share /= double(mat.grid) * warps;
     for (int s = 0; s < int(b->slots.size()); ++s) {
         const Slot& sl = b->slots[s];
         if (!sl.in_use || sl.finished) continue;
@@ -270,10 +283,13 @@ bool rebuild_tiles(lulesh_batch* b) {
         int pos = 0;
         for (size_t c = 0; c < sl.repCount.size(); ++c) {
             const int end = pos + sl.repCount[c];
-            for (int t = pos; t < end; t += T) {
-                const int cnt = std::min(T, end - t);
+            const int lanes = lulesh::lanes_for_rep(sl.repValue[c], passes);
+            const int rounds = std::max(1, std::min(T / mat.block, int(share / (2 * cost(sl.repValue[c])))));
+            const int TM = rounds * warps * (32 / lanes);
+            for (int t = pos; t < end; t += TM) {
+                const int cnt = std::min(TM, end - t);
                 b->h_tiles[lulesh::TILES_MAT].push_back(
-                    {s, t, cnt, cnt * sl.repValue[c], lulesh::lanes_for_rep(sl.repValue[c], passes)});
+                    {s, t, cnt, cnt * sl.repValue[c], lanes});
             }
             pos = end;
         }
@@ -456,11 +472,14 @@ int lulesh_batch_create(int32_t precision, uint64_t pool_bytes, int32_t max_slot
         cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(unsigned), b->stream) != cudaSuccess ||
         cudaStreamSynchronize(b->stream) != cudaSuccess)
         return fail(LULESH_ECUDA);
-    // defaults until lulesh_batch_autotune: the single-problem kernels' shapes
-    const int blocks[4] = {128, 256, 128, 128};
+    // defaults until lulesh_batch_autotune: the single-problem kernels'
+    // shapes, but for smaller blocks of the phases whose queues end raggedly
+    // (14 problems of s=16-64, mixed: nodes of 256 530, of 128 524 us; material
+    // of 128 544, of 64 530, of 32 530)
+    const int blocks[4] = {128, 128, 128, 64};
     for (int p = 0; p < 4; ++p) {
         b->tuning.block[p] = blocks[p];
-        b->tuning.blocks_per_sm[p] = 8;
+        b->tuning.blocks_per_sm[p] = p == 1 || p == 3 ? 16 : 8;
         b->tuning.grab[p] = 1;
     }
     b->tuning.tile = 1024;

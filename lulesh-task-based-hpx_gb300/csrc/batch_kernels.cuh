@@ -17,9 +17,14 @@
 // its tiles are done, so that its cost-sorted queue stays dynamically
 // balanced (reserving ahead cost 4-6 % of a serving run).
 //
-// The bound asks ptxas for at least one resident block per SM: without the
-// minimum, its heuristic held the material phase to 64 registers with
-// spills inside the EOS loop (6 % slower batched cycles).
+// The bounds (kBatchBlocks, blocks of kBatchMaxBlock per SM by phase) keep the
+// phases near the occupancy of the single-problem kernels: inlined into the
+// tile loop the double forces and kinematics take 200 registers by
+// themselves, which leaves 8 warps per SM. us per cycle of 14 problems of
+// s=16-64, and of 10 of 18-40, with one block asked for and as given here:
+// double 943, 498 -> 768, 344, mixed 570, 260 -> 548, 245; exact 18-40 2163
+// -> 1459. More blocks cost spills (double material 3: 787, 4: 805; mixed
+// material 4: 590; double kinematics 3: 832).
 // Each instance keeps its own dt (DevTime), and the material phase lowers
 // the instance's Courant/hydro minima with atomic minima on the doubles' bit
 // patterns (exact for positive values, so the order does not matter).
@@ -34,8 +39,15 @@ __device__ __forceinline__ void atomic_min_pos(double* addr, double v) {
               static_cast<unsigned long long>(__double_as_longlong(v)));
 }
 
+#if LULESH_EXACT
+constexpr int kBatchBlocks[4] = {3, 4, 2, 3};  // forces, nodes, kinematics, material
+#elif LULESH_FLOAT_Q
+constexpr int kBatchBlocks[4] = {3, 4, 3, 3};
+#else
+constexpr int kBatchBlocks[4] = {2, 4, 2, 2};
+#endif
 template <int PHASE>
-__global__ void __launch_bounds__(kBatchMaxBlock, 1) kb_phase(BatchCtl c, int grab) {
+__global__ void __launch_bounds__(kBatchMaxBlock, kBatchBlocks[PHASE]) kb_phase(BatchCtl c, int grab) {
     constexpr int kind = (PHASE == 1) ? TILES_NODE : (PHASE == 3) ? TILES_MAT : TILES_ELEM;
     constexpr bool kPrefetch = PHASE != 3;
     __shared__ __align__(16) unsigned long long s_mesh[(sizeof(Mesh) + 7) / 8];

@@ -140,3 +140,21 @@ def test_mixed_ensemble_against_double(lulesh):
         assert err64 == errm == 0, sp
         assert cm == c64, sp
         assert abs(em - e64) / abs(e64) <= 1e-5, (sp, em, e64)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_exact"])
+@pytest.mark.parametrize("block,tile", [(None, None), (32, 32), (64, 4096), (256, 48), (256, 1024)])
+def test_tiles_cover_every_element_once(lulesh, precision, block, tile):
+    """The material tiles follow the block's warps, the lanes of a class and
+    its share of the phase, the others the tuned tile: with fewer and more
+    elements than a tile, leftover lanes and one or many rounds, every problem
+    equals its solo run."""
+    specs = [dict(s=1, nr=1), dict(s=2, nr=1), dict(s=5, cost=4), dict(s=17, nr=21), dict(s=26, nr=16, balance=2, cost=7)]
+    b = lulesh.Batch(precision, pool_bytes=256 << 20, max_slots=8)
+    if block:
+        b.set_tuning([block] * 4, [3] * 4, tile)
+    slots = [b.admit(**sp) for sp in specs]
+    b.run(7)
+    for slot, sp in zip(slots, specs):
+        alone, _ = _alone(lulesh, precision, its=7, **sp)
+        _assert_same(b.download(slot), alone)

@@ -360,8 +360,9 @@ int lulesh_dev_profile_end(lulesh_dev* dev, lulesh_profile* out);
  * lulesh_leapfrog_timeline_read returns the last call's marks: ms[k] is the
  * time of mark k after the call's first device work, stage[k] its kind
  * (LULESH_TL_*), index[k] its slab, node range or kinematics group, and
- * wall_ms the call's wall time on the host. Off (the default) it costs
- * nothing. */
+ * wall_ms the call's wall time on the host. A call with the timeline on takes
+ * every mesh in slabs; otherwise a small one (up to 200,000 elements) is taken
+ * whole. Off (the default) it costs nothing. */
 #define LULESH_TL_UPLOAD 1     /* a slab's inputs are on the device */
 #define LULESH_TL_FORCES 2     /* a slab's corner forces are formed */
 #define LULESH_TL_ENERGY_UP 3  /* the energy is on the device */

@@ -112,10 +112,15 @@ struct lulesh_dev {
 };
 
 // Slabs of lulesh_leapfrog (element planes per slab = s / slabs). At s=150
-// the drop-in ran at 3.79e8, 3.82e8 and 3.60e8 zone-cycles/s with 4, 8 and
-// 16 slabs: fewer leave more of the copies exposed, more add copy and
-// launch overhead.
+// a call of the drop-in takes 4.95, 4.91, 5.01 and 5.25 ms with 4, 6, 8 and 16
+// slabs: fewer leave more of the copies exposed, more add copy and launch
+// overhead.
 constexpr int kLeapfrogSlabs = 8;
+// Up to this many elements a call takes the mesh whole: a slab costs some 17
+// us of copies and launches, more than it hides of a small mesh's. us per
+// call with 1 and 8 slabs: s=8 80, 187; s=30 125, 216; s=45 241, 308; s=64
+// 566, 543; s=91 1407, 1225.
+constexpr int kLeapfrogWhole = 200000;
 
 // Slabs of a handle's problem: whole element planes of the cube of edge s
 // (one slab when the mesh is not an s^3 cube).
@@ -749,7 +754,8 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     //     going down behind it; each slab lowers its own dt minima (its own
     //     block partials and counter), folded on the host at the end.
     const int s = d->nx;
-    const int slabs = slab_count(s, m.numElem);
+    // the timeline shows the pipeline, so a small mesh too is cut for it
+    const int slabs = d->tl_on || m.numElem > kLeapfrogWhole ? slab_count(s, m.numElem) : 1;
     const bool cube = slabs > 1 || (s >= 1 && int64_t(s) * s * s == int64_t(m.numElem));
     const int64_t plane_n = cube ? int64_t(s + 1) * (s + 1) : m.numNode;
     const int64_t plane_e = cube ? int64_t(s) * s : m.numElem;
@@ -893,13 +899,14 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     if (slabs > 1) ms.matOrder = d->matOrderSlab;
     int part = 0;  // first block partial of the slab
     for (int sl = 0; sl < slabs; ++sl) {
-        // no grid-stride: blocks schedule dynamically, the slab's most
-        // expensive elements first (repeat-count order within a slab)
+        // slabs without a grid stride: blocks schedule dynamically, the
+        // slab's most expensive elements first (repeat-count order within it)
         cudaStream_t cs = (sl & 1) ? d->stream2 : d->stream;
         ms.partials = m.partials + part;
         ms.result = d->slab_result + sl;
-        part += d->mat_slab[sl].grid;
-        d->launches += d->L.material(ms, d->mat_slab[sl], cs);
+        const MatPlan& plan = slabs > 1 ? d->mat_slab[sl] : d->mat;
+        part += plan.grid;
+        d->launches += d->L.material(ms, plan, cs);
         if (int st = elem_down(out_mat, e_lo[sl], e_hi[sl], d->ev_mat[sl], cs, lulesh::kKernelCopyBytes, LULESH_TL_MAT, sl)) return st;
     }
     CK(cudaGetLastError());
@@ -1146,17 +1153,18 @@ int validate_view(const lulesh_domain_view* v) { return check_view(v); }
 
 // The time of a material phase whose lanes run at most k passes each is the
 // longest lane's chain plus the warps' work over the 4 quarters of each SM (a
-// warp's passes and, for the Q terms and the save, `rest` more). Fitted to
-// 1..20 passes per lane at s=8..120, r=16 (mean error 5 %): a chain costs
-// 0.96 us a pass and the work 0.66 (fast double), 4.2 and 4.0 (exact), 2.7
-// and 1.2 (mixed). Few elements leave the quarters idle, so more lanes per
-// element win (20 passes in one lane against the choice: s=8 37 -> 16 us, s=30
-// 40 -> 23, exact s=45 162 -> 137, mixed s=45 86 -> 51); many keep them busy,
-// and spreading an element then only repeats its Q terms (fast double s=91:
-// 188 us with one lane, 211 with 4). A split has to save a tenth.
+// warp's passes and, for the Q terms and the save, `rest` more), the chain in
+// units of the work of a pass. Fitted to 1..20 passes per lane at s=8..120,
+// r=16, where the choice takes 1.011 (fast double), 1.018 (exact) and 1.000
+// (mixed) times the best. Few elements leave the quarters idle, so more lanes
+// per element win (20 passes in one lane against the choice: s=8 33 -> 14 us,
+// s=30 35 -> 20, exact s=45 182 -> 106, mixed s=45 74 -> 39); many keep them
+// busy, and spreading an element then only repeats its Q terms (fast double
+// s=91: 169 us with one lane, 193 with 4; mixed 192, 271). A split has to save
+// a tenth.
 int mat_passes_per_lane(const RepClasses& classes, int sms, int precision) {
-    const double chain_cost = precision == LULESH_FP64 ? 1.45 : precision == LULESH_MIXED ? 2.2 : 1.05;
-    const double rest = precision == LULESH_FP64 ? 2.5 : precision == LULESH_MIXED ? 0.5 : 1.0;
+    const double chain_cost = precision == LULESH_FP64 ? 0.7 : precision == LULESH_MIXED ? 0.9 : 1.9;
+    const double rest = precision == LULESH_MIXED ? 0.5 : 1.5;
     int top = 1;
     for (const int2& c : classes) top = std::max(top, c.x);
     int best = top;

@@ -857,3 +857,24 @@ def test_exact_compares_and_products(lulesh, params):
         live = ~np.isnan(w)
         np.testing.assert_array_equal(np.signbit(got)[live], np.signbit(w)[live], err_msg=f)
     dev.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64_exact", "fp64", "mixed"])
+@pytest.mark.parametrize("s", [1, 2, 7, 31, 58, 59])
+def test_dropin_slabs_equal_the_step(lulesh, precision, s):
+    """The drop-in call takes a small mesh whole and cuts a larger one into
+    slabs: on both sides of the choice its cycles are the step's, bit for
+    bit."""
+    a, b = lulesh.HostDomain(s, 11), lulesh.HostDomain(s, 11)
+    dev_a, dev_b = lulesh.Device(a, precision), lulesh.Device(b, precision)
+    a.pin()
+    n = dev_b.run(3)  # s=1 and s=2 reach the stoptime first
+    dev_b.download()
+    for _ in range(n):
+        a.time_increment()
+        dev_a.leapfrog()
+    for f in ("x", "y", "z", "xd", "yd", "zd", "e", "p", "q", "v", "ss", "ql", "qq", "vdov", "arealg", "fx"):
+        np.testing.assert_array_equal(getattr(a, f), getattr(b, f), err_msg=f)
+    assert (a.time_state.dtcourant, a.time_state.dthydro) == (b.time_state.dtcourant, b.time_state.dthydro)
+    dev_a.close()
+    dev_b.close()

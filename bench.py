@@ -26,7 +26,7 @@ ours (default) prints one JSON line:
   serving        the continuous-batching loop on Poisson arrivals: p50/p99
                  time to solution and zone-cycles/s
   roofline       dominant kernel vs the measured HBM copy bandwidth, plus its
-                 FP64-pipe roof (the bound that actually applies)
+                 share of the FP64-pipe rate
   fom            the reference's report figures for value (and mixed):
                  grind time in us per zone-cycle and FOM = 1000 / grind
   cpu_baseline   the CPU oracle (a bit-exact restatement of the reference's
@@ -76,28 +76,26 @@ BYTES_PER_UNIT = {
     "mixed": {"forces": 224, "nodes": 236, "kinematics": 160, "material": 160},
 }
 STEP_BYTES_PER_ZONE_CYCLE = {"fp64": 1020, "mixed": 780}
-# What this implementation's layout moves on top of that: the double path's
-# resident loop passes 48 doubles of element geometry per element from
-# kinematics (written) to the next force phase (read instead of the node
-# positions), and the mixed path reads float-pair node mirrors.
+# What this implementation's layout moves: the corner lists and the material
+# order besides, and in the mixed path float-pair node mirrors.
 LAYOUT_BYTES_PER_UNIT = {
-    "fp64": {"forces": 680, "nodes": 381, "kinematics": 568, "material": 204},
+    "fp64": {"forces": 320, "nodes": 381, "kinematics": 184, "material": 204},
     "mixed": {"forces": 224, "nodes": 333, "kinematics": 184, "material": 180},
 }
 # DRAM bytes (read + write) and FP64-pipe instructions (thread level:
-# sm__inst_executed_pipe_fp64 x 32) per unit, measured by ncu on this
-# workload (s=150 r=21, the third cycle); every array a kernel streams is
+# sm__inst_executed_pipe_fp64 x 32) per unit, measured by ncu on the same
+# problem at s=120 r=21 (the third cycle); every array a kernel streams is
 # larger than L2. The material kernel's count depends on the state (EOS
 # passes, compressing elements); these are early cycles of the run. The FP64
-# pipe carries only part of the double arithmetic: the fast kernels run many
-# of their multiplies on the integer pipes (dmul_ipipe).
+# pipe carries only a small part of the double path's arithmetic: its element
+# kernels work in block fixed point on the integer pipes.
 TRAFFIC_PER_UNIT = {
-    "fp64": {"forces": 672, "nodes": 368, "kinematics": 563, "material": 230},
-    "mixed": {"forces": 215, "nodes": 315, "kinematics": 178, "material": 199},
+    "fp64": {"forces": 295, "nodes": 355, "kinematics": 169, "material": 210},
+    "mixed": {"forces": 204, "nodes": 298, "kinematics": 169, "material": 177},
 }
 FP64_INSTR_PER_UNIT = {
-    "fp64": {"forces": 449.0, "nodes": 32.7, "kinematics": 320.0, "material": 136.1},
-    "mixed": {"forces": 8.0, "nodes": 24.0, "kinematics": 76.0, "material": 115.1},
+    "fp64": {"forces": 66.0, "nodes": 29.7, "kinematics": 78.0, "material": 26.4},
+    "mixed": {"forces": 7.0, "nodes": 12.0, "kinematics": 71.0, "material": 83.7},
 }
 # Double-precision operations per unit of the reference's formulation (adds,
 # multiplies, divides, square and cube roots each counted once), from
@@ -266,13 +264,13 @@ def roofline(prof: dict, precision: str, ne: int, nn: int, rep_avg: float,
         peak_rate = fp64_peak * 1e12 / 2  # DFMA thread instructions per second
         fp64_pipe = {"achieved_ginst_s": round(rate / 1e9, 1), "peak_ginst_s": round(peak_rate / 1e9, 1),
                      "frac": round(rate / peak_rate, 4), "instr_per_unit": ipu,
-                     "note": "FP64-pipe instructions per unit (ncu, this workload) x units / launch time; peak = "
+                     "note": "FP64-pipe instructions per unit (ncu, s=120 r=21) x units / launch time; peak = "
                              f"DFMA issue rate, {fp64_kind} (lulesh_probe_pipe_rates)"}
     return {
         "bound": "hbm", "kernel": dom, "achieved": round(achieved, 1), "peak": peak,
         "unit": "GB/s", "frac": sig4(achieved / peak),
         "traffic": tpu * units if tpu else None,
-        "traffic_note": "ncu dram bytes per unit on this workload x units per launch" if tpu else None,
+        "traffic_note": "ncu dram bytes per unit at s=120 r=21 x units per launch" if tpu else None,
         "peak_kind": f"{kind} ({'MEASURED_PEAKS.json hbm_gbs' if kind == 'measured' else 'recipe fallback'})",
         "bytes_per_launch": bytes_launch, "bytes_per_unit": BYTES_PER_UNIT[precision][dom],
         "avg_launch_ms": round(km[dom] / cyc, 4),

@@ -507,11 +507,12 @@ int build_graph(lulesh_dev* d, int which) {
 }
 
 // Material blocks per SM of the grid-stride launch (elements in repeat-count
-// order, so the grid's first blocks hold the long chains). At s=150 exact: 8;
-// mixed: 6, 8, 12 per SM and one thread per element gave 0.92, 0.98, 0.95,
-// 1.08 ms; fast double (6 resident): 6 and 24 gave 0.71 and 0.66.
+// order, so the grid's first blocks hold the long chains). Exact: 8. Fast
+// double (6 resident): 24 take 0.93 of the time of 6. Mixed (8 resident), s=120:
+// 24 0.358 ms, 8 0.366; few more than the resident ones leave a short last
+// wave (6 resident: 6, 8, 12, 24 gave 0.365, 0.449, 0.388, 0.363).
 int mat_blocks_per_sm(int precision) {
-    return precision == LULESH_FP64 ? 24 : precision == LULESH_MIXED ? 6 : 8;
+    return precision == LULESH_FP64_EXACT ? 8 : 24;
 }
 
 // A handle for ne elements and nn nodes: the arena carved, the stream and

@@ -451,9 +451,9 @@ __global__ void __launch_bounds__(kKinBlock, kKinBlocks) k_kinematics(Mesh m, do
 // Elements visited in repeat-count order so a warp's lanes run the same
 // number of EOS passes; the dt minima end in a last-block reduction. Exact
 // variant: 8 blocks of 128 per SM (64 registers), the passes being a chain of
-// dependent FP64 operations. Fast variant: 6 (80 registers): its integer
-// passes are bound by the ALU pipe, and more blocks spill (s=150: 0.69 ms
-// with 8, 0.66 with 6, 0.71 with 5).
+// dependent operations (s=60: 0.266 ms, 7 and 6 blocks 0.286 and 0.295). Fast
+// variant: 6 (80 registers): its integer passes are bound by the ALU pipe, and
+// more blocks spill (s=150: 0.616, 0.610, 0.619, 0.623 ms with 5 to 8).
 constexpr int kMatBlocks = LULESH_EXACT ? 8 : 6;
 // SPREAD: some class has several lanes per element (MatPlan).
 template <bool SPREAD>
@@ -478,10 +478,11 @@ __global__ void __launch_bounds__(kMatBlock, kMatBlocks) k_material(Mesh m, cons
 }
 
 // Up to this many elements the forces' axes, and the kinematics' parts, go to
-// threads of their own: forces s=8 16.7 -> 10.5 us, s=16 16.6 -> 12.5, s=24
-// (13,824) the same, s=30 20.7 -> 22.8; kinematics s=8 14.3 -> 11.9, s=30
-// (27,000) 18.4 -> 16.4, s=34 20.6 -> 22.5.
-constexpr int kSplitElems = LULESH_EXACT ? 0 : 12000, kSplitKinElems = LULESH_EXACT ? 0 : 30000;
+// threads of their own: forces s=12 14.7 -> 10.5 us, s=20 14.7 -> 12.5, s=27
+// (19,683) 17.7 -> 16.2, s=30 the same, s=34 20.8 -> 22.8; kinematics s=12
+// 14.3 -> 11.9, s=27 16.4 -> 15.3, s=30 (27,000) 16.4 -> 16.2, s=37 18.4 ->
+// 20.4.
+constexpr int kSplitElems = LULESH_EXACT ? 0 : 20000, kSplitKinElems = LULESH_EXACT ? 0 : 30000;
 
 int launch_forces_range(const Mesh& m, int first, int end, cudaStream_t s) {
     const int n = end - first, blocks = blocks_for(n, kForceBlock);

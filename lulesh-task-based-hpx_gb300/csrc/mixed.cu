@@ -196,9 +196,10 @@ __global__ void __launch_bounds__(kNodeBlock) k_nodes(Mesh m, double dt) {
     if (n < m.numNode) nodes_node(m, n, dt);
 }
 
-// all elements, or (RANGED) elements [first, end)
+// all elements, or (RANGED) elements [first, end). s=120: 0.237 ms with 4
+// blocks per SM, 0.238 with 5, 0.283 with 6, 0.246 at the compiler's choice.
 template <bool RANGED>
-__global__ void __launch_bounds__(kKinBlock) k_kinematics(Mesh m, double dt, int first, int end) {
+__global__ void __launch_bounds__(kKinBlock, 4) k_kinematics(Mesh m, double dt, int first, int end) {
     if (m.dtime) {
         if (!m.dtime->active) return;
         dt = m.dtime->deltatime;
@@ -207,9 +208,11 @@ __global__ void __launch_bounds__(kKinBlock) k_kinematics(Mesh m, double dt, int
     if (i < (RANGED ? end : m.numElem)) kinematics_elem(m, i, dt);
 }
 
-// SPREAD: some class has several lanes per element (MatPlan).
+// SPREAD: some class has several lanes per element (MatPlan). 8 blocks per SM
+// (64 registers), with 24 launched: s=120 0.358 ms, 7 blocks 0.360, at the
+// compiler's 72 registers 0.363.
 template <bool SPREAD>
-__global__ void __launch_bounds__(kMatBlock) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
+__global__ void __launch_bounds__(kMatBlock, 8) k_material(Mesh m, const __grid_constant__ MatPlan plan) {
     if (m.dtime && !m.dtime->active) return;
     DtMin<true> dt;
     if (SPREAD) {

@@ -353,10 +353,10 @@ def test_pinned_and_pageable_copies_agree(lulesh, s, precision):
         dev.close()
 
 
-@pytest.mark.parametrize("s", [8, 22, 23, 31, 32])
+@pytest.mark.parametrize("s", [8, 27, 28, 31, 32])
 def test_split_kernels_equal_whole_ones(lulesh, s):
     """Few elements give each axis of the forces and each part of the
-    kinematics a thread of its own (up to 12,000 and 30,000 elements: s=22 and
+    kinematics a thread of its own (up to 20,000 and 30,000 elements: s=27 and
     s=31 are the last). The drop-in call's slabs are below those sizes where
     the whole mesh is not: same bits, with some elements outside the fixed
     point's range (a flat and a fast one)."""

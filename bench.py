@@ -105,7 +105,7 @@ FP64_INSTR_PER_UNIT = {
 # many of these operations.
 FLOPS_PER_UNIT = {"forces": 1809, "nodes": 63, "kinematics": 864, "material_base": 69,
                   "material_per_rep": 68}
-# Measured on a GB300 of this machine (DFMA throughput probe): 597 G FMA/s.
+# Measured on a GB300 (DFMA throughput probe): 597 G FMA/s.
 FP64_PEAK_TFLOPS = 1.194
 HBM_FALLBACK_GBS = 6800.0
 

@@ -7,7 +7,7 @@
 // 32-bit integer multiply-adds, shifts and adds: the same bits as the FP64
 // pipe's multiply (a NaN result may carry another NaN payload), so a kernel
 // can move some of its multiplies there and run them beside the FP64 pipe's
-// adds and multiply-adds. Measured on this machine's GB300: the FP64 pipe
+// adds and multiply-adds. Measured on a GB300: the FP64 pipe
 // 5.0e11 multiplies/s, the integer form 4.8e11/s, both together 7.9e11/s;
 // a 3x3 cofactor kernel with the first product of each cofactor on the
 // integer pipes ran 1.37x faster.

@@ -1,5 +1,5 @@
 // Double-precision add on the integer pipes, for the measurement probes only
-// (liblulesh_probe.so): no step kernel uses it. Measured on this machine's
+// (liblulesh_probe.so): no step kernel uses it. Measured on a
 // GB300 it is exact (the FP64 pipe's bits) but slow: 2.4e11 adds/s alone,
 // 4.7e11/s with half the chains on each pipe, below the FP64 pipe's 5.3e11/s
 // alone, because its alignment, normalisation and rounding take several

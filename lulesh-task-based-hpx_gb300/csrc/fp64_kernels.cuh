@@ -5,9 +5,10 @@
 //   fp64_exact.cu  LULESH_VARIANT=fp64x, LULESH_EXACT=1, nvcc --fmad=false
 // With the reference's operand order kept in step_math.cuh, the exact
 // variant rounds every operation as the reference does and matches the CPU
-// oracle bit for bit (the oracle then uses the same portable cube root); the
-// fast variant lets nvcc fuse multiply-adds, which moves results by a few
-// ulps and saves FP64-pipe instructions.
+// oracle bit for bit (the oracle then uses the same portable cube root). The
+// fast variant works in block fixed point on the integer pipes
+// (block_fixed.cuh, eos_fixed.cuh), with double forms beside it for what does
+// not fit.
 //
 // One cycle = four phases, each a per-element (or per-node) device function
 // used both by the single-problem kernels below and by the batched
@@ -24,14 +25,6 @@
 
 namespace lulesh {
 namespace LULESH_VARIANT {
-
-__device__ __forceinline__ double cube_root(double x) {
-#if LULESH_EXACT
-    return cbrt_portable(x);
-#else
-    return cbrt(x);
-#endif
-}
 
 #if LULESH_EXACT
 // Stress and hourglass corner forces of element i, stored separately
@@ -74,7 +67,7 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
         hourgam_all(hg, x, y, z, dvdx, dvdy, dvdz, rcp(determ));
     }
     const double coefficient =
-        -m.prm.hgcoef * 0.01 * LD(m.ss + i) * LD(m.elemMass + i) / cube_root(determ);
+        -m.prm.hgcoef * 0.01 * LD(m.ss + i) * LD(m.elemMass + i) / cbrt_portable(determ);
     double vel[8], f[8];
     double* outs[3] = {m.fhx, m.fhy, m.fhz};
     const double* vels[3] = {m.xd, m.yd, m.zd};

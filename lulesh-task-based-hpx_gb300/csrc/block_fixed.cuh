@@ -48,6 +48,7 @@ namespace bf {
 constexpr int kLow = 29;         // bits of the low limb
 constexpr int kUnit = 2 * kLow;  // a product's value is in units of 2^kUnit
 constexpr int kBias = 1019;      // + width: exponent field of the largest value whose fix8 unit is 1
+constexpr int kLeast = 64;       // exponent field of the largest value of a fix8 block that is not zero, at least
 
 struct Limb {
     int32_t h, l;
@@ -65,7 +66,7 @@ LULESH_BF int64_t bits_of(double x) { return __double_as_longlong(x); }
 LULESH_BF int64_t tested_bits(double x) { return static_cast<int64_t>(dmul_bits(x)); }
 LULESH_BF double of_bits(int64_t b) { return __longlong_as_double(b); }
 LULESH_BF int32_t high_word(double x) { return int32_t(bits_of(x) >> 32); }
-// x times 2^k through the exponent field (x normal, or 0 with k < 1000: a tiny number)
+// x times 2^k through the exponent field (x normal; of 0 and subnormals up to 2^(k - 1022))
 LULESH_BF double up_exponent(double x, int k) { return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x)); }
 LULESH_BF int64_t round_to_int(double x) { return __double2ll_rn(x); }
 LULESH_BF double to_double(int64_t v) { return __ll2double_rn(v); }
@@ -153,17 +154,23 @@ LULESH_BF int64_t down(int64_t v, int s) { return v >> s; }
 LULESH_BF int clamp63(int s) { return s < 63 ? s : 63; }
 
 // 8 doubles as integers up to 2^(WIDTH - 3), so that their signed sums stay
-// below 2^WIDTH, times 2^unit. False where they do not fit. A block of zeros
-// (or of values below 2^-1042) is all zero.
+// below 2^WIDTH, times 2^unit. False where they do not fit, as where all are
+// below 2^-959 but not all zero. CVT: a block of zeros, of either sign, is all
+// zero. Else its values are +-2^(WIDTH - 4) by their signs, in a unit below
+// kUnitMin: the callers send it to their double path unless all sums cancel.
 template <int WIDTH, bool CVT>
 LULESH_BF bool fix8(const double v[8], int64_t q[8], int& unit) {
-    int32_t top = 0;
+    int32_t top = 0, low = 0;
     LULESH_UNROLL
     for (int k = 0; k < 8; ++k) {
         const int32_t m = high_word(v[k]) & 0x7fffffff;
         top = m > top ? m : top;
+        low |= int32_t(bits_of(v[k]));
     }
     const int e = top >> 20;
+    // all that fit but zeros have e >= kLeast; the exponent of these then
+    // becomes that of 2^-11 or less
+    const int up = kBias + WIDTH - (e > kLeast ? e : kLeast);
     unit = e - (kBias + WIDTH);
     // CVT: by the FP64 pipe's conversion, 62 cycles. Else the significand is
     // shifted into place by 15 integer instructions. The kernels take what
@@ -174,7 +181,7 @@ LULESH_BF bool fix8(const double v[8], int64_t q[8], int& unit) {
     LULESH_UNROLL
     for (int k = 0; k < 8; ++k) {
         if (CVT) {
-            q[k] = round_to_int(up_exponent(v[k], kBias + WIDTH - e));
+            q[k] = round_to_int(up_exponent(v[k], up));
             continue;
         }
         const int64_t b = bits_of(v[k]);
@@ -183,7 +190,7 @@ LULESH_BF bool fix8(const double v[8], int64_t q[8], int& unit) {
         const int64_t a = int64_t(m >> clamp63(n)), s = b >> 63;
         q[k] = (a ^ s) - s;
     }
-    return top == 0 || (e >= 64 && e <= kBias + WIDTH);
+    return (CVT ? top | low : top) == 0 || (e >= kLeast && e <= kBias + WIDTH);
 }
 
 // A normal double as limbs (below 2^58) and unit; false for 0, subnormals,
@@ -380,7 +387,7 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
     int64_t q[8], v[3], amp[4];
     int unit;
     bool ok = fix8<kUnit - 1, true>(vel, q, unit);
-    const bool still = unit == -(kBias + kUnit - 1);  // all zero
+    const bool still = unit == -(kBias + kUnit - 1);  // all zero, or none of it fits
     walsh(q, v, amp);
     Top m;
     m.add(v[0], v[1]);
@@ -501,6 +508,7 @@ LULESH_BF bool force_axis(const ForceGeo& o, const ForceScale& f, const int64_t 
     walsh_corners(x, h, q);
     LULESH_UNROLL
     for (int k = 0; k < 8; ++k) out[k] = scaled(q[k], u + 2);
+    // a unit by kNone: both parts are zero, and so is every q[k]
     return ok && (u < kNone / 2 || (u > -1000 && u < 950));
 }
 

@@ -320,6 +320,40 @@ def test_force_and_kinematics_ranges(lulesh, oracle_mod, s, kind):
     dev.close()
 
 
+@pytest.mark.parametrize("precision", ["fp64_exact", "fp64", "mixed"])
+@pytest.mark.parametrize("s", [3, 28])
+def test_still_mesh_of_signed_zeros(lulesh, precision, s):
+    """Velocities that are zeros of both signs (a masked or mirrored field)
+    are rest: the corner forces of cold elements, whose sound speed is the
+    cutoff's and not zero, are zeros, the others those of a mesh of +0, and so
+    is everything a cycle makes of them (axes of an element in threads of
+    their own, and in one)."""
+    rng = np.random.default_rng(17)
+    a, b = lulesh.HostDomain(s, 11), lulesh.HostDomain(s, 11)
+    cold = rng.uniform(size=s ** 3) < 0.7
+    for d in (a, b):
+        d.e[:] = 0.0
+        d.p[:] = np.where(cold, 0.0, 3.0)
+        d.ss[:] = .3333333e-18
+    for f in ("xd", "yd", "zd"):
+        getattr(b, f)[:] = np.where(rng.integers(0, 2, b.numNode) == 1, -0.0, 0.0)
+    assert np.signbit(b.xd).any() and not np.signbit(a.xd).any()
+    devs = [lulesh.Device(d, precision) for d in (a, b)]
+    for dev in devs:
+        dev.phase(lulesh.PHASE_FORCES, 1e-7)
+    for fa, fb in zip(*(dev.corner_forces() for dev in devs)):
+        np.testing.assert_array_equal(fa, fb)
+        assert not fb.reshape(-1, 8)[cold].any()
+        assert fb.reshape(-1, 8)[~cold].any()
+    for dev, d in zip(devs, (a, b)):
+        d.time_state.deltatime = 1e-7
+        dev.leapfrog()
+    for f in NODE + ELEM:
+        np.testing.assert_array_equal(getattr(a, f), getattr(b, f), err_msg=f)
+    for dev in devs:
+        dev.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("s", [1, 2, 3, 7, 11, 16, 30, 51, 52])
 def test_pinned_and_pageable_copies_agree(lulesh, s, precision):

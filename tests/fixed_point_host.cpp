@@ -1,7 +1,7 @@
-// Host build of the block fixed point (block_fixed.cuh): the integer
-// arithmetic of the double path's kernels, element by element, for
+// Host build of the block fixed point (block_fixed.cuh, eos_fixed.cuh): the
+// integer arithmetic of the double path's kernels, element by element, for
 // test_fixed_point.py.
-#include "block_fixed.cuh"
+#include "eos_fixed.cuh"
 
 using namespace lulesh::bf;
 
@@ -26,6 +26,20 @@ void host_forces(int n, const double* x, const double* vel, const double* sc, co
             const bool fit = force_axis(g, f, col, g.unit[a], vel + 24 * i + 8 * a, out + 24 * i + 8 * a);
             fits[3 * i + a] = ok && fit;
         }
+    }
+}
+
+// One EOS evaluation of n elements: in[k] = e, p, q, ql, qq, delv, v and
+// out[k] = e, p, q, ss, each of n values; the cutoffs of e and q are 1e-7.
+// fits[n]: the element does not need the double form.
+void host_eos(int n, const double* in, double p_cut, double* out, int* fits) {
+    const EosCuts cuts = eos_cuts(1e-7, p_cut, 1e-7, 0.0, -1e15, 1.0);
+    auto at = [&](int k, int i) { return in[size_t(k) * n + i]; };
+    for (int i = 0; i < n; ++i) {
+        double* o = out + i;
+        fits[i] = cuts.ok && eos_pass(at(0, i), at(1, i), at(2, i), at(3, i), at(4, i), at(5, i), at(6, i), cuts, o[0],
+                                      o[n], o[2 * size_t(n)], o[3 * size_t(n)]);
+        if (at(5, i) <= 0.0 && fabs(o[2 * size_t(n)]) < 1e-7) o[2 * size_t(n)] = 0.0;
     }
 }
 

@@ -1,4 +1,4 @@
-"""The double path's integer arithmetic (block_fixed.cuh) in its host build,
+"""The double path's integer arithmetic (block_fixed.cuh, eos_fixed.cuh) in its host build,
 element by element: the same integers as on the GPU, without one."""
 from __future__ import annotations
 
@@ -21,6 +21,7 @@ def host(tmp_path_factory):
                     str(ROOT / "tests" / "fixed_point_host.cpp"), "-o", str(lib)], check=True)
     lib = C.CDLL(str(lib))
     lib.host_forces.argtypes = [C.c_int] + [DOUBLES] * 6 + [INTS]
+    lib.host_eos.argtypes = [C.c_int, DOUBLES, C.c_double, DOUBLES, INTS]
     return lib
 
 
@@ -60,3 +61,84 @@ def test_forces_of_still_corners(host, coef, press):
         slow = np.zeros((n, 3, 8))
         slow[:, :, 5] = tiny
         assert not _forces(host, x, slow, coef, press)[1].any()
+
+
+def eos_reference(kind, e0, p0, q0, ql, qq, delv, v, p_cut):
+    """One EOS evaluation (lulesh.cc:1692-1871, with 2/3 / v for the
+    reference's 2/3 (comp + 1)) in the arithmetic of numpy type `kind`."""
+    e0, p0, q0, ql, qq, delv, v = (np.asarray(a, kind) for a in (e0, p0, q0, ql, qq, delv, v))
+    cls, half = kind(2) / kind(3), delv / 2
+
+    def pressure(bvc, e):
+        return np.where(bvc * e < p_cut, kind(0), bvc * e)
+
+    def viscosity(e, vol, p):
+        ss2 = cls * (e + vol * p)
+        ss = np.where(ss2 <= .1111111e-36, kind(.3333333e-18), np.sqrt(np.maximum(ss2, kind(0))))
+        return np.where(delv > 0, kind(0), ss * ql + qq), ss
+
+    def cut(e):
+        return np.where(np.abs(e) < 1e-7, kind(0), e)
+
+    vhalf, pq = v - half, p0 + q0
+    e = e0 - half * pq
+    p = pressure(cls / vhalf, e)
+    pqh = p + viscosity(e, vhalf, p)[0]
+    e = cut(e + half * (3 * pq - 4 * pqh))
+    p = pressure(cls / v, e)
+    e = cut(e - (7 * pq - 8 * pqh + p + viscosity(e, v, p)[0]) * (delv / 6))
+    p = pressure(cls / v, e)
+    q, ss = viscosity(e, v, p)
+    return e, p, np.where((delv <= 0) & (np.abs(q) < 1e-7), kind(0), q), ss
+
+
+def _eos_errors(host, state, p_cut=1e-7):
+    """Worst relative error over the elements of e, p, q and ss: of the
+    integers, and of plain double arithmetic."""
+    state = np.array(np.broadcast_arrays(*state), np.float64)
+    n = state.shape[1]
+    out, fits = np.empty((4, n)), np.empty(n, np.int32)
+    host.host_eos(n, state, p_cut, out, fits)
+    assert fits.all()
+    exact, plain = eos_reference(np.longdouble, *state, p_cut), eos_reference(np.float64, *state, p_cut)
+    errors = []
+    for got, want, dbl in zip(out, exact, plain):
+        np.testing.assert_array_equal(got == 0.0, want == 0)
+        live = want != 0
+        errors.append([float(np.max(np.abs((x - want)[live] / want[live]), initial=0.0)) for x in (got, dbl)])
+    return errors
+
+
+def _assert_no_worse_than_double(errors):
+    # 4 units of half a last place: a few truncations of integers of 2^57
+    for name, (got, plain) in zip(("e", "p", "q", "ss"), errors):
+        assert got <= max(plain, 4 * 2.0 ** -53), (name, got, plain)
+
+
+@pytest.mark.parametrize("delv", [-1e-5, -0.01, -0.1, -0.2])
+@pytest.mark.parametrize("du2", [1e-3, 1.0, 1e4, 1e6, 1e10])
+@pytest.mark.parametrize("e0", [1e-6, 1e-3, 1.0, 1e4])
+def test_eos_at_a_shock_front(host, e0, du2, delv):
+    """Cold elements that a shock of velocity jump du compresses: the work of
+    the viscosity is many orders above the old energy, which still counts
+    through the sound speed."""
+    rng = np.random.default_rng(23)
+    n = 2000
+    v, e = rng.uniform(0.75, 1.0, n), e0 * rng.uniform(0.5, 1.0, n)
+    p = 2.0 / 3.0 * e / v
+    du2 = du2 * rng.uniform(0.5, 1.0, n)
+    state = e, np.where(p < 1e-7, 0.0, p), 0.0, np.sqrt(du2) / 2, 2.0 / 3.0 * du2, delv * v * rng.uniform(0.9, 1.0, n), v
+    _assert_no_worse_than_double(_eos_errors(host, state))
+
+
+@pytest.mark.parametrize("delv", [1e-5, 0.01, 0.1])
+@pytest.mark.parametrize("ratio", [0.0, 1.0, 1e6, 1e12])
+def test_eos_of_opening_elements(host, ratio, delv):
+    """Opening elements take no viscosity: whatever qq and ql hold (here the
+    pressure times `ratio` and its root) has no part in the result."""
+    rng = np.random.default_rng(29)
+    n = 2000
+    v, e = rng.uniform(0.8, 1.5, n), 10.0 ** rng.uniform(-4, 4, n)
+    p = 2.0 / 3.0 * e / v
+    state = e, p, 0.0, np.sqrt(ratio * p), ratio * p, delv * v * rng.uniform(0.9, 1.0, n), v
+    _assert_no_worse_than_double(_eos_errors(host, state))

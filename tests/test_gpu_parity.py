@@ -16,6 +16,7 @@ import numpy as np
 import pytest
 
 from conftest import golden_dump, rel_err
+from test_fixed_point import eos_reference
 
 pytestmark = pytest.mark.gpu
 
@@ -474,6 +475,40 @@ def test_material_ranges(lulesh, kind, params):
         dom.close()
     for f, want in out["fp64_exact"].items():
         assert rel_err(out["fp64"][f], want) < 1e-12, f
+
+
+@pytest.mark.parametrize("e0", [1e-6, 1e-2, 1e3])
+@pytest.mark.parametrize("way", [-1, 1])
+def test_material_of_each_element(lulesh, e0, way):
+    """Element by element, the double path's energies, pressures and
+    viscosities stay within rounding of the EOS in extended precision: cold
+    and warm elements that a shock of some 100 m/s closes, and opening ones."""
+    s = 6
+    rng = np.random.default_rng(41)
+    pos, vel, volo, _ = _distorted(s, "plain", rng)
+    ne = s ** 3
+    vnew, e = rng.uniform(0.75, 1.0, ne), e0 * rng.uniform(0.5, 1.0, ne)
+    delv, p, q = way * rng.uniform(0.0, 0.15, ne) * vnew, 2.0 / 3.0 * e / vnew, np.zeros(ne)
+    dom = lulesh.HostDomain(s, 11)
+    for f, a in zip(("x", "y", "z", "xd", "yd", "zd"), pos + vel):
+        getattr(dom, f)[:] = a
+    dom.volo[:], dom.elemMass[:] = volo, volo * 1.3
+    dev = lulesh.Device(dom, "fp64")
+    dev.phase(lulesh.PHASE_KINEMATICS, 1e-7)
+    dev.download()
+    dom.vnew[:], dom.delv[:], dom.e[:], dom.p[:], dom.q[:] = vnew, delv, e, p, q
+    dev.upload(lulesh.F_KIN | lulesh.F_EPQ)
+    dev.phase(lulesh.PHASE_MATERIAL)
+    dev.download()
+    assert (np.asarray(dom.qq) > 0).sum() > ne // 4
+    want = eos_reference(np.longdouble, e, p, q, dom.ql, dom.qq, delv, vnew, 1e-7)
+    for f, w in zip(("e", "p", "q", "ss"), want):
+        got = np.asarray(getattr(dom, f))
+        np.testing.assert_array_equal(got == 0.0, w == 0, err_msg=f)
+        live = w != 0
+        # the chain's 45 roundings in double come to 8 half ulps at most on such states
+        assert np.max(np.abs((got - w)[live] / w[live]), initial=0.0) < 16 * 2.0 ** -53, f
+    dev.close()
 
 
 @pytest.mark.parametrize("field,value", [("x", np.nan), ("zd", np.inf), ("yd", np.nan)])

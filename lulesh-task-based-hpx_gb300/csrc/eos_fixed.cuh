@@ -160,8 +160,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     const int up = tp - 57, ue = te - 58;
     ok &= cut.emin - 1023 > te + 3;
     const int64_t po = mantissa(p_old) >> clamp63(up0 - (xp - 1080)), qo = mantissa(q_old) >> clamp63(up0 - (xq - 1080)),
-                  qb = mantissa(qq) >> clamp63(up - (xqq - 1080)), pc = cut_in(cut.p_cut, cut.up, up),
-                  ec = cut_in(cut.e_cut, cut.ue, ue);
+                  qb = mantissa(qq) >> clamp63(up - (xqq - 1080)), ec = cut_in(cut.e_cut, cut.ue, ue);
     // volumes: 2/3 over the half-step one and the new one
     const int64_t mv = mantissa(v), md = mantissa(delv);
     int64_t mh = mv - (md >> clamp63(xv - xd + 1));  // in (2^56, 1.25 2^58)
@@ -169,7 +168,11 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     mh = (mh << nh) >> 1;
     const int uh = xv - 1080 + 1 - nh;
     const Limb bh = limb(mul(reciprocal(mh), kTwoThirds)), bv = limb(mul(reciprocal(mv), kTwoThirds));
-    const int nph = up - (ue0 + 58 - 115 - uh), npv = up - (ue + 58 - 115 - (xv - 1080));
+    // pressures of an energy, in units of the energy's own precision: there the
+    // cutoff is tested, which may be far below the unit of their sums
+    const int uph = ue0 + 58 - 115 - uh, upv = ue + 58 - 115 - (xv - 1080);
+    const int64_t pch = cut_in(cut.p_cut, cut.up, uph), pcv = cut_in(cut.p_cut, cut.up, upv);
+    const int nph = up - uph, npv = up - upv;
     // work factors: delv / 2 in a unit that takes it to 2^59, delv / 6 in half of it
     const Limb hd = limb(2 * md), d6 = limb(mul(md, 4 * kThird));
     const int nw0 = ue0 - (xd - 1082 + up0 + 58), nw = ue - (xd - 1082 + up + 58);
@@ -177,12 +180,12 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     const int sph = clamp63(nph), spv = clamp63(npv), sw2 = clamp63(nw - 2);
     const Limb lf = limb(mul(mantissa(ql), kRootFull)), lc = limb(mul(mantissa(ql), kRootCut));
     const int ul = xl - 1080 + 1, ql_unit = up - (ul + 58);
-    // the viscosity of an energy and the pressure that came of it
-    auto viscosity = [&](int64_t e, int unit, int64_t p) {
+    // the viscosity of an energy, whose pressure may have been cut
+    auto viscosity = [&](int64_t e, int unit, bool off) {
         int us;
         const int64_t s = energy_root(e, unit, us);
         const int n = ql_unit - us;
-        const int64_t lin = mul(limb(s), p == 0 ? lc : lf) >> (n < 0 ? 0 : clamp63(n));
+        const int64_t lin = mul(limb(s), off ? lc : lf) >> (n < 0 ? 0 : clamp63(n));
         ok &= n >= 0 || e <= 0;
         return (e > 0 ? lin : 0) + qb;
     };
@@ -191,25 +194,27 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     // evaluation follow the viscosity, which at a shock front is some 2^30
     // times the cold element's energy, and its root is a part of the result
     int64_t e = (mantissa(e_old) >> clamp63(ue0 - (xe - 1080))) - (mul(hd, limb(po + qo)) >> clamp63(nw0));
-    int64_t p = mul(bh, limb(e)) >> sph;
-    p = p < pc ? 0 : p;
+    int64_t p = mul(bh, limb(e));
+    bool off = p < pch;
+    p = off ? 0 : p >> sph;
     const int64_t pq = (po + qo) >> clamp63(up - up0);
-    const int64_t pqh = p + viscosity(e, ue0, p);
+    const int64_t pqh = p + viscosity(e, ue0, off);
     ok &= pqh < kBig && pqh > -kBig;
     e = (e >> clamp63(ue - ue0)) + (mul(hd, limb((3 * pq - 4 * pqh) >> 2)) >> sw2);
     e = e < ec && e > -ec ? 0 : e;
     ok &= e < 2 * kBig && e > -2 * kBig;
     // corrector
-    p = mul(bv, limb(e)) >> spv;
-    p = p < pc ? 0 : p;
-    const int64_t pqt = p + viscosity(e, ue, p);
+    p = mul(bv, limb(e));
+    off = p < pcv;
+    p = off ? 0 : p >> spv;
+    const int64_t pqt = p + viscosity(e, ue, off);
     ok &= pqt < kBig && pqt > -kBig;
     e -= mul(d6, limb((7 * pq - 8 * pqh + pqt) >> 3)) >> sw2;
     e = e < ec && e > -ec ? 0 : e;
     ok &= e < 2 * kBig && e > -2 * kBig;
     // the pressure, the viscosity and the sound speed from the energy's own
     // mantissa and root
-    const bool off = (mul(bv, limb(e)) >> spv) < pc;
+    off = mul(bv, limb(e)) < pcv;
     const bool warm = e > 0;
     int us;
     const int64_t s = energy_root(e, ue, us);

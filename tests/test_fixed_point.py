@@ -142,3 +142,19 @@ def test_eos_of_opening_elements(host, ratio, delv):
     p = 2.0 / 3.0 * e / v
     state = e, p, 0.0, np.sqrt(ratio * p), ratio * p, delv * v * rng.uniform(0.9, 1.0, n), v
     _assert_no_worse_than_double(_eos_errors(host, state))
+
+
+@pytest.mark.parametrize("p_cut", [1e-7, 1e-3])
+@pytest.mark.parametrize("delv", [-1e-5, -0.01, -0.1])
+@pytest.mark.parametrize("e0", [1e-5, 1e-2])
+def test_eos_cuts_pressures_by_their_own_size(host, e0, delv, p_cut):
+    """Whether a pressure is below the cutoff decides the sound speed that
+    goes into the viscosity, at a front so strong that the pressure itself is
+    lost beside the viscosity."""
+    rng = np.random.default_rng(31)
+    n = 2000
+    v, e = rng.uniform(0.75, 1.0, n), e0 * rng.uniform(0.01, 1.0, n)
+    p = 2.0 / 3.0 * e / v
+    du2 = 1e14 * rng.uniform(0.5, 1.0, n)
+    state = e, np.where(p < p_cut, 0.0, p), 0.0, np.sqrt(du2) / 2, 2.0 / 3.0 * du2, delv * v * rng.uniform(0.9, 1.0, n), v
+    _assert_no_worse_than_double(_eos_errors(host, state, p_cut))

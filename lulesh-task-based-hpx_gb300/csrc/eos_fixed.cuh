@@ -155,6 +155,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     te = th + tp + 2 > te ? th + tp + 2 : te;
     const int tl = xl - 1022 + ((te + 3) >> 1);  // of the linear viscosity
     tp = te + tb > tp ? te + tb : tp;
+    ok &= tl <= tp + 3;  // else the corrector's own sets a unit too coarse for the pressures it comes from
     tp = tl > tp ? tl : tp;
     te = th + tp + 2 > te ? th + tp + 2 : te;
     const int up = tp - 57, ue = te - 58;

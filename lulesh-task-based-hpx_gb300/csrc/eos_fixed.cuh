@@ -74,6 +74,8 @@ LULESH_BF int64_t root(int64_t m) {
     return s + mul(s, C);
 }
 
+constexpr double kCold = 1e-30;  // energies above have more than the least sound speed, .3333333e-18
+
 // The parameters the integer path depends on: it needs pmin = 0, a unit
 // reference density and cutoffs that hide what it flushes to zero.
 struct EosCuts {
@@ -99,9 +101,11 @@ LULESH_BF EosCuts eos_cuts(double e_cut, double p_cut, double q_cut, double pmin
     c.ue = exponent(e_cut) - 1080;
     c.up = exponent(p_cut) - 1080;
     c.emin = exponent(emin);
-    // cutoffs in [2^-300, 2^300], as far from the flushed 2^-1022 as from overflow
+    // cutoffs in [2^-300, 2^300], as far from the flushed 2^-1022 as from overflow;
+    // that of energies above those that have the least sound speed
     auto sane = [](double x) { return bits_of(x) >= bits_of(4.9e-91) && bits_of(x) <= bits_of(2.0e90); };
-    c.ok = sane(e_cut) && sane(p_cut) && sane(q_cut) && bits_of(pmin) << 1 == 0 && bits_of(emin) < 0 && bits_of(emin) << 1 != 0 &&
+    c.ok = sane(e_cut) && bits_of(e_cut) >= bits_of(kCold) && sane(p_cut) && sane(q_cut) && bits_of(pmin) << 1 == 0 &&
+           bits_of(emin) < 0 && bits_of(emin) << 1 != 0 &&
            uint64_t(bits_of(emin)) <= 0xfff0000000000000ull && bits_of(refdens) == bits_of(1.0);
     return c;
 }
@@ -155,11 +159,16 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     te = th + tp + 2 > te ? th + tp + 2 : te;
     const int tl = xl - 1022 + ((te + 3) >> 1);  // of the linear viscosity
     tp = te + tb > tp ? te + tb : tp;
-    ok &= tl <= tp + 3;  // else the corrector's own sets a unit too coarse for the pressures it comes from
+    ok &= tl <= tp + 1;  // else the corrector's own sets a unit too coarse for the pressures it comes from
     tp = tl > tp ? tl : tp;
     te = th + tp + 2 > te ? th + tp + 2 : te;
     const int up = tp - 57, ue = te - 58;
     ok &= cut.emin - 1023 > te + 3;
+    // Without energy the linear viscosity is .3333333e-18 ql, left out below:
+    // less than half a last place of qq unless ql is above 2^7 qq, and of no
+    // account while all energies are below the cutoff with and without it
+    const int tc = cut.ue + 56;  // of half the cutoff
+    ok &= xl <= xqq + 7 || (te < tc && xl - 1079 + th <= tc) || (bits_of(e_old) >= bits_of(kCold) && xl < 1053);
     const int64_t po = mantissa(p_old) >> clamp63(up0 - (xp - 1080)), qo = mantissa(q_old) >> clamp63(up0 - (xq - 1080)),
                   qb = mantissa(qq) >> clamp63(up - (xqq - 1080)), ec = cut_in(cut.e_cut, cut.ue, ue);
     // volumes: 2/3 over the half-step one and the new one
@@ -195,6 +204,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     // evaluation follow the viscosity, which at a shock front is some 2^30
     // times the cold element's energy, and its root is a part of the result
     int64_t e = (mantissa(e_old) >> clamp63(ue0 - (xe - 1080))) - (mul(hd, limb(po + qo)) >> clamp63(nw0));
+    ok &= e >= 0 || xl == 0;  // the unit of the pressures counts a root in
     int64_t p = mul(bh, limb(e));
     bool off = p < pch;
     p = off ? 0 : p >> sph;
@@ -225,8 +235,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     p_new = warm && !off ? scaled(mul(bv, limb(m)), ue - n - 115 - (xv - 1080) + 58) : 0.0;
     const double lin = scaled(mul(limb(s), off ? lc : lf), us + ul + 58);
     q_new = (warm ? lin : .3333333e-18 * ql) + qq;
-    ss = scaled(mul(s, off ? kRootCut : kRootFull), us + 1);
-    ss = warm && bits_of(ss) > bits_of(.33333331e-18) ? ss : .3333333e-18;
+    ss = warm ? scaled(mul(s, off ? kRootCut : kRootFull), us + 1) : .3333333e-18;
     return ok;
 }
 

@@ -175,3 +175,19 @@ def test_eos_of_linear_viscosity(host, e0, qq, ql, delv):
     qq = np.where(np.arange(n) % 5 == 0, 0.0, qq * rng.uniform(0.5, 1.0, n))
     state = e, 0.0, q, ql * rng.uniform(0.5, 1.0, n), qq, delv * v * rng.uniform(0.9, 1.0, n), v
     _assert_no_worse_than_double(_eos_errors(host, state, all_fit=False))
+
+
+@pytest.mark.parametrize("delv", [-1e-4, -0.01, -0.2])
+@pytest.mark.parametrize("ql", [0.0, 1.0, 6.0, 1e8])
+@pytest.mark.parametrize("qq", [2e-3, 1e3, 1e9])
+@pytest.mark.parametrize("e0", [0.0, -1e-7, -1e-3, -1e3, 1e-60])
+def test_eos_of_no_energy(host, e0, qq, ql, delv):
+    """Energies at and below zero, and those whose root is below the least
+    sound speed, have that sound speed: its part in the viscosity counts."""
+    rng = np.random.default_rng(37)
+    n = 2000
+    v, e = rng.uniform(0.75, 1.0, n), e0 * rng.uniform(0.5, 1.0, n)
+    q = np.where(np.arange(n) % 3 == 0, 0.0, qq * rng.uniform(0.0, 1.0, n))
+    qq = np.where(np.arange(n) % 5 == 0, 0.0, qq * rng.uniform(0.5, 1.0, n))
+    state = e, 0.0, q, ql * rng.uniform(0.5, 1.0, n), qq, delv * v * rng.uniform(0.9, 1.0, n), v
+    _assert_no_worse_than_double(_eos_errors(host, state, all_fit=False))

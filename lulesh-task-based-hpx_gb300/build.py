@@ -9,7 +9,9 @@ Floating-point contraction is part of the numerics contract:
   * fp64_exact.cu, time_increment.cu, verify.cu and device_init.cu are
     built with --fmad=false, so the exact double path, the device
     TimeIncrement, the device final report and the device problem build
-    round every operation separately, as the reference source is written;
+    round every operation separately, as the reference source is written
+    (the material kernels of the other units advance the time too: their
+    contraction is kept out of it in the code, time_advance.cuh);
   * domain.cpp (problem set-up, host TimeIncrement) is built with
     -ffp-contract=off so the host numbers do not depend on whether the host
     compiler fuses multiply-adds (GCC does by default on aarch64).

@@ -1,9 +1,9 @@
 // Device-side TimeIncrement, shared by the time kernels and by the material
 // kernel, whose last block advances the time of the graph form's next cycle.
-// No operation here can be contracted (a product is divided or stored, never
-// added to), so every unit rounds it as the host TimeIncrement does, whatever
-// its contraction setting, and the graph forms and the host loop pick
-// identical time steps.
+// Units compile it with and without contraction. The one product that could
+// reach a sum, olddt * deltatimemultub, is rounded by itself (__dmul_rn; the
+// others are exact or divided), so all round as the host TimeIncrement does,
+// and the graph forms and the host loop pick identical time steps.
 #pragma once
 
 #include "lulesh_dev.h"
@@ -29,7 +29,7 @@ static __device__ __forceinline__ bool advance_time(DevTime* t, const StepResult
         const double ratio = newdt / olddt;
         if (ratio >= 1.0) {
             if (ratio < t->deltatimemultlb) newdt = olddt;
-            else if (ratio > t->deltatimemultub) newdt = olddt * t->deltatimemultub;
+            else if (ratio > t->deltatimemultub) newdt = __dmul_rn(olddt, t->deltatimemultub);
         }
         if (newdt > t->dtmax) newdt = t->dtmax;
         t->deltatime = newdt;

@@ -1,7 +1,7 @@
 // Device-side time control for the CUDA-graph forms of the time loop.
-// Built with --fmad=false: every operation is rounded as the host
-// TimeIncrement rounds it, so the graph forms and the host loop pick
-// identical time steps.
+// Built with --fmad=false, as the host TimeIncrement is built without
+// contraction; time_advance.cuh rounds alike either way, as the material
+// kernels compile it too.
 #include "time_advance.cuh"
 
 namespace lulesh {

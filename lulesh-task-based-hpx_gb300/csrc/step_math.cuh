@@ -51,7 +51,7 @@ __device__ __forceinline__ float pmul(float a, float b) { return a * b; }
 // element in k_forces, of which 680 products go here. Out of line, as so many
 // do not fit the instruction cache: inlined for the hourglass forces alone
 // k_forces takes 0.60 ms at s=60, with two products to a call 0.567, this way
-// 0.527 (0.609 without; k_kinematics 0.331 -> 0.273, material with its
+// 0.527 (0.609 without; k_kinematics 0.331 -> 0.277, material with its
 // compares in integers 0.341 -> 0.266). Plain in the other variants.
 #if LULESH_EXACT
 __device__ __noinline__ double xmul(double a, double b) { return dmul_ipipe(a, b); }
@@ -115,9 +115,7 @@ __device__ __forceinline__ R hex_volume(const R x[8], const R y[8], const R z[8]
     return pmul(vol, twelveth);
 }
 
-// 8 times the centre Jacobian of CalcElemShapeFunctionDerivatives
-// (lulesh.cc:277-305): the powers of two of its determinant and shape
-// derivatives commute with rounding and cancel in the velocity gradient.
+// Centre Jacobian of CalcElemShapeFunctionDerivatives (lulesh.cc:277-305).
 template <class R>
 struct Jac {
     R fjxxi, fjxet, fjxze, fjyxi, fjyet, fjyze, fjzxi, fjzet, fjzze;
@@ -125,20 +123,21 @@ struct Jac {
 
 template <class R>
 __device__ __forceinline__ Jac<R> jacobian(const R x[8], const R y[8], const R z[8]) {
+    const R c = R(.125);
     Jac<R> j;
-    j.fjxxi = (x[6] - x[0]) + (x[5] - x[3]) - (x[7] - x[1]) - (x[4] - x[2]);
-    j.fjxet = (x[6] - x[0]) - (x[5] - x[3]) + (x[7] - x[1]) - (x[4] - x[2]);
-    j.fjxze = (x[6] - x[0]) + (x[5] - x[3]) + (x[7] - x[1]) + (x[4] - x[2]);
-    j.fjyxi = (y[6] - y[0]) + (y[5] - y[3]) - (y[7] - y[1]) - (y[4] - y[2]);
-    j.fjyet = (y[6] - y[0]) - (y[5] - y[3]) + (y[7] - y[1]) - (y[4] - y[2]);
-    j.fjyze = (y[6] - y[0]) + (y[5] - y[3]) + (y[7] - y[1]) + (y[4] - y[2]);
-    j.fjzxi = (z[6] - z[0]) + (z[5] - z[3]) - (z[7] - z[1]) - (z[4] - z[2]);
-    j.fjzet = (z[6] - z[0]) - (z[5] - z[3]) + (z[7] - z[1]) - (z[4] - z[2]);
-    j.fjzze = (z[6] - z[0]) + (z[5] - z[3]) + (z[7] - z[1]) + (z[4] - z[2]);
+    j.fjxxi = c * ((x[6] - x[0]) + (x[5] - x[3]) - (x[7] - x[1]) - (x[4] - x[2]));
+    j.fjxet = c * ((x[6] - x[0]) - (x[5] - x[3]) + (x[7] - x[1]) - (x[4] - x[2]));
+    j.fjxze = c * ((x[6] - x[0]) + (x[5] - x[3]) + (x[7] - x[1]) + (x[4] - x[2]));
+    j.fjyxi = c * ((y[6] - y[0]) + (y[5] - y[3]) - (y[7] - y[1]) - (y[4] - y[2]));
+    j.fjyet = c * ((y[6] - y[0]) - (y[5] - y[3]) + (y[7] - y[1]) - (y[4] - y[2]));
+    j.fjyze = c * ((y[6] - y[0]) + (y[5] - y[3]) + (y[7] - y[1]) + (y[4] - y[2]));
+    j.fjzxi = c * ((z[6] - z[0]) + (z[5] - z[3]) - (z[7] - z[1]) - (z[4] - z[2]));
+    j.fjzet = c * ((z[6] - z[0]) - (z[5] - z[3]) + (z[7] - z[1]) - (z[4] - z[2]));
+    j.fjzze = c * ((z[6] - z[0]) + (z[5] - z[3]) + (z[7] - z[1]) + (z[4] - z[2]));
     return j;
 }
 
-// 64 times the determinant only (lulesh.cc:308-373 without the B matrix).
+// An eighth of the determinant only (lulesh.cc:308-373 without the B matrix).
 template <class R>
 __device__ __forceinline__ R jac_det(const Jac<R>& j) {
     const R cjxet = -(j.fjyxi * j.fjzze) + (j.fjzxi * j.fjyze);
@@ -202,8 +201,8 @@ __device__ __forceinline__ bool jacobian_singular(const R x[8], const R y[8], co
 #endif
 }
 
-// 64 times the shape-function derivatives b[a][0..3] (b[a][4..7] are their
-// negatives, lulesh.cc:337-364) and 64 times the determinant.
+// Shape-function derivatives b[a][0..3] (b[a][4..7] are their negatives,
+// lulesh.cc:337-364) and the determinant.
 template <class R>
 __device__ __forceinline__ R shape_derivs(const Jac<R>& j, R b[3][4]) {
     const R cjxxi = xmul(j.fjyet, j.fjzze) - xmul(j.fjzet, j.fjyze);
@@ -227,7 +226,7 @@ __device__ __forceinline__ R shape_derivs(const Jac<R>& j, R b[3][4]) {
     b[2][1] = cjzxi - cjzet - cjzze;
     b[2][2] = cjzxi + cjzet - cjzze;
     b[2][3] = -cjzxi + cjzet - cjzze;
-    return xmul(j.fjxet, cjxet) + xmul(j.fjyet, cjyet) + xmul(j.fjzet, cjzet);
+    return R(8.) * (xmul(j.fjxet, cjxet) + xmul(j.fjyet, cjyet) + xmul(j.fjzet, cjzet));
 }
 
 // Division helpers. x / refdens is x itself when refdens is 1 (the
@@ -846,62 +845,65 @@ __device__ __forceinline__ R max_face_area(const R x[8], const R y[8], const R z
 // Monotonic-Q gradients of CalcMonotonicQGradientsForElemsTask
 // (lulesh.cc:1341-1416). vol = volo * vnew. Outputs
 // g[0..2] = delv_xi, delv_eta, delv_zeta and g[3..5] = delx_xi, delx_eta, delx_zeta.
-// The reference's factors 0.25 of the differences are left to the end, where
-// there are fewer: powers of two commute with rounding.
+// (The factors 0.25, and the Jacobian's 0.125, stay where the reference has
+// them: left out, as powers of two that commute with rounding, k_kinematics
+// takes 0.273 in place of 0.277 ms at s=60, but squares of areas overflow and
+// determinants underflow at other sizes.)
 template <class R>
 __device__ __forceinline__ void q_gradients(const R x[8], const R y[8], const R z[8], const R xv[8],
                                             const R yv[8], const R zv[8], R vol, R g[6]) {
     const R ptiny = R(1.e-36);
-    const R norm = rcp(vol + ptiny), pt = R(256.0) * ptiny, vol16 = R(16.0) * vol, scale = R(0.015625);
-    const R dxj = -((x[0] + x[1] + x[5] + x[4]) - (x[3] + x[2] + x[6] + x[7]));
-    const R dyj = -((y[0] + y[1] + y[5] + y[4]) - (y[3] + y[2] + y[6] + y[7]));
-    const R dzj = -((z[0] + z[1] + z[5] + z[4]) - (z[3] + z[2] + z[6] + z[7]));
-    const R dxi = (x[1] + x[2] + x[6] + x[5]) - (x[0] + x[3] + x[7] + x[4]);
-    const R dyi = (y[1] + y[2] + y[6] + y[5]) - (y[0] + y[3] + y[7] + y[4]);
-    const R dzi = (z[1] + z[2] + z[6] + z[5]) - (z[0] + z[3] + z[7] + z[4]);
-    const R dxk = (x[4] + x[5] + x[6] + x[7]) - (x[0] + x[1] + x[2] + x[3]);
-    const R dyk = (y[4] + y[5] + y[6] + y[7]) - (y[0] + y[1] + y[2] + y[3]);
-    const R dzk = (z[4] + z[5] + z[6] + z[7]) - (z[0] + z[1] + z[2] + z[3]);
+    const R q = R(0.25), mq = R(-0.25);
+    const R norm = rcp(vol + ptiny);
+    const R dxj = mq * ((x[0] + x[1] + x[5] + x[4]) - (x[3] + x[2] + x[6] + x[7]));
+    const R dyj = mq * ((y[0] + y[1] + y[5] + y[4]) - (y[3] + y[2] + y[6] + y[7]));
+    const R dzj = mq * ((z[0] + z[1] + z[5] + z[4]) - (z[3] + z[2] + z[6] + z[7]));
+    const R dxi = q * ((x[1] + x[2] + x[6] + x[5]) - (x[0] + x[3] + x[7] + x[4]));
+    const R dyi = q * ((y[1] + y[2] + y[6] + y[5]) - (y[0] + y[3] + y[7] + y[4]));
+    const R dzi = q * ((z[1] + z[2] + z[6] + z[5]) - (z[0] + z[3] + z[7] + z[4]));
+    const R dxk = q * ((x[4] + x[5] + x[6] + x[7]) - (x[0] + x[1] + x[2] + x[3]));
+    const R dyk = q * ((y[4] + y[5] + y[6] + y[7]) - (y[0] + y[1] + y[2] + y[3]));
+    const R dzk = q * ((z[4] + z[5] + z[6] + z[7]) - (z[0] + z[1] + z[2] + z[3]));
     R ax, ay, az, dxv, dyv, dzv;
 
     // zeta: i cross j
     ax = xmul(dyi, dzj) - xmul(dzi, dyj);
     ay = xmul(dzi, dxj) - xmul(dxi, dzj);
     az = xmul(dxi, dyj) - xmul(dyi, dxj);
-    g[5] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
+    g[5] = div_sqrt(vol, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + ptiny);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = (xv[4] + xv[5] + xv[6] + xv[7]) - (xv[0] + xv[1] + xv[2] + xv[3]);
-    dyv = (yv[4] + yv[5] + yv[6] + yv[7]) - (yv[0] + yv[1] + yv[2] + yv[3]);
-    dzv = (zv[4] + zv[5] + zv[6] + zv[7]) - (zv[0] + zv[1] + zv[2] + zv[3]);
-    g[2] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
+    dxv = q * ((xv[4] + xv[5] + xv[6] + xv[7]) - (xv[0] + xv[1] + xv[2] + xv[3]));
+    dyv = q * ((yv[4] + yv[5] + yv[6] + yv[7]) - (yv[0] + yv[1] + yv[2] + yv[3]));
+    dzv = q * ((zv[4] + zv[5] + zv[6] + zv[7]) - (zv[0] + zv[1] + zv[2] + zv[3]));
+    g[2] = xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv);
 
     // xi: j cross k
     ax = xmul(dyj, dzk) - xmul(dzj, dyk);
     ay = xmul(dzj, dxk) - xmul(dxj, dzk);
     az = xmul(dxj, dyk) - xmul(dyj, dxk);
-    g[3] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
+    g[3] = div_sqrt(vol, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + ptiny);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = (xv[1] + xv[2] + xv[6] + xv[5]) - (xv[0] + xv[3] + xv[7] + xv[4]);
-    dyv = (yv[1] + yv[2] + yv[6] + yv[5]) - (yv[0] + yv[3] + yv[7] + yv[4]);
-    dzv = (zv[1] + zv[2] + zv[6] + zv[5]) - (zv[0] + zv[3] + zv[7] + zv[4]);
-    g[0] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
+    dxv = q * ((xv[1] + xv[2] + xv[6] + xv[5]) - (xv[0] + xv[3] + xv[7] + xv[4]));
+    dyv = q * ((yv[1] + yv[2] + yv[6] + yv[5]) - (yv[0] + yv[3] + yv[7] + yv[4]));
+    dzv = q * ((zv[1] + zv[2] + zv[6] + zv[5]) - (zv[0] + zv[3] + zv[7] + zv[4]));
+    g[0] = xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv);
 
     // eta: k cross i
     ax = xmul(dyk, dzi) - xmul(dzk, dyi);
     ay = xmul(dzk, dxi) - xmul(dxk, dzi);
     az = xmul(dxk, dyi) - xmul(dyk, dxi);
-    g[4] = div_sqrt(vol16, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + pt);
+    g[4] = div_sqrt(vol, xmul(ax, ax) + xmul(ay, ay) + xmul(az, az) + ptiny);
     ax *= norm;
     ay *= norm;
     az *= norm;
-    dxv = -((xv[0] + xv[1] + xv[5] + xv[4]) - (xv[3] + xv[2] + xv[6] + xv[7]));
-    dyv = -((yv[0] + yv[1] + yv[5] + yv[4]) - (yv[3] + yv[2] + yv[6] + yv[7]));
-    dzv = -((zv[0] + zv[1] + zv[5] + zv[4]) - (zv[3] + zv[2] + zv[6] + zv[7]));
-    g[1] = scale * (xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv));
+    dxv = mq * ((xv[0] + xv[1] + xv[5] + xv[4]) - (xv[3] + xv[2] + xv[6] + xv[7]));
+    dyv = mq * ((yv[0] + yv[1] + yv[5] + yv[4]) - (yv[3] + yv[2] + yv[6] + yv[7]));
+    dzv = mq * ((zv[0] + zv[1] + zv[5] + zv[4]) - (zv[3] + zv[2] + zv[6] + zv[7]));
+    g[1] = xmul(ax, dxv) + xmul(ay, dyv) + xmul(az, dzv);
 }
 
 // Trace of the velocity gradient at the half-step geometry

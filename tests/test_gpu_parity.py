@@ -321,6 +321,42 @@ def test_force_and_kinematics_ranges(lulesh, oracle_mod, s, kind):
     dev.close()
 
 
+@pytest.mark.parametrize("power", [-358, -170, 250, 253, 256, 258])
+def test_exact_variant_at_extreme_sizes(lulesh, oracle_mod, power):
+    """The exact variant's intermediate values overflow and underflow where
+    the reference's do: a mesh scaled by a power of two either raises the
+    reference's error (a Jacobian determinant that underflows to zero) or
+    gives the oracle's bits, squares of areas that overflow included."""
+    s, scale = 3, 2.0 ** power
+    pos, vel, volo, _ = _distorted(s, "plain", np.random.default_rng(13))  # without pressure: coasting nodes
+    o = oracle_mod.Oracle(s, 11, 1, 1, threads=1, portable_cbrt=True)
+    dom = lulesh.HostDomain(s, 11)
+    dt = 1e-7 * scale
+    for put in (lambda f, a: getattr(dom, f).__setitem__(slice(None), a),
+                lambda f, a: o.field(f).__setitem__(slice(None), a)):
+        for f, a in zip(("x", "y", "z", "xd", "yd", "zd"), [a * scale for a in pos] + vel):
+            put(f, a)
+        put("volo", np.maximum(volo * scale * scale * scale, 1e-300))
+    o.set_scalar("deltatime", dt)
+    dev = lulesh.Device(dom, "fp64_exact")
+    if power == -358:
+        assert o.leapfrog() != 0
+        with pytest.raises(lulesh.LuleshError) as ei:
+            dev.phase(lulesh.PHASE_FORCES, dt)
+        assert ei.value.status == lulesh.EVOLUME
+    else:
+        o.leapfrog()
+        for phase in (lulesh.PHASE_FORCES, lulesh.PHASE_NODES, lulesh.PHASE_KINEMATICS):
+            dev.phase(phase, dt)
+        dev.download()
+        for f in ("x", "zd", "vnew", "delv", "arealg", "vdov"):
+            np.testing.assert_array_equal(getattr(dom, f), o.field(f), err_msg=f)
+        grads = [o.field(f) for f in ("delv_xi", "delv_eta", "delv_zeta", "delx_xi", "delx_eta", "delx_zeta")]
+        for got, want in zip(dev.gradients(), grads):
+            np.testing.assert_array_equal(got, want)
+    dev.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64_exact", "fp64", "mixed"])
 @pytest.mark.parametrize("s", [3, 28])
 def test_still_mesh_of_signed_zeros(lulesh, precision, s):

@@ -45,6 +45,13 @@ __device__ __forceinline__ void mirror_node(const Mesh& m, int n) {
     m.vzp[n] = split(m.zd[n]);
 }
 
+// x <= 0 on the integer pipe; false for a NaN of either sign, which f_le takes
+// by its sign bit.
+__device__ __forceinline__ bool not_positive(double x) {
+    const unsigned long long b = dmul_bits(x);
+    return b - 1ull >= 0x7fffffffffffffffull && b <= 0xfff0000000000000ull;
+}
+
 // Stress + hourglass corner forces of element i in float, stored combined
 // (corner-major).
 __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
@@ -71,7 +78,7 @@ __device__ __forceinline__ void forces_elem(const Mesh& m, int i) {
         }
     }
     const double determ = LD(m.volo + i) * LD(m.v + i);
-    if (f_le(determ, 0.0)) {
+    if (not_positive(determ)) {
         raise_error(m.result, i, PHASE_FORCES);
         return;
     }

@@ -574,6 +574,25 @@ def test_non_finite_nodes_stay_local(lulesh, field, value):
             assert not np.isfinite(out[1][k][near]).any()
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64_exact"])
+@pytest.mark.parametrize("v,refused", [(np.nan, False), (-np.nan, False), (0.0, True), (-0.0, True), (-1e-9, True),
+                                       (-np.inf, True), (5e-324, False), (np.inf, False)])
+def test_volumes_refused_by_the_force_phase(lulesh, precision, v, refused):
+    """The force phase refuses relative volumes that are <= 0 (lulesh.cc:908),
+    which a NaN of either sign is not."""
+    dom = lulesh.HostDomain(3)
+    dom.v[13] = v
+    dom.volo[13] = 1.0
+    dev = lulesh.Device(dom, precision)
+    if refused:
+        with pytest.raises(lulesh.LuleshError) as ei:
+            dev.phase(lulesh.PHASE_FORCES, 1e-9)
+        assert ei.value.status == lulesh.EVOLUME
+    else:
+        dev.phase(lulesh.PHASE_FORCES, 1e-9)
+    dev.close()
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_graph_loop_equals_host_loop(lulesh, precision):
     a, _, na = _run_device(lulesh, 12, 11, 1, 1, precision)

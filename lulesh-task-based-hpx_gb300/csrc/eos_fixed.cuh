@@ -268,8 +268,8 @@ LULESH_BF bool limiter_fixed(double self, double dm, double dp, int64_t& phi) {
 
 // The linear and quadratic viscosity coefficients (lulesh.cc:1600-1656):
 // ql = -qlc rho sum dxi (1 - phi), qq = qqc rho sum dxi^2 (1 - phi^2) with
-// dxi = min(0, delv delx) of each direction. False where the double path has
-// to do it.
+// dxi = min(0, delv delx) of each direction; subnormal gradients count as
+// zero. False where the double path has to do it.
 LULESH_BF bool q_sums(const double dv[3], const double dm[3], const double dp[3], const double dx[3], double& lin,
                       double& quad) {
     bool ok = true;
@@ -279,9 +279,11 @@ LULESH_BF bool q_sums(const double dv[3], const double dm[3], const double dp[3]
         int64_t phi;
         ok &= limiter_fixed(dv[d], dm[d], dp[d], phi);
         const int xv = exponent(dv[d]), xx = exponent(dx[d]);
-        ok &= xv < 1500 && xx < 1500 && xx > 500;
+        ok &= uint32_t(xx - 501) < 999u;
         const int64_t t = mul(mantissa(dv[d]), mantissa(dx[d]));  // delv delx, up to 2^58
-        const bool push = t < 0 && xv > 500;
+        // delv delx, its square and 2^-57 of that are normal numbers
+        ok &= t >= 0 || uint32_t(xv + xx - (2046 - 480)) < 960u;
+        const bool push = t < 0;
         const int u = xv + xx - 2160 + 58;
         // 1 - phi at full width, and with it 1 - phi^2 = (1 - phi) (1 + phi)
         const int64_t rest = kOne - phi;

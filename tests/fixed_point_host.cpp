@@ -43,4 +43,11 @@ void host_eos(int n, const double* in, double p_cut, double* out, int* fits) {
     }
 }
 
+// The viscosity sums of n elements: velocity gradients, those of the minus and
+// plus neighbours and lengths [n][3], sums lin and quad. fits[n] as above.
+void host_q_sums(int n, const double* dv, const double* dm, const double* dp, const double* dx, double* lin,
+                 double* quad, int* fits) {
+    for (int i = 0; i < n; ++i) fits[i] = q_sums(dv + 3 * i, dm + 3 * i, dp + 3 * i, dx + 3 * i, lin[i], quad[i]);
+}
+
 }  // extern "C"

@@ -22,6 +22,7 @@ def host(tmp_path_factory):
     lib = C.CDLL(str(lib))
     lib.host_forces.argtypes = [C.c_int] + [DOUBLES] * 6 + [INTS]
     lib.host_eos.argtypes = [C.c_int, DOUBLES, C.c_double, DOUBLES, INTS]
+    lib.host_q_sums.argtypes = [C.c_int] + [DOUBLES] * 6 + [INTS]
     return lib
 
 
@@ -191,3 +192,39 @@ def test_eos_of_no_energy(host, e0, qq, ql, delv):
     qq = np.where(np.arange(n) % 5 == 0, 0.0, qq * rng.uniform(0.5, 1.0, n))
     state = e, 0.0, q, ql * rng.uniform(0.5, 1.0, n), qq, delv * v * rng.uniform(0.9, 1.0, n), v
     _assert_no_worse_than_double(_eos_errors(host, state, all_fit=False))
+
+
+@pytest.mark.parametrize("length", [0.01, 1e-100, 1e100])
+@pytest.mark.parametrize("scale", [1e250, 1e140, 1e100, 1e4, 1e-7, 1e-100, 1e-152, 1e-160, 1e-300, 1e-310])
+def test_viscosity_sums(host, scale, length):
+    """The limited sums of the viscosity (lulesh.cc:1600-1656) over every size
+    of gradient (subnormal ones count as zero) and length: those that the
+    integers take are exact, those of which a square or a limited part would
+    leave the range they do not take."""
+    rng = np.random.default_rng(43)
+    n = 4000
+    dv, dm, dp = (scale * rng.uniform(-1.0, 1.0, (n, 3)) for _ in range(3))
+    for a in (dv, dm, dp):
+        a[rng.uniform(size=a.shape) < 0.1] = 0.0
+    dx = length * rng.uniform(0.1, 1.0, (n, 3))
+    lin, quad, fits = np.empty(n), np.empty(n), np.empty(n, np.int32)
+    host.host_q_sums(n, dv, dm, dp, dx, lin, quad, fits)
+    if 1e-130 < scale * length < 1e130:
+        assert fits.all()
+
+    dv[np.abs(dv) < 2.0 ** -1022] = 0.0
+
+    def limited(kind):
+        norm = 1 / (kind(1) * dv + kind(1e-36))
+        m, p = dm * norm, dp * norm
+        phi = np.clip(np.minimum(np.minimum((m + p) / 2, 2 * m), 2 * p), 0, 1)
+        d = np.minimum(kind(1) * dv * dx, 0)
+        return -(d * (1 - phi)).sum(axis=1), (d * d * (1 - phi * phi)).sum(axis=1)
+
+    with np.errstate(over="ignore", invalid="ignore"):
+        exact, plain = limited(np.longdouble), limited(np.float64)
+    for got, want, dbl in zip(*((a[fits != 0] for a in x) for x in ((lin, quad), exact, plain))):
+        np.testing.assert_array_equal(got == 0.0, want == 0)
+        live = want != 0
+        err = [np.max(np.abs((x - want)[live] / want[live]), initial=0.0) for x in (got, dbl)]
+        assert err[0] <= max(err[1], 4 * 2.0 ** -53), err

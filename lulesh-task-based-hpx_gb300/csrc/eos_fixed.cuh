@@ -163,7 +163,8 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     tp = tl > tp ? tl : tp;
     te = th + tp + 2 > te ? th + tp + 2 : te;
     const int up = tp - 57, ue = te - 58;
-    ok &= cut.emin - 1023 > te + 3;
+    // no result below emin, infinite or subnormal
+    ok &= cut.emin - 1023 > te + 3 && tp < 1000 && uint32_t(xl - 1) >= 200u;
     // Without energy the linear viscosity is .3333333e-18 ql, left out below:
     // less than half a last place of qq unless ql is above 2^7 qq, and of no
     // account while all energies are below the cutoff with and without it

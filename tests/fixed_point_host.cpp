@@ -32,8 +32,8 @@ void host_forces(int n, const double* x, const double* vel, const double* sc, co
 // One EOS evaluation of n elements: in[k] = e, p, q, ql, qq, delv, v and
 // out[k] = e, p, q, ss, each of n values; the cutoffs of e and q are 1e-7.
 // fits[n]: the element does not need the double form.
-void host_eos(int n, const double* in, double p_cut, double* out, int* fits) {
-    const EosCuts cuts = eos_cuts(1e-7, p_cut, 1e-7, 0.0, -1e15, 1.0);
+void host_eos_above(int n, const double* in, double p_cut, double emin, double* out, int* fits) {
+    const EosCuts cuts = eos_cuts(1e-7, p_cut, 1e-7, 0.0, emin, 1.0);
     auto at = [&](int k, int i) { return in[size_t(k) * n + i]; };
     for (int i = 0; i < n; ++i) {
         double* o = out + i;
@@ -41,6 +41,10 @@ void host_eos(int n, const double* in, double p_cut, double* out, int* fits) {
                                       o[n], o[2 * size_t(n)], o[3 * size_t(n)]);
         if (at(5, i) <= 0.0 && fabs(o[2 * size_t(n)]) < 1e-7) o[2 * size_t(n)] = 0.0;
     }
+}
+
+void host_eos(int n, const double* in, double p_cut, double* out, int* fits) {
+    host_eos_above(n, in, p_cut, -1e15, out, fits);
 }
 
 // The viscosity sums of n elements: velocity gradients, those of the minus and

@@ -22,6 +22,7 @@ def host(tmp_path_factory):
     lib = C.CDLL(str(lib))
     lib.host_forces.argtypes = [C.c_int] + [DOUBLES] * 6 + [INTS]
     lib.host_eos.argtypes = [C.c_int, DOUBLES, C.c_double, DOUBLES, INTS]
+    lib.host_eos_above.argtypes = [C.c_int, DOUBLES, C.c_double, C.c_double, DOUBLES, INTS]
     lib.host_q_sums.argtypes = [C.c_int] + [DOUBLES] * 6 + [INTS]
     return lib
 
@@ -225,6 +226,36 @@ def test_viscosity_sums(host, scale, length):
         exact, plain = limited(np.longdouble), limited(np.float64)
     for got, want, dbl in zip(*((a[fits != 0] for a in x) for x in ((lin, quad), exact, plain))):
         np.testing.assert_array_equal(got == 0.0, want == 0)
+        live = want != 0
+        err = [np.max(np.abs((x - want)[live] / want[live]), initial=0.0) for x in (got, dbl)]
+        assert err[0] <= max(err[1], 4 * 2.0 ** -53), err
+
+
+@pytest.mark.parametrize("delv", [-0.1, -1e-12, 1e-3])
+@pytest.mark.parametrize("v0", [1e-90, 1.0, 1e100])
+@pytest.mark.parametrize("power", [-306, -200, 150, 230])
+@pytest.mark.parametrize("field", ["e", "p", "q", "ql", "qq"])
+@pytest.mark.parametrize("base", [1.0, 1e-6])
+def test_eos_of_extreme_magnitudes(host, base, field, power, v0, delv):
+    """One input of extreme size beside ordinary ones, with relative volumes
+    and an energy floor far outside the reference's: what the integers take
+    is exact, and what would leave the range of a double they do not take."""
+    rng = np.random.default_rng(47)
+    n = 300
+    v = v0 * rng.uniform(0.75, 1.0, n)
+    e, p, q, ql, qq = (base * rng.uniform(0.5, 1.0, n) for _ in range(5))
+    big = 10.0 ** power * rng.uniform(0.5, 1.0, n)
+    state = [e, p, q, ql, qq, delv * v * rng.uniform(0.9, 1.0, n), v]
+    state["epq".index(field) if len(field) == 1 else 3 if field == "ql" else 4] = big
+    state = np.array(state)
+    out, fits = np.empty((4, n)), np.empty(n, np.int32)
+    host.host_eos_above(n, state, 1e-7, -1e300, out, fits)
+    taken = fits != 0
+    with np.errstate(all="ignore"):
+        exact, plain = (np.array(eos_reference(k, *state[:, taken], 1e-7)) for k in (np.longdouble, np.float64))
+    for got, want, dbl in zip(out[:, taken], exact, plain):
+        np.testing.assert_array_equal(got == 0.0, want == 0)
+        assert np.all(np.abs(want) < 1.7e308)
         live = want != 0
         err = [np.max(np.abs((x - want)[live] / want[live]), initial=0.0) for x in (got, dbl)]
         assert err[0] <= max(err[1], 4 * 2.0 ** -53), err

@@ -248,7 +248,8 @@ typedef struct lulesh_batch_tuning {
  * problems at once. */
 int lulesh_batch_create(int32_t precision, uint64_t pool_bytes, int32_t max_slots, lulesh_batch** out);
 void lulesh_batch_destroy(lulesh_batch* b);
-/* Device bytes one s^3 problem takes in a pool of this precision. */
+/* Device bytes one s^3 problem takes in a pool of this precision (for
+ * LULESH_FP64 with a reserve of 384 bytes per element that is not used). */
 int lulesh_batch_footprint(int32_t precision, int32_t s, uint64_t* bytes);
 /* Builds the problem on the device in its pool block (the state
  * Domain::Domain makes, bit for bit; the region runs of the reference's

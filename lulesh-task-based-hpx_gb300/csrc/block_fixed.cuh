@@ -529,7 +529,10 @@ struct KinGeo {
 
 // Axes whose units differ by more than this (an element some 8 to 16 times
 // longer than wide) take the double path: squares of vectors are summed in
-// the coarsest axis' unit, which costs their components that many bits.
+// the coarsest axis' unit, which costs their components that many bits. A
+// mesh of nothing but such elements pays for both paths: s=150, 32 times
+// wider than high, k_kinematics 2.42 ms in place of 0.64 (the double path by
+// itself took 2.09; the forces stay at 0.78).
 constexpr int kAspect = 3;
 
 LULESH_BF bool kin_geometry(const Sums& s, KinGeo& o) {

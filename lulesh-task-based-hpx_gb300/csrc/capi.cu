@@ -111,10 +111,12 @@ struct lulesh_dev {
     int64_t prof_cycles = 0, prof_launch0 = 0;
 };
 
-// Slabs of lulesh_leapfrog (element planes per slab = s / slabs). At s=150
-// a call of the drop-in takes 4.95, 4.91, 5.01 and 5.25 ms with 4, 6, 8 and 16
-// slabs: fewer leave more of the copies exposed, more add copy and launch
-// overhead.
+// Slabs of lulesh_leapfrog (element planes per slab = s / slabs): one count,
+// which the material order is built for, at every size above kLeapfrogWhole.
+// ms per call with 4, 6, 8 and 16 slabs: s=91 1.277, 1.244, 1.225; s=120 2.71,
+// 2.63, 2.70; s=150 4.95, 4.91, 5.01, 5.25. Fewer leave more of the copies
+// exposed, more add copy and launch overhead; 8 is the best at s=91 and 2 to
+// 3 % from it above.
 constexpr int kLeapfrogSlabs = 8;
 // Up to this many elements a call takes the mesh whole: a slab costs some 17
 // us of copies and launches, more than it hides of a small mesh's. us per
@@ -730,8 +732,8 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     }
     const Mesh& m = d->m;
     const double dt = v->time->deltatime;
-    // The cycle runs in slabs of whole element planes (the handle's matOrder
-    // is slab-major), on six streams: uploads (cstream), compute (stream,
+    // The cycle runs in slabs of whole element planes (matOrderSlab holds the
+    // material order slab by slab), on six streams: uploads (cstream), compute (stream,
     // and stream2 for every other slab, so that the tail of one slab's
     // launch overlaps the next; nstream for the node ranges, beside the
     // force slabs) and downloads (mstream for the results of stream and
@@ -745,8 +747,8 @@ int lulesh_leapfrog(lulesh_dev* d, lulesh_domain_view* v) {
     //     -> forces of slab k;
     //   node update in ranges, one after every two force slabs (the node
     //     planes below the next slab's, whose corner forces are then all
-    //     formed; later slabs' uploads, checks and forces touch only node
-    //     planes above them, so the ranges run beside the force phase) and
+    //     formed; later slabs' uploads and forces touch only node planes
+    //     above them, so the ranges run beside the force phase) and
     //     the rest after the last, each range's fields going down behind it;
     //   kinematics in slabs of two force slabs, each one's fields going down
     //     while the next runs, so that they are down before the material
@@ -1192,9 +1194,9 @@ size_t mesh_bytes(int precision, int numElem, int numNode) {
     Mesh m{};
     Arena a;
     carve_mesh(m, a, precision, numElem, numNode);
-    // A double problem's block of a pool has 48 doubles per element in reserve
-    // (once its stored geometry), so that what pools and budgets sized by the
-    // footprint admit and refuse stays as it was.
+    // A double problem's block of a pool has 48 doubles per element in reserve,
+    // which nothing reads or writes (once its stored geometry): what pools and
+    // budgets sized by the footprint admit and refuse stays as it was.
     if (precision == LULESH_FP64) a.used += 48 * sizeof(double) * size_t(numElem);
     return (a.used + 255) & ~size_t(255);
 }

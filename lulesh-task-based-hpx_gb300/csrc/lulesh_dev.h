@@ -280,7 +280,8 @@ size_t mesh_bytes(int precision, int numElem, int numNode);
 int validate_view(const lulesh_domain_view* v);
 // Carves the mesh arrays out of base (mesh_bytes long), uploads topology and
 // the full state of v on stream s and waits for the copies; leaves
-// partials/result/dtime/matGrid to the caller.
+// partials, result, dtime and report (null where no host word takes the
+// cycle's result) to the caller.
 int mesh_init(Mesh& m, char* base, const lulesh_domain_view* v, int precision, cudaStream_t s);
 // Checks a problem description (sizes that fit the int32 indices).
 int check_problem(const lulesh_problem* p);

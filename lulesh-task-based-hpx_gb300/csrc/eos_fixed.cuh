@@ -142,9 +142,8 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     qq = opening ? 0.0 : qq;
     const int xe = exponent(e_old), xp = exponent(p_old), xq = exponent(q_old), xl = exponent(ql), xqq = exponent(qq),
               xd = exponent(delv), xv = exponent(v);
-    // everything normal or zero, of sane magnitude; |delv| below v / 2
-    bool ok = xe < 1800 && xp < 1800 && xq < 1800 && xl < 1800 && xqq < 1800 && xd + 2 <= xv && xv > 700 && xv < 1400 &&
-              bits_of(v) >= 0;
+    // everything normal or zero, of sane magnitude; v positive and |delv| below v / 2
+    bool ok = max3(max3(xe, xp, xq), xl, xqq) < 1800 && xd + 2 <= xv && uint32_t((high_word(v) >> 20) - 701) < 699u;
     // |x| < 2^(exponent - 1022): tops of the pressures (tp) and energies (te),
     // which their sums pass by a factor 3 at most
     const int tb = opening ? 1024 - xv : 1023 - xv;  // of 2/3 / v and 2/3 / vhalf
@@ -169,7 +168,7 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     // less than half a last place of qq unless ql is above 2^7 qq, and of no
     // account while all energies are below the cutoff with and without it
     const int tc = cut.ue + 56;  // of half the cutoff
-    ok &= xl <= xqq + 7 || (te < tc && xl - 1079 + th <= tc) || (bits_of(e_old) >= bits_of(kCold) && xl < 1053);
+    ok &= xl <= xqq + 7 || (te < tc && xl - 1079 + th <= tc) || (high_word(e_old) > high_word(kCold) && xl < 1053);
     const int64_t po = mantissa(p_old) >> clamp63(up0 - (xp - 1080)), qo = mantissa(q_old) >> clamp63(up0 - (xq - 1080)),
                   qb = mantissa(qq) >> clamp63(up - (xqq - 1080)), ec = cut_in(cut.e_cut, cut.ue, ue);
     // volumes: 2/3 over the half-step one and the new one
@@ -184,10 +183,10 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     const int uph = ue0 + 58 - 115 - uh, upv = ue + 58 - 115 - (xv - 1080);
     const int64_t pch = cut_in(cut.p_cut, cut.up, uph), pcv = cut_in(cut.p_cut, cut.up, upv);
     const int nph = up - uph, npv = up - upv;
-    // work factors: delv / 2 in a unit that takes it to 2^59, delv / 6 in half of it
+    // work factors: delv / 2 in a unit that takes it to 2^59, delv / 6 in half of it.
+    // (By the bounds te and tp: nph, npv >= 1, nw0 >= 0, nw >= 2, |pqh| below 2.7 2^57.)
     const Limb hd = limb(2 * md), d6 = limb(mul(md, 4 * kThird));
     const int nw0 = ue0 - (xd - 1082 + up0 + 58), nw = ue - (xd - 1082 + up + 58);
-    ok &= nph >= 0 && npv >= 0 && nw >= 2;
     const int sph = clamp63(nph), spv = clamp63(npv), sw2 = clamp63(nw - 2);
     const Limb lf = limb(mul(mantissa(ql), kRootFull)), lc = limb(mul(mantissa(ql), kRootCut));
     const int ul = xl - 1080 + 1, ql_unit = up - (ul + 58);
@@ -211,7 +210,6 @@ LULESH_BF bool eos_pass(double e_old, double p_old, double q_old, double ql, dou
     p = off ? 0 : p >> sph;
     const int64_t pq = (po + qo) >> clamp63(up - up0);
     const int64_t pqh = p + viscosity(e, ue0, off);
-    ok &= pqh < kBig && pqh > -kBig;
     e = (e >> clamp63(ue - ue0)) + (mul(hd, limb((3 * pq - 4 * pqh) >> 2)) >> sw2);
     e = e < ec && e > -ec ? 0 : e;
     ok &= e < 2 * kBig && e > -2 * kBig;

@@ -90,12 +90,12 @@ LAYOUT_BYTES_PER_UNIT = {
 # pipe carries only a small part of the double path's arithmetic: its element
 # kernels work in block fixed point on the integer pipes.
 TRAFFIC_PER_UNIT = {
-    "fp64": {"forces": 295, "nodes": 355, "kinematics": 169, "material": 210},
-    "mixed": {"forces": 204, "nodes": 298, "kinematics": 169, "material": 177},
+    "fp64": {"forces": 294, "nodes": 355, "kinematics": 169, "material": 205},
+    "mixed": {"forces": 204, "nodes": 298, "kinematics": 168, "material": 171},
 }
 FP64_INSTR_PER_UNIT = {
-    "fp64": {"forces": 66.0, "nodes": 29.7, "kinematics": 78.0, "material": 26.4},
-    "mixed": {"forces": 7.0, "nodes": 12.0, "kinematics": 71.0, "material": 83.7},
+    "fp64": {"forces": 66.0, "nodes": 29.7, "kinematics": 78.0, "material": 22.9},
+    "mixed": {"forces": 7.0, "nodes": 12.0, "kinematics": 71.0, "material": 86.6},
 }
 # Double-precision operations per unit of the reference's formulation (adds,
 # multiplies, divides, square and cube roots each counted once), from

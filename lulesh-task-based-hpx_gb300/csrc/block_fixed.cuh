@@ -62,7 +62,7 @@ LULESH_BF int64_t bits_of(double x) { return __double_as_longlong(x); }
 // The bits for a test of the whole of them: seen as a double's, the compiler
 // would make it an FP64 compare (dmul_bits). Not for every use: the opaque
 // move keeps it from sharing work too (the EOS and Q terms, which use none,
-// take 0.616 ms at s=150, with it 0.635).
+// take 0.628 ms at s=150, with it 0.644).
 LULESH_BF int64_t tested_bits(double x) { return static_cast<int64_t>(dmul_bits(x)); }
 LULESH_BF double of_bits(int64_t b) { return __longlong_as_double(b); }
 LULESH_BF int32_t high_word(double x) { return int32_t(bits_of(x) >> 32); }

@@ -389,7 +389,7 @@ __device__ __forceinline__ void material_elem(const Mesh& m, int t, int r, int l
 // with 4, 5, 6 blocks, k_kinematics 0.643, 0.633, 0.641. The exact variant's
 // out-of-line products leave a warp waiting on their chains: at s=60 k_forces
 // takes 0.594, 0.62, 0.536, 0.661 ms with 1 to 4 blocks, k_kinematics 0.274,
-// 0.274, 0.277, 0.282 (and 0.273 with 3 and its compares in integers).
+// 0.274, 0.277, 0.282 (before its compares were integers; now 0.277 with 3).
 constexpr int kForceBlocks = LULESH_EXACT ? 3 : 4, kKinBlocks = LULESH_EXACT ? 3 : 5;
 
 #if !LULESH_EXACT
@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(kKinBlock, kKinBlocks) k_kinematics(Mesh m, do
 // variant: 8 blocks of 128 per SM (64 registers), the passes being a chain of
 // dependent operations (s=60: 0.266 ms, 7 and 6 blocks 0.286 and 0.295). Fast
 // variant: 6 (80 registers): its integer passes are bound by the ALU pipe, and
-// more blocks spill (s=150: 0.616, 0.610, 0.619, 0.623 ms with 5 to 8).
+// more blocks spill (5 to 8: s=150 0.645, 0.628, 0.627, 0.652 ms, s=45 0.0416,
+// 0.0421, 0.0430, 0.0440).
 constexpr int kMatBlocks = LULESH_EXACT ? 8 : 6;
 // SPREAD: some class has several lanes per element (MatPlan).
 template <bool SPREAD>
